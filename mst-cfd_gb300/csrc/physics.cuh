@@ -102,72 +102,77 @@ __host__ __device__ __forceinline__ void ausm_axis(const T ql[4], const AusmSide
   f[d + 1] += pF;
 }
 
-// The same AUSM+ quantities for the FP32 production path, with each
-// state's 1/rho computed once and the supersonic branches in closed form
-// ((M + |M|) / (2M) = 1 for M > 1, (M - |M|) = 0): fewer divisions, the
-// same formulas as ausm_axis (including the pressure polynomial whose
-// second term is not scaled by p) up to rounding.  Not used by the exact
-// path.
-struct AusmSideF {
-  float ir, p, a_face, a_true, fc[4];
-};
+// 1/sqrt(x) of the production paths: the FP64 one costs 5.5 FP64-pipe
+// instructions on this GPU against 9.3 for a square root and 8.8 for a
+// division (measured: one FP64 instruction holds an SM sub-partition for 64
+// cycles whatever the occupancy), the FP32 one is a single MUFU operation.
+__device__ __forceinline__ double inv_sqrt(double x) { return rsqrt(x); }
+__device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
 
-__host__ __device__ __forceinline__ AusmSideF ausm_side_f(const float q[4]) {
-  AusmSideF s;
-  const float gm1 = Gas<float>::gm1();
-  s.ir = 1.0f / q[0];
-  const float m2 = q[1] * q[1] + q[2] * q[2];
-  s.p = (q[3] - 0.5f * m2 * s.ir) * gm1;
-  const float h = (q[3] + s.p) * s.ir;
-  const float as = sqrtf(h * (2.0f * gm1 / Gas<float>::gp1()));
-  const float U = sqrtf(m2) * s.ir;
-  s.a_face = as * as / fmaxf(as, U);
-  s.a_true = sqrtf(Gas<float>::gamma() * s.p * s.ir);
-  s.fc[0] = q[0];
-  s.fc[1] = q[1];
-  s.fc[2] = q[2];
-  s.fc[3] = q[3] + s.p;
+// AUSM+ of both axes of a face for the production paths (FP64 and FP32): the
+// formulas of ausm_side / ausm_axis (including the pressure polynomial whose
+// second term is not scaled by p) up to rounding, arranged for few divisions
+// and no divergence:
+//   * per side one reciprocal (1/rho), one reciprocal square root for the
+//     interface speed a*^2 / max(a*, |U|), one square root (sound speed);
+//     one reciprocal of the common interface speed for both axes;
+//   * the convected flux 1/2 (M (aL fL + aR fR) - |M| (aR fR - aL fL)) is the
+//     upwind side's M a f;
+//   * the side order of each axis (bit d of `flags`: c0 is the left state)
+//     selects the operands, so a warp whose faces differ in it runs the axis
+//     once.
+template <class T>
+struct AusmCell {
+  T u[2], p, a_face, a_true, w[4];  // w = a_true (rho, rho u, rho v, rho H)
+};
+template <class T>
+__device__ __forceinline__ AusmCell<T> ausm_cell(const T q[4]) {
+  const T gm1 = Gas<T>::gm1();
+  AusmCell<T> s;
+  const T ir = T(1) / q[0];
+  s.u[0] = q[1] * ir;
+  s.u[1] = q[2] * ir;
+  s.p = (q[3] - T(0.5) * (q[1] * s.u[0] + q[2] * s.u[1])) * gm1;
+  const T rh = q[3] + s.p;
+  const T as2 = rh * ir * (T(2) * gm1 / Gas<T>::gp1());
+  const T U2 = s.u[0] * s.u[0] + s.u[1] * s.u[1];
+  s.a_face = as2 * inv_sqrt(as2 < U2 ? U2 : as2);
+  s.a_true = sqrt(Gas<T>::gamma() * s.p * ir);
+  s.w[0] = s.a_true * q[0];
+  s.w[1] = s.a_true * q[1];
+  s.w[2] = s.a_true * q[2];
+  s.w[3] = s.a_true * rh;
   return s;
 }
-
-__host__ __device__ __forceinline__ void ausm_axis_f(const float ql[4], const AusmSideF& L,
-                                                     const float qr[4], const AusmSideF& R, int d,
-                                                     float f[4]) {
-  const float iaF = 1.0f / fminf(R.a_face, L.a_face);
-  const float mL = ql[d + 1] * L.ir * iaF;
-  const float mR = qr[d + 1] * R.ir * iaF;
-  float mp, mm, pp, pm;
-  if (mL <= 1.0f) {
-    const float a = (mL + 1.0f) * (mL + 1.0f), b = (mL * mL - 1.0f) * (mL * mL - 1.0f);
-    mp = 0.25f * a + 0.125f * b;
-    pp = L.p * 0.25f * a * (2.0f - mL) + 0.1875f * mL * b;
-  } else {
-    mp = mL;
-    pp = L.p;
-  }
-  if (mR <= 1.0f) {
-    const float a = (mR - 1.0f) * (mR - 1.0f), b = (mR * mR - 1.0f) * (mR * mR - 1.0f);
-    mm = -0.25f * a - 0.125f * b;
-    pm = R.p * 0.25f * a * (2.0f + mR) - 0.1875f * mR * b;
-  } else {
-    mm = 0.0f;
-    pm = 0.0f;
-  }
-  const float mF = mm + mp, pF = pm + pp, amF = fabsf(mF);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float al = L.a_true * L.fc[k], ar = R.a_true * R.fc[k];
-    f[k] = 0.5f * (mF * (al + ar) - amF * (ar - al));
-  }
-  f[d + 1] += pF;
-}
-
-// AUSM+ flux of the split-axis scheme along axis d (0 = x, 1 = y).
 template <class T>
-__host__ __device__ __forceinline__ void ausm_flux(const T ql[4], const T qr[4],
-                                                   int d, T f[4]) {
-  const AusmSide<T> L = ausm_side(ql), R = ausm_side(qr);
-  ausm_axis(ql, L, qr, R, d, f);
+__device__ __forceinline__ void ausm_face(const T qa[4], const T qb[4], int flags, T F[8]) {
+  const AusmCell<T> A = ausm_cell(qa), B = ausm_cell(qb);
+  // (the zero product hands a sound speed that is not a number -- a state
+  // without positive pressure or density on either side -- to every flux)
+  const T ia = T(1) / (B.a_face < A.a_face ? B.a_face : A.a_face) +
+               T(0) * (A.a_true + B.a_true);
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {
+    const bool c0l = (flags >> d) & 1;  // c0 (qa) is the left state
+    const T mL = (c0l ? A.u[d] : B.u[d]) * ia, mR = (c0l ? B.u[d] : A.u[d]) * ia;
+    const T pL = c0l ? A.p : B.p, pR = c0l ? B.p : A.p;
+    T mp = mL, pp = pL, mm = T(0), pm = T(0);
+    if (!(mL > T(1))) {
+      const T s = mL + T(1), h = T(0.25) * (s * s), t = mL * mL - T(1), b = t * t;
+      mp = h + T(0.125) * b;
+      pp = (pL * h) * (T(2) - mL) + (T(0.1875) * mL) * b;
+    }
+    if (!(mR > T(1))) {
+      const T s = mR - T(1), h = T(0.25) * (s * s), t = mR * mR - T(1), b = t * t;
+      mm = -h - T(0.125) * b;
+      pm = (pR * h) * (T(2) + mR) - (T(0.1875) * mR) * b;
+    }
+    const T mF = mm + mp;
+    const bool up = (mF >= T(0)) == c0l;  // the upwind side is c0
+#pragma unroll
+    for (int k = 0; k < 4; ++k) F[4 * d + k] = mF * (up ? A.w[k] : B.w[k]);
+    F[5 * d + 1] += pp + pm;
+  }
 }
 
 template <class T>
@@ -298,55 +303,62 @@ __host__ __device__ __forceinline__ void roe_flux(const T ql[4], const T qr[4],
   }
 }
 
-// The same Roe flux for the production paths: |A| dQ in closed form as the
-// sum over the waves of |lambda_k| alpha_k r_k, with the wave strengths
-// from the primitive jumps and the Roe-averaged state (equal to
-// R |Lambda| R^-1 dQ of roe_flux for that state, without the 4x4 inverse
-// and the two 4x4 products); the same entropy-fixed eigenvalues, physical
-// fluxes and EOR denominators.  Not used by the exact path.
+// Roe of both axes of a face for the production paths (FP64 and FP32): the
+// same physical fluxes, entropy-fixed eigenvalues and EOR denominators as
+// roe_flux, with |A| dQ in closed form (the sum over the waves of
+// |lambda_k| alpha_k r_k) and everything that does not depend on the axis
+// formed once per face: the Roe average is symmetric in the two states and
+// the jumps change sign with their order, so the dissipation of axis d only
+// enters with the sign of the side order (bit d of `flags`: c0 is the left
+// state).  One reciprocal square root gives a and 1/a^2.  Not used by the
+// exact path.
 template <class T>
-__host__ __device__ __forceinline__ void roe_flux_fast(const T ql[4], const T qr[4], int d,
-                                                       T f[4]) {
-  const T eor = T(1e-10);
-  const int t = 1 - d;
-  const T irL = T(1) / ql[0], irR = T(1) / qr[0];
-  const T D = sqrt(fabs(qr[0] * irL));
+__device__ __forceinline__ T entropy_fix_fast(T x) {
+  const T ax = fabs(x), e = T(0.125);
+  return ax > e ? ax : (x * x + e * e) * (T(0.5) / e);
+}
+template <class T>
+__device__ __forceinline__ void roe_face(const T L[4], const T R[4], int flags, T F[8]) {
+  const T eor = T(1e-10), gm1 = Gas<T>::gm1();
+  const T irL = T(1) / L[0], irR = T(1) / R[0];
+  const T uL[2] = {L[1] * irL, L[2] * irL}, uR[2] = {R[1] * irR, R[2] * irR};
+  const T pL = (L[3] - T(0.5) * (L[1] * uL[0] + L[2] * uL[1])) * gm1;
+  const T pR = (R[3] - T(0.5) * (R[1] * uR[0] + R[2] * uR[1])) * gm1;
+  const T hL = (L[3] + pL) * irL, hR = (R[3] + pR) * irR;
+  const T x = fabs(R[0] * irL);
+  const T D = x * inv_sqrt(x);
   const T iD = T(1) / (T(1) + D);
-  const T uL[2] = {ql[1] * irL, ql[2] * irL}, uR[2] = {qr[1] * irR, qr[2] * irR};
   const T u[2] = {(uL[0] + D * uR[0]) * iD, (uL[1] + D * uR[1]) * iD};
-  const T pL = th_p(ql), pR = th_p(qr);
-  const T hL = (ql[3] + pL) * irL, hR = (qr[3] + pR) * irR;
   const T H = (hL + D * hR) * iD;
   const T ke = T(0.5) * (u[0] * u[0] + u[1] * u[1]);
-  const T a2 = fabs(Gas<T>::gm1() * (H - ke));
-  const T a = sqrt(a2);
-  const T ud = u[d], ut = u[t];
-  const T l1 = entropy_fix(fabs(ud - a)), l2 = entropy_fix(fabs(ud)),
-          l4 = entropy_fix(fabs(ud + a));
-  const T rt = D * ql[0];
-  const T dp = pR - pL, dud = uR[d] - uL[d], dut = uR[t] - uL[t];
-  const T ia2 = T(1) / a2;
-  const T w1 = l1 * (T(0.5) * (dp - rt * a * dud) * ia2);
-  const T w4 = l4 * (T(0.5) * (dp + rt * a * dud) * ia2);
-  const T w2 = l2 * ((qr[0] - ql[0]) - dp * ia2);
-  const T w3 = l2 * (rt * dut);
-  T dis[4];
-  dis[0] = w1 + w2 + w4;
-  dis[1 + d] = w1 * (ud - a) + w2 * ud + w4 * (ud + a);
-  dis[1 + t] = (w1 + w2 + w4) * ut + w3;
-  dis[3] = w1 * (H - ud * a) + w2 * ke + w4 * (H + ud * a) + w3 * ut;
-  const T iL = T(1) / (ql[0] + eor), iR = T(1) / (qr[0] + eor);
-  T FL[4], FR[4];
-  FL[0] = ql[1 + d];
-  FR[0] = qr[1 + d];
-  FL[1 + d] = ql[1 + d] * ql[1 + d] * iL + pL;
-  FR[1 + d] = qr[1 + d] * qr[1 + d] * iR + pR;
-  FL[1 + t] = ql[1] * ql[2] * iL;
-  FR[1 + t] = qr[1] * qr[2] * iR;
-  FL[3] = hL * ql[1 + d];
-  FR[3] = hR * qr[1 + d];
+  const T a2 = fabs(gm1 * (H - ke));
+  const T ia = inv_sqrt(a2);
+  const T a = a2 * ia, ia2 = ia * ia;
+  const T rt = D * L[0];
+  const T dp = pR - pL, du[2] = {uR[0] - uL[0], uR[1] - uL[1]};
+  const T al2 = (R[0] - L[0]) - dp * ia2;
+  const T hia2 = T(0.5) * ia2, rta = rt * a;
+  const T iL = T(1) / (L[0] + eor), iR = T(1) / (R[0] + eor);
+  // momentum / (rho + EOR), momentum fluxes' second factor
+  const T vL[2] = {L[1] * iL, L[2] * iL}, vR[2] = {R[1] * iR, R[2] * iR};
 #pragma unroll
-  for (int k = 0; k < 4; ++k) f[k] = T(0.5) * (FL[k] + FR[k]) - T(0.5) * dis[k];
+  for (int d = 0; d < 2; ++d) {
+    const int t = 1 - d;
+    const T ud = u[d], ut = u[t];
+    const T l1 = entropy_fix_fast(ud - a), l2 = entropy_fix_fast(ud),
+            l4 = entropy_fix_fast(ud + a);
+    const T rd = rta * du[d];
+    const T w1 = l1 * ((dp - rd) * hia2), w4 = l4 * ((dp + rd) * hia2);
+    const T w2 = l2 * al2, w3 = l2 * (rt * du[t]);
+    const T ws = (w1 + w2) + w4, wd = (w4 - w1) * a;
+    const T sg = ((flags >> d) & 1) ? T(-0.5) : T(0.5);
+    const T mL = L[1 + d], mR = R[1 + d];
+    F[4 * d] = T(0.5) * (mL + mR) + sg * ws;
+    F[4 * d + 1 + d] = T(0.5) * ((mL * vL[d] + mR * vR[d]) + (pL + pR)) + sg * (ws * ud + wd);
+    F[4 * d + 1 + t] = T(0.5) * (mL * vL[t] + mR * vR[t]) + sg * (ws * ut + w3);
+    F[4 * d + 3] = T(0.5) * (hL * mL + hR * mR) +
+                   sg * ((w1 + w4) * H + (wd * ud + (w2 * ke + w3 * ut)));
+  }
 }
 
 }  // namespace mst

@@ -1,0 +1,59 @@
+"""FP64 production path (fused multiply-add, shared reciprocals, one Riemann
+solve per face) against the FP64_EXACT path on the same inputs."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+
+
+def _mesh(nx, ny, seed):
+    from mstcfd import Mesh
+    from mstcfd import meshgen as mg
+    m = mg.reorient(mg.tri_box(nx, ny, 4.0, 2.0, jitter=0.2, seed=seed), "random", seed=3)
+    return m, Mesh.from_arrays(m["node_xy"], m["face_nodes"], m["face_cells"], m["zones"],
+                               m["n_cells"])
+
+
+def _state(kind, xy, seed):
+    from mstcfd import meshgen as mg
+    if kind == "supersonic":  # both signs, |u| above and below the sound speed
+        return mg.random_state(len(xy), seed=seed, umax=4.0)
+    q = mg.smooth_state(xy)
+    if kind == "partly_uniform":  # zero and vanishing differences
+        left = xy[:, 0] < 2.0
+        q[left] = q[0]
+        q[left, 2] = 1e-170 * (1 + xy[left, 1])
+    return q
+
+
+@pytest.mark.parametrize("flux", [0, 1], ids=["ausm", "roe"])
+@pytest.mark.parametrize("limiter,viscous", [(0, 0), (1, 0), (2, 0), (3, 0), (1, 1), (3, 1)])
+@pytest.mark.parametrize("kind", ["smooth", "supersonic", "partly_uniform"])
+def test_fp64_residual_matches_exact(flux, limiter, viscous, kind):
+    from mstcfd import Solver
+    m, mesh = _mesh(13, 7, 5)
+    arr = mesh.arrays()
+    q = _state(kind, arr["cell_ctr"], 1)
+    kw = dict(flux=flux, order=2, limiter=limiter, reference_quirks=0, dt=1e-5, viscous=viscous)
+    if viscous:
+        kw.update(mu=1e-3, lambda_=-2e-3 / 3, kappa=2e-3, cv=1.7857)
+    out = {}
+    for prec in (0, 1):
+        s = Solver(mesh, precision=prec, **kw)
+        s.set_state(q)
+        s.solve()
+        out[prec] = (s.residual(), s.face_flux())
+        s.close()
+    # a face's flux is a chain of a few hundred roundings of numbers of the
+    # size of the largest flux; a cell adds its faces'
+    F = np.abs(out[0][1]).max()
+    S = np.zeros(m["n_cells"])
+    for k in range(2):
+        on = m["face_cells"][:, k] >= 0
+        np.add.at(S, m["face_cells"][on, k], arr["face_area"][on])
+    tol = 500 * EPS * F * S[:, None]
+    assert np.all(np.isfinite(out[1][0]))
+    assert np.all(np.abs(out[1][0] - out[0][0]) <= tol)
+    assert np.abs(out[1][1] - out[0][1]).max() <= 500 * EPS * F
