@@ -264,6 +264,7 @@ mst_status launch_grad(mst_ctx* c, const double4_32a* q, const float4* qf = null
 }
 
 mst_status launch_flux(mst_ctx* c, const mst::StepArgs& a) {
+  if (a.fx) c->last_launches++;  // the face / cell kernel pair
   ProfScope ps(c, c->p.precision != MST_PREC_FP32 ? "k_flux_update<f64>"
                   : a.tile_grad                   ? "k_flux_update<f32,tg>"
                                                   : "k_flux_update<f32>");
@@ -326,6 +327,34 @@ mst::StepArgs base_args(mst_ctx* c) {
   return a;
 }
 
+template <class T>
+mst_status dalloc(mst_ctx* c, T** p, size_t bytes) {
+  CU(cudaMalloc((void**)p, std::max<size_t>(bytes, 256)));
+  c->allocs.push_back(*p);
+  return MST_OK;
+}
+
+// the face-flux buffer of the context's FP64 path (none on the FP32 path);
+// at creation and when the parameters change, never while stepping
+mst_status ensure_face_buffer(mst_ctx* c, int precision) {
+  if (precision == MST_PREC_FP32) return MST_OK;
+  const size_t words = precision == MST_PREC_FP64_EXACT ? 8 : 4;
+  if (words <= c->fx_words) return MST_OK;
+  double* p = nullptr;
+  const size_t bytes = std::max<size_t>(words * c->dm.n_faces * sizeof(double), 256);
+  CU(cudaMalloc((void**)&p, bytes));
+  if (c->fx) {
+    CU(cudaStreamSynchronize(c->stream));
+    cudaFree(c->fx);
+    *std::find(c->allocs.begin(), c->allocs.end(), (void*)c->fx) = p;
+  } else {
+    c->allocs.push_back(p);
+  }
+  c->fx = p;
+  c->fx_words = words;
+  return MST_OK;
+}
+
 // one residual evaluation + update of stage 'stage' from q into qn
 // Buffers of one stage: FP64 state q -> qn (q0 = Q^n for stage 1); on the
 // FP32 path the float-pair state (qf, ql) -> (qfn, qln) with (q0f, q0l).
@@ -374,6 +403,7 @@ mst_status run_stage(mst_ctx* c, const StageBufs& b, int stage, bool fixed_dt, b
     else a.dt_dev = c->scal;
   }
   a.partials = norms ? c->partials : nullptr;
+  a.fx = pairs(c) ? nullptr : c->fx;
   return launch_flux(c, a);
 }
 
@@ -443,13 +473,6 @@ mst_status read_norms(mst_ctx* c, mst_norms* out) {
     out->dt = h[kNormSlots];
     out->time = h[kNormSlots + 1];
   }
-  return MST_OK;
-}
-
-template <class T>
-mst_status dalloc(mst_ctx* c, T** p, size_t bytes) {
-  CU(cudaMalloc((void**)p, std::max<size_t>(bytes, 256)));
-  c->allocs.push_back(*p);
   return MST_OK;
 }
 
@@ -839,7 +862,8 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
       (st = dalloc(c.get(), &c->dt_cell, nC * sizeof(double))) ||
       (st = dalloc(c.get(), &c->dt_cell_ff, nC * sizeof(float2))) ||
       (st = dalloc(c.get(), &c->scal, 4 * sizeof(double))) ||
-      (st = dalloc(c.get(), &c->norms, (kNormSlots + 2) * sizeof(double))))
+      (st = dalloc(c.get(), &c->norms, (kNormSlots + 2) * sizeof(double))) ||
+      (st = ensure_face_buffer(c.get(), p->precision)))
     return st;
   CU(cudaMemset(c->q_old, 0, qbytes));
   CU(cudaMemset(c->q_new, 0, qbytes));
@@ -873,6 +897,7 @@ mst_status mst_ctx_set_params(mst_ctx* c, const mst_params* p) {
   if (!c) return fail(MST_EINVAL, "NULL context");
   mst_status st = check_params(p);
   if (st) return st;
+  if ((st = ensure_face_buffer(c, p->precision))) return st;
   const bool was = pairs(c);
   const bool to_pairs = p->precision == MST_PREC_FP32 && !was;
   if (was && p->precision != MST_PREC_FP32) {  // the FP64 buffers were not kept

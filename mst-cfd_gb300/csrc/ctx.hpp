@@ -62,6 +62,10 @@ struct mst_ctx {
   float4 *ql_old = nullptr, *ql_new = nullptr, *ql_stage = nullptr;
   void* grad = nullptr;
   double* flux = nullptr;      // [nF][8] debug output
+  // FP64 paths: the face-flux buffer, 4 (production) or 8 (exact) doubles
+  // per face; allocated once a context runs one of them
+  double* fx = nullptr;
+  size_t fx_words = 0;
   double* partials = nullptr;  // [max(nT, nBlocks)][kNormSlots]
   double* dt_part = nullptr;   // [nBlocks]
   double* dt_cell = nullptr;   // [nC]

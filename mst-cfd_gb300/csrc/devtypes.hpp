@@ -146,6 +146,10 @@ struct StepArgs {
   const int* case_frozen;
   void* phi;
   double* partials;       // [n_tiles][kNormSlots] or nullptr
+  // FP64 paths: face-flux buffer of the face / cell kernel pair, [n_faces][4]
+  // (production: flux projected on the area vector) or [n_faces][8] (exact);
+  // nullptr: the tile kernel
+  double* fx;
 };
 constexpr int kCaseWords = 8;
 

@@ -20,7 +20,7 @@ def _state(kind, xy, seed):
     from mstcfd import meshgen as mg
     if kind == "supersonic":  # both signs, |u| above and below the sound speed
         return mg.random_state(len(xy), seed=seed, umax=4.0)
-    q = mg.smooth_state(xy)
+    q = mg.smooth_state(xy, umax=2.5 if kind == "fast" else 0.8)
     if kind == "partly_uniform":  # zero and vanishing differences
         left = xy[:, 0] < 2.0
         q[left] = q[0]
@@ -28,9 +28,13 @@ def _state(kind, xy, seed):
     return q
 
 
-@pytest.mark.parametrize("flux", [0, 1], ids=["ausm", "roe"])
+# (random states reconstruct to unphysical ones on some faces; the closed
+# form of |A| dQ equals the exact path's R |L| R^-1 dQ only where the Roe
+# average has a positive squared sound speed, so Roe takes the smooth ones)
 @pytest.mark.parametrize("limiter,viscous", [(0, 0), (1, 0), (2, 0), (3, 0), (1, 1), (3, 1)])
-@pytest.mark.parametrize("kind", ["smooth", "supersonic", "partly_uniform"])
+@pytest.mark.parametrize("flux,kind", [(0, "smooth"), (0, "fast"), (0, "supersonic"),
+                                       (0, "partly_uniform"), (1, "smooth"), (1, "fast"),
+                                       (1, "partly_uniform")])
 def test_fp64_residual_matches_exact(flux, limiter, viscous, kind):
     from mstcfd import Solver
     m, mesh = _mesh(13, 7, 5)
@@ -48,12 +52,16 @@ def test_fp64_residual_matches_exact(flux, limiter, viscous, kind):
         s.close()
     # a face's flux is a chain of a few hundred roundings of numbers of the
     # size of the largest flux; a cell adds its faces'
-    F = np.abs(out[0][1]).max()
+    # (an unlimited reconstruction of the random state may leave the physical
+    # range: both paths then give no number on the same faces and cells)
+    ok = [np.isfinite(out[0][i]) for i in range(2)]
+    for i in range(2):
+        assert np.array_equal(np.isfinite(out[1][i]), ok[i])
+    F = np.abs(out[0][1][ok[1]]).max()
     S = np.zeros(m["n_cells"])
     for k in range(2):
         on = m["face_cells"][:, k] >= 0
         np.add.at(S, m["face_cells"][on, k], arr["face_area"][on])
     tol = 500 * EPS * F * S[:, None]
-    assert np.all(np.isfinite(out[1][0]))
-    assert np.all(np.abs(out[1][0] - out[0][0]) <= tol)
-    assert np.abs(out[1][1] - out[0][1]).max() <= 500 * EPS * F
+    assert np.all((np.abs(out[1][0] - out[0][0]) <= tol)[ok[0]])
+    assert np.abs(out[1][1] - out[0][1])[ok[1]].max() <= 500 * EPS * F
