@@ -44,7 +44,8 @@ __global__ void k_batch_gather(const double4_32a* __restrict__ src,
 // those flagged in `flag` (restarts from the fallback states, which also
 // un-count a retired case and start its iteration numbers at *iter).
 struct CaseProgress {
-  double *cfl, *l2_win, *stall_best;
+  double *cfl, *dfac, *l2_win, *stall_best;
+  double omega;
   int *conv_iter, *diverged, *frozen, *stall_best_it, *restart_it, *n_conv, *iter;
 };
 __global__ void k_batch_reset(int n_cases, double cfl0, CaseProgress p, const int* flag) {
@@ -53,6 +54,7 @@ __global__ void k_batch_reset(int n_cases, double cfl0, CaseProgress p, const in
   if (i < n_cases && (!flag || flag[i])) {
     if (flag && p.conv_iter[i] >= 0) atomicSub(p.n_conv, 1);
     p.cfl[i] = cfl0;
+    p.dfac[i] = 1.0 / cfl0 + 0.5 * p.omega;
     p.conv_iter[i] = -1;
     p.diverged[i] = 0;
     p.frozen[i] = 0;
@@ -93,13 +95,12 @@ struct mst_batch {
   mst_implicit_params ip{};
   std::vector<int> color_off;    // [n_colors + 1] into color_cells
   std::vector<int> color_file;   // colour of every union cell, file order
-  int* color = nullptr;          // device order
-  int* color_cells = nullptr;
+  int4* color_cells = nullptr;   // sweep entries of all cells, by colour (LusgsArgs)
   int* c_case = nullptr;
   int* case_first = nullptr;
   double* case_tab = nullptr;
   float* case_tab_f = nullptr;
-  double *cfl = nullptr, *first = nullptr, *last = nullptr;
+  double *cfl = nullptr, *dfac = nullptr, *first = nullptr, *last = nullptr;
   int *conv_iter = nullptr, *n_conv = nullptr, *iter = nullptr;
   int* diverged = nullptr;       // per case: retired with a non-finite L2
   int* frozen = nullptr;         // per-case limiter-freezing state
@@ -117,9 +118,9 @@ struct mst_batch {
   // compaction: once most cases have converged, the residual kernels visit
   // the tiles and the sweeps the cells of unconverged cases only
   std::vector<int> c_case_h;     // case of every device cell
-  std::vector<int> color_cells_h;
+  std::vector<int4> color_cells_h;
   int* tile_list = nullptr;      // device [n_tiles]
-  int* act_cells = nullptr;      // device [n_cells]: per colour, active cells
+  int4* act_cells = nullptr;     // device [n_cells]: per colour, active cells
   std::vector<int> act_off;      // [n_colors + 1] into act_cells
   bool compact = false;          // lists in use
   long long list_cells = 0;      // cells of the cases the lists hold
@@ -129,7 +130,8 @@ struct mst_batch {
   float4* dqf = nullptr;         // FP32 sweeps: dQ* / dQ in FP32
   bool sweep32 = false;
   bool first_fixed = false;      // reference L2s set by mst_batch_set_l2_ref
-  double* norm_part = nullptr;   // [n_cases][8] partial L2 sums
+  double* norm_part = nullptr;   // [n_cases][kMaxNormParts] partial L2 sums
+  unsigned* norm_ticket = nullptr;
   int cur = 0;                   // which of ctx->q_old / q_new holds Q
   // mixed precision: each case evaluates the FP32 residual (FP32 state
   // copy, FP32 gradient) until it is ready for the FP64 one; lo is set
@@ -243,11 +245,8 @@ mst::LusgsArgs sweep_args(mst_batch* b, int which) {
   la.diag = b->diag;
   la.qn = qbuf(b, 1 - which);
   la.qfn = qfbuf(b, 1 - which);
-  la.color = b->color;
-  la.c_case = b->c_case;
-  la.cfl = b->cfl;
+  la.dfac = b->dfac;
   la.case_tab = b->case_tab;
-  la.mu = c->p.mu;
   la.viscous = c->p.viscous;
   la.omega = b->ip.omega;
   la.conv_iter = b->conv_iter;
@@ -258,7 +257,6 @@ mst::LusgsArgs sweep_args(mst_batch* b, int which) {
     la.qf = qfbuf(b, which);
     la.dqf = b->dqf;
     la.case_tab_f = b->case_tab_f;
-    la.mu_f = (float)c->p.mu;
   }
   return la;
 }
@@ -267,17 +265,20 @@ mst_status enqueue_sweeps(mst_batch* b, int which, int threads) {
   mst_ctx* c = b->ctx;
   mst::LusgsArgs la = sweep_args(b, which);
   for (int pass = 0; pass < 2; ++pass) {
-    for (int i = 0; i < b->n_colors; ++i) {
+    // forward over the colours; the last one is updated in its forward
+    // launch (its cells have no neighbour of higher colour), so the backward
+    // sweep starts at the one before
+    for (int i = pass; i < b->n_colors; ++i) {
       const int col = pass == 0 ? i : b->n_colors - 1 - i;
-      la.col = col;
-      const int* cells = b->compact ? b->act_cells : b->color_cells;
+      const bool turn = col == b->n_colors - 1;
+      const int4* cells = b->compact ? b->act_cells : b->color_cells;
       const std::vector<int>& off = b->compact ? b->act_off : b->color_off;
       la.cells = cells + off[col];
       la.n = off[col + 1] - off[col];
       cudaError_t e;
       if (pass == 0)
-        e = exact(b) ? mst::exact::lusgs_forward_t(c->dm, la, threads, c->stream)
-                     : mst::fast::lusgs_forward_t(c->dm, la, threads, c->stream);
+        e = exact(b) ? mst::exact::lusgs_forward_t(c->dm, la, threads, turn, c->stream)
+                     : mst::fast::lusgs_forward_t(c->dm, la, threads, turn, c->stream);
       else
         e = exact(b) ? mst::exact::lusgs_backward_t(c->dm, la, threads, c->stream)
                      : mst::fast::lusgs_backward_t(c->dm, la, threads, c->stream);
@@ -298,6 +299,8 @@ mst_status enqueue_iteration(mst_batch* b, int which) {
   na.first = b->first;
   na.last = b->last;
   na.cfl = b->cfl;
+  na.dfac = b->dfac;
+  na.omega = b->ip.omega;
   na.conv_iter = b->conv_iter;
   na.n_conv = b->n_conv;
   na.diverged = b->diverged;
@@ -317,6 +320,7 @@ mst_status enqueue_iteration(mst_batch* b, int which) {
   na.freeze_tol = b->ip.freeze_tol;
   na.first_fixed = b->first_fixed ? 1 : 0;
   na.part = b->norm_part;
+  na.ticket = b->norm_ticket;
   na.cfl0 = b->ip.cfl0;
   na.cfl_max = b->ip.cfl_max;
   na.tol = b->ip.tol;
@@ -402,9 +406,9 @@ void update_both(mst_batch* b) {
 }
 
 CaseProgress progress(mst_batch* b) {
-  return CaseProgress{b->cfl,       b->l2_win,        b->stall_best, b->conv_iter,
-                      b->diverged,  b->frozen,        b->stall_best_it,
-                      b->restart_it, b->n_conv,       b->iter};
+  return CaseProgress{b->cfl,       b->dfac,   b->l2_win, b->stall_best,    b->ip.omega,
+                      b->conv_iter, b->diverged, b->frozen, b->stall_best_it,
+                      b->restart_it, b->n_conv, b->iter};
 }
 
 mst_status reset_progress(mst_batch* b) {
@@ -480,13 +484,13 @@ mst_status build_lists(mst_batch* b, const std::vector<int>& cv) {
         break;
       }
   }
-  std::vector<int> cells;
+  std::vector<int4> cells;
   cells.reserve(nC);
   b->act_off.assign(b->n_colors + 1, 0);
   for (int col = 0; col < b->n_colors; ++col) {
     for (int i = b->color_off[col]; i < b->color_off[col + 1]; ++i) {
-      const int d = b->color_cells_h[i];
-      if (cv[b->c_case_h[d]] < 0) cells.push_back(d);
+      const int4 e = b->color_cells_h[i];
+      if (cv[e.z] < 0) cells.push_back(e);
     }
     b->act_off[col + 1] = (int)cells.size();
   }
@@ -494,7 +498,7 @@ mst_status build_lists(mst_batch* b, const std::vector<int>& cv) {
     B_CU(cudaMemcpy(b->tile_list, tiles.data(), sizeof(int) * tiles.size(),
                     cudaMemcpyHostToDevice));
   if (!cells.empty())
-    B_CU(cudaMemcpy(b->act_cells, cells.data(), sizeof(int) * cells.size(),
+    B_CU(cudaMemcpy(b->act_cells, cells.data(), sizeof(int4) * cells.size(),
                     cudaMemcpyHostToDevice));
   c->dm.tile_list = b->tile_list;
   c->dm.n_list = (int)tiles.size();
@@ -618,8 +622,31 @@ mst_status mst_batch_create(const mst_mesh* const* meshes, const mst_case_params
   b->color_off.assign(ncol + 1, 0);
   for (int d = 0; d < nC; ++d) b->color_off[color_dev[d] + 1]++;
   for (int i = 0; i < ncol; ++i) b->color_off[i + 1] += b->color_off[i];
-  std::vector<int> fill(b->color_off.begin(), b->color_off.end() - 1), cells(nC);
-  for (int d = 0; d < nC; ++d) cells[fill[color_dev[d]]++] = d;
+  // each cell's neighbours of lower and of higher colour
+  std::vector<int> code(nC);
+  for (int c = 0; c < nC; ++c) {
+    int n[2] = {0, 0}, at[2][4];
+    for (int k = h.cell_ptr[c]; k < h.cell_ptr[c + 1]; ++k) {
+      if (h.face_cells[2 * h.cell_faces[k] + 1] < 0 || h.cell_faces[k] >= h.n_int_faces) continue;
+      const int cj = b->color_file[h.cell_nb[k]];
+      if (cj == b->color_file[c]) continue;
+      const int up = cj > b->color_file[c];
+      at[up][n[up]++] = k - h.cell_ptr[c];
+    }
+    int w = n[0] | n[1] << 3 | (h.cell_ptr[c + 1] - h.cell_ptr[c] - 1) << 6;
+    for (int i = 0; i < n[0] + n[1]; ++i)
+      w |= (i < n[0] ? at[0][i] : at[1][i - n[0]]) << (8 + 2 * i);
+    code[L.cell_perm[c]] = w;
+  }
+  // the cells of a colour listed by their number of lower neighbours (the
+  // higher ones fall as those rise), so that the lanes of a warp have the
+  // same number of terms; device order within
+  std::vector<int4> cells;
+  cells.reserve(nC);
+  std::vector<std::vector<int>> by(8 * (size_t)ncol);
+  for (int d = 0; d < nC; ++d) by[8 * (size_t)color_dev[d] + (code[d] & 7)].push_back(d);
+  for (const auto& v : by)
+    for (int d : v) cells.push_back(make_int4(d, code[d], c_case[d], L.c_ptr[d]));
   std::vector<double> tab((size_t)mst::kCaseWords * n_cases);
   std::vector<float> tabf(tab.size());
   for (int k = 0; k < n_cases; ++k) {
@@ -631,13 +658,13 @@ mst_status mst_batch_create(const mst_mesh* const* meshes, const mst_case_params
       tabf[8 * (size_t)k + j] = (float)v[j];
     }
   }
-  if ((st = bupload(b.get(), &b->color, color_dev)) ||
-      (st = bupload(b.get(), &b->color_cells, cells)) ||
+  if ((st = bupload(b.get(), &b->color_cells, cells)) ||
       (st = bupload(b.get(), &b->c_case, c_case)) ||
       (st = bupload(b.get(), &b->case_first, case_first)) ||
       (st = bupload(b.get(), &b->case_tab, tab)) ||
       (st = bupload(b.get(), &b->case_tab_f, tabf)) ||
       (st = balloc(b.get(), &b->cfl, sizeof(double) * n_cases)) ||
+      (st = balloc(b.get(), &b->dfac, sizeof(double) * n_cases)) ||
       (st = balloc(b.get(), &b->first, sizeof(double) * n_cases)) ||
       (st = balloc(b.get(), &b->last, sizeof(double) * n_cases)) ||
       (st = balloc(b.get(), &b->conv_iter, sizeof(int) * n_cases)) ||
@@ -655,7 +682,9 @@ mst_status mst_batch_create(const mst_mesh* const* meshes, const mst_case_params
       (st = balloc(b.get(), &b->dq, sizeof(double4_32a) * (size_t)nC)) ||
       (st = balloc(b.get(), &b->diag, sizeof(double) * (size_t)nC)) ||
       (st = balloc(b.get(), &b->dqf, b->sweep32 ? sizeof(float4) * (size_t)nC : 0)) ||
-      (st = balloc(b.get(), &b->norm_part, sizeof(double) * 8 * (size_t)n_cases)) ||
+      (st = balloc(b.get(), &b->norm_part,
+                   sizeof(double) * mst::kMaxNormParts * (size_t)n_cases)) ||
+      (st = bupload(b.get(), &b->norm_ticket, std::vector<unsigned>(1, 0u))) ||
       (st = balloc(b.get(), &b->grad32, p->precision != MST_PREC_FP32 && ip->fp32_until > 0
                                             ? sizeof(float) * 8 * (size_t)nC : 0)) ||
       (st = balloc(b.get(), &b->case_lo, sizeof(int) * n_cases)) ||
@@ -664,7 +693,7 @@ mst_status mst_batch_create(const mst_mesh* const* meshes, const mst_case_params
       (st = balloc(b.get(), &b->restart_it, sizeof(int) * n_cases)) ||
       (st = balloc(b.get(), &b->restart_flag, sizeof(int) * n_cases)) ||
       (st = balloc(b.get(), &b->tile_list, sizeof(int) * (size_t)L.n_tiles)) ||
-      (st = balloc(b.get(), &b->act_cells, sizeof(int) * (size_t)nC)) ||
+      (st = balloc(b.get(), &b->act_cells, sizeof(int4) * (size_t)nC)) ||
       (st = reset_progress(b.get()))) {
     cleanup();
     return st;

@@ -770,6 +770,10 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
       }
       CU(up(&d.cf_dir, as_d2(cd)));
       CU(up(&d.cf_dir32, as_f2(cd)));
+      std::vector<double> len(cd.size() / 2);
+      for (size_t k = 0; k < len.size(); ++k)
+        len[k] = std::sqrt(cd[2 * k] * cd[2 * k] + cd[2 * k + 1] * cd[2 * k + 1]);
+      CU(up(&d.cf_len, len));
     }
     {
       std::vector<double> fe(L.n_faces);
@@ -834,6 +838,7 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
   dm.cf_w32 = d.cf_w32;
   dm.cf_dir = d.cf_dir;
   dm.cf_dir32 = d.cf_dir32;
+  dm.cf_len = d.cf_len;
   dm.t_own_ptr = d.t_own_ptr;
   dm.t_bor_ptr = d.t_bor_ptr;
   dm.t_bor = d.t_bor;

@@ -35,6 +35,7 @@ struct DevArrays {
          *cf_dir32 = nullptr;
   double* f_eta = nullptr;
   float* f_eta32 = nullptr;
+  double* cf_len = nullptr;
   double* c_vol = nullptr;
   double* c_ivol = nullptr;
   float2* c_ivol_ff = nullptr;

@@ -37,6 +37,7 @@ struct DevMesh {
   // f_dir of cf_face): a contiguous load instead of a gather
   const double2* cf_dir;
   const float2* cf_dir32;
+  const double* cf_len;   // its length (rounded as sqrt(x x + y y))
   const int* t_own_ptr;
   const int* t_bor_ptr;
   const int* t_bor;
@@ -176,17 +177,19 @@ struct LusgsArgs {
   const double4_32a* q;    // Q^n, device order
   const double4_32a* r;    // R(Q^n)
   double4_32a* dq;         // dQ* after the forward sweep, dQ after the backward
-  double* diag;            // D_i (written by the forward sweep)
+  double* diag;            // D_i (written by the forward sweep; production
+                           // paths: 1 / D_i)
   double4_32a* qn;         // Q^{n+1} (backward sweep)
   float4* qfn;             // its FP32 copy, or nullptr
-  const int* color;        // colour of every device cell
-  const int* cells;        // the cells of the colour being swept
+  // the cells of the colour being swept, (cell, code, case, first cell-face):
+  // code holds the number of the cell's neighbours of lower colour (bits
+  // 0-2) and of higher colour (3-5), its faces less one (6-7), then two bits
+  // each from bit 8: the position in its face list of the lower ones, then
+  // of the higher ones, each in face order
+  const int4* cells;
   int n;                   // their number
-  int col;                 // the colour
-  const int* c_case;       // case of every device cell (nullptr: case 0)
-  const double* cfl;       // CFL number of every case
-  const double* case_tab;  // per-case coefficients (mu at [4]) or nullptr
-  double mu;               // viscosity of a single case
+  const double* dfac;      // 1 / CFL + omega / 2 of every case
+  const double* case_tab;  // per-case coefficients (mu at [4])
   int viscous;
   double omega;
   const int* conv_iter;    // [n_cases] converged cases keep their state
@@ -196,7 +199,6 @@ struct LusgsArgs {
   const float4* qf;
   float4* dqf;
   const float* case_tab_f;
-  float mu_f;
   double p_floor;          // temperature floor p >= p_floor * rho (0: off)
   int* case_bad;           // [n_cases] set to 1 when a swept state has a
                            // non-positive (or NaN) density or pressure
@@ -208,17 +210,20 @@ struct LusgsArgs {
 // is kept; CFL = clamp(cfl0 * L2_first / L2, cfl0, cfl_max) (switched
 // evolution relaxation); a case converges at the first iteration whose
 // L2 / L2_first < tol.
+constexpr int kMaxNormParts = 32;
 struct CaseNormArgs {
   const double4_32a* r;
   const int* case_first;   // [n_cases + 1] device cell ranges
   double* first;           // [n_cases] L2 of iteration 0
   double* last;            // [n_cases] latest L2
   double* cfl;             // [n_cases]
+  double* dfac;            // [n_cases] 1 / CFL + omega / 2 for the sweeps
+  double omega;
   int* conv_iter;          // [n_cases] -1 until the case is done (converged
                            // or diverged): the iteration it finished at
   int* n_conv;             // number of finished cases
   int* diverged;           // [n_cases] 1 once the case's L2 is not finite
-  int* iter;               // iteration counter (advanced by k_iter_advance)
+  int* iter;               // iteration counter (advanced by the norms)
   int* frozen;             // [n_cases] limiter-freezing state (or nullptr)
   double* l2_win;          // [n_cases] L2 at the last freezing-window check
   double* own_first;       // [n_cases] L2 of this run's first iteration (the
@@ -228,7 +233,8 @@ struct CaseNormArgs {
   int refreeze_window;     // see mst_implicit_params (0: off)
   double cfl0, cfl_max, tol, freeze_tol;
   int first_fixed;         // first[] holds reference L2s set by the caller
-  double* part;            // [n_cases][8] partial sums of (R_rho / V)^2
+  double* part;            // [n_cases][kMaxNormParts] partial sums of (R_rho / V)^2
+  unsigned* ticket;        // blocks that have finished (0 between launches)
   const int* case_lo;      // [n_cases] 1 while a case's residual is FP32 (the
                            // freezing state machine waits for FP64), or nullptr
   const int* restart_it;   // [n_cases] iteration of the case's (re)start
@@ -265,7 +271,7 @@ enum { kFluxAusm = 0, kFluxRoe = 1 };
                                  double* dt_cell, double* partials,           \
                                  cudaStream_t s);                             \
   cudaError_t lusgs_forward_t(const DevMesh& m, const LusgsArgs& a,          \
-                              int threads, cudaStream_t s);                   \
+                              int threads, bool turn, cudaStream_t s);        \
   cudaError_t lusgs_backward_t(const DevMesh& m, const LusgsArgs& a,         \
                                int threads, cudaStream_t s);                  \
   cudaError_t launch_cfl_dt_pairs(const DevMesh& m, const float4* qf,        \
