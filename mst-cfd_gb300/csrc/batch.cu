@@ -641,12 +641,12 @@ mst_status mst_batch_create(const mst_mesh* const* meshes, const mst_case_params
   // the cells of a colour listed by their number of lower neighbours (the
   // higher ones fall as those rise), so that the lanes of a warp have the
   // same number of terms; device order within
-  std::vector<int4> cells;
-  cells.reserve(nC);
-  std::vector<std::vector<int>> by(8 * (size_t)ncol);
-  for (int d = 0; d < nC; ++d) by[8 * (size_t)color_dev[d] + (code[d] & 7)].push_back(d);
-  for (const auto& v : by)
-    for (int d : v) cells.push_back(make_int4(d, code[d], c_case[d], L.c_ptr[d]));
+  std::vector<int4> cells(nC);
+  std::vector<int> at(8 * (size_t)ncol + 1, 0);
+  auto bucket = [&](int d) { return 8 * color_dev[d] + (code[d] & 7); };
+  for (int d = 0; d < nC; ++d) at[bucket(d) + 1]++;
+  for (size_t i = 1; i < at.size(); ++i) at[i] += at[i - 1];
+  for (int d = 0; d < nC; ++d) cells[at[bucket(d)]++] = make_int4(d, code[d], c_case[d], L.c_ptr[d]);
   std::vector<double> tab((size_t)mst::kCaseWords * n_cases);
   std::vector<float> tabf(tab.size());
   for (int k = 0; k < n_cases; ++k) {
