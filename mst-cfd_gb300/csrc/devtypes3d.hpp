@@ -24,6 +24,7 @@ struct DevMesh3 {
   const float2* c_ivol_ff;  // 1/V as a float pair
   const int* c_ptr;
   const int* cf_slot;       // tile slot << 1 | (cell is c1 of the face)
+  const int* cf_face;       // device face, ~face where the cell is its c1
   const int* cf_nb;         // neighbour device cell, -1 on boundary faces
   const double* cf_w;       // [tot][2] face-value weights (self, neighbour)
   const double* cf_dir;     // [tot][3] outward area vector
@@ -54,6 +55,8 @@ struct Step3Args {
   const float* pl1;
   const void* grad;       // [nC][kGrad3] in the path's precision ([3][5] + pad)
   double* r_out;          // [nC][5] residual (residual-only launches)
+  double* fx;             // FP64 paths: face-flux buffer, [nF][6] (production:
+                          // projected on the area vector) or [nF][16] (exact)
   const double* scal;     // device [0] = dt (FP64 paths)
   const float* dt_ff;     // device dt as a float pair (FP32 path)
   int stage;              // 0: Q - dt/V R;  1: 0.5 Q0 + 0.5 (Q - dt/V R)

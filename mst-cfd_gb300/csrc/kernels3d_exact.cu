@@ -16,8 +16,8 @@ cudaError_t gradient(int, const DevMesh3& m, const Step3Args& a, void* grad, dou
 }
 cudaError_t flux_update(int, int order, bool visc, int mode, const DevMesh3& m,
                         const Step3Args& a, cudaStream_t s) {
-  if (mode == 3) return flux3_dispatch<double, 3>(order, visc, m, a, s);
-  return flux3_dispatch<double, 0>(order, visc, m, a, s);
+  if (mode == 3) return flux3_dispatch<false, 3>(order, visc, m, a, s);
+  return flux3_dispatch<false, 0>(order, visc, m, a, s);
 }
 cudaError_t finalize_dt(const double* part, int n, double t_end, double* scal, float* dt_ff,
                         cudaStream_t s) {
@@ -27,9 +27,13 @@ cudaError_t kinetic(int, const DevMesh3& m, const Step3Args& a, double* part, do
                     cudaStream_t s) {
   return kinetic3_t<0>(m, a, part, out, s);
 }
-cudaError_t pairs(bool to_pairs, double* q, int n, float4* h4, float* h1, float4* l4, float* l1,
-                  cudaStream_t s) {
-  return pairs3(to_pairs, q, n, h4, h1, l4, l1, s);
+cudaError_t pairs(bool to_pairs, double* q, const int* idx, int n, float4* h4, float* h1,
+                  float4* l4, float* l1, cudaStream_t s) {
+  return pairs3(to_pairs, q, idx, n, h4, h1, l4, l1, s);
+}
+cudaError_t rows(const void* src, bool src_f32, int ld, const int* idx, int n, int w, double* dst,
+                 cudaStream_t s) {
+  return rows3(src, src_f32, ld, idx, n, w, dst, s);
 }
 }  // namespace exact3
 }  // namespace mst

@@ -18,8 +18,10 @@ namespace mst {
                           float* dt_ff, cudaStream_t s);                                    \
   cudaError_t kinetic(int prec, const DevMesh3& m, const Step3Args& a, double* part,        \
                       double* out, cudaStream_t s);                                         \
-  cudaError_t pairs(bool to_pairs, double* q, int n, float4* h4, float* h1, float4* l4,     \
-                    float* l1, cudaStream_t s);
+  cudaError_t pairs(bool to_pairs, double* q, const int* idx, int n, float4* h4, float* h1, \
+                    float4* l4, float* l1, cudaStream_t s);                                  \
+  cudaError_t rows(const void* src, bool src_f32, int ld, const int* idx, int n, int w,     \
+                   double* dst, cudaStream_t s);
 namespace exact3 {
 MST_LAUNCH3D_DECLS
 }

@@ -293,6 +293,7 @@ int build_layout3d(const SolverMesh3D& m, DevLayout3D* L, std::string* err) {
   }
   const int tot = L->c_ptr[nC];
   L->cf_slot.assign(tot, 0);
+  L->cf_face.assign(tot, 0);
   L->cf_nb.assign(tot, -1);
   L->cf_w.assign(2 * (size_t)tot, 0.0);
   L->cf_dir.assign(3 * (size_t)tot, 0.0);
@@ -319,6 +320,7 @@ int build_layout3d(const SolverMesh3D& m, DevLayout3D* L, std::string* err) {
         }
         const bool own = m.face_cells[2 * (size_t)f] == c;
         L->cf_slot[dk] = (slot << 1) | (own ? 0 : 1);
+        L->cf_face[dk] = own ? df : ~df;
         const int nb = m.cell_nb[k];
         L->cf_nb[dk] = nb >= 0 ? L->cell_perm[nb] : -1;
         L->cf_w[2 * (size_t)dk] = m.cell_w[2 * (size_t)k];

@@ -51,6 +51,7 @@ struct DevLayout3D {
   std::vector<double> f_eta;                // [nF]
   std::vector<double> c_vol;                // [nC]
   std::vector<int> c_ptr, cf_slot, cf_nb;   // cf_slot = tile slot << 1 | (cell is c1)
+  std::vector<int> cf_face;                 // device face, ~face where the cell is c1
   std::vector<double> cf_w, cf_dir;         // [tot][2], [tot][3]
   std::vector<int> t_own_ptr, t_bor_ptr, t_bor;
 };
