@@ -13,17 +13,17 @@ constexpr int kGrad3 = 16;
 // 3D mesh in device order (mesh3d.hpp DevLayout3D): FP64 vectors of 3
 // packed (x, y, z) per face or cell-face, and FP32 copies packed in float4
 struct DevMesh3 {
-  int n_cells, n_faces, n_tiles, max_tile_faces;
+  int n_cells, n_faces;
   const int2* f_c0c1;
   const int* f_info;
   const double *f_dir, *f_r0, *f_r1, *f_eta;
   // FP32 copies packed for one 16-byte load each: (S, eta0), (r0, 0), (r1, 0)
-  const float4 *f_dir_eta32, *f_r0_32, *f_r1_32;
+  // and (r0 - r1, 0)
+  const float4 *f_dir_eta32, *f_r0_32, *f_r1_32, *f_d32;
   const double* c_vol;
   const double* c_ivol;     // 1/V
   const float2* c_ivol_ff;  // 1/V as a float pair
   const int* c_ptr;
-  const int* cf_slot;       // tile slot << 1 | (cell is c1 of the face)
   const int* cf_face;       // device face, ~face where the cell is its c1
   const int* cf_nb;         // neighbour device cell, -1 on boundary faces
   const double* cf_w;       // [tot][2] face-value weights (self, neighbour)
@@ -31,7 +31,6 @@ struct DevMesh3 {
   // FP32 copies: (outward S, self weight) and the neighbour weight
   const float4* cf_dw32;
   const float* cf_w1_32;
-  const int *t_own_ptr, *t_bor_ptr, *t_bor;
 };
 
 // One stage of the 3D path.  FP64 state: q [nC][5].  FP32 path: the state
@@ -57,6 +56,8 @@ struct Step3Args {
   double* r_out;          // [nC][5] residual (residual-only launches)
   double* fx;             // FP64 paths: face-flux buffer, [nF][6] (production:
                           // projected on the area vector) or [nF][16] (exact)
+  float4* fx4;            // FP32 path: the projected flux, components 0-3
+  float* fx1;             // and 4
   const double* scal;     // device [0] = dt (FP64 paths)
   const float* dt_ff;     // device dt as a float pair (FP32 path)
   int stage;              // 0: Q - dt/V R;  1: 0.5 Q0 + 0.5 (Q - dt/V R)

@@ -34,7 +34,7 @@ struct mst_ctx3d {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   mst::DevMesh3 dm{};
   const int *cell_perm = nullptr, *cell_iperm = nullptr;  // device: file -> device cell, back
-  int n_cell_faces = 0, n_borrowed = 0;
+  int n_cell_faces = 0, n_borrowed = 0, n_tiles = 0, max_tile_faces = 0;
   std::vector<void*> allocs;
   size_t bytes = 0;
   // FP64 state buffers (cur, stage, next) or float pairs for the FP32 path
@@ -43,7 +43,10 @@ struct mst_ctx3d {
   float *h1[3] = {}, *l1[3] = {};
   double* qtmp = nullptr;  // [nC][5] state in file order on its way in or out / residual
   double* file = nullptr;  // [nC][15] rows in file order of the residual and gradient exports
-  double* fx = nullptr;    // face-flux buffer of the FP64 paths
+  // face-flux buffer: FP64 paths, FP32 path
+  double* fx = nullptr;
+  float4* fx4 = nullptr;
+  float* fx1 = nullptr;
   void* grad = nullptr;
   double* dt_part = nullptr;
   double* scal = nullptr;  // [0] dt, [1] time
@@ -168,6 +171,8 @@ mst::Step3Args args3(mst_ctx3d* c, int in, int out, int prev, int stage) {
   }
   a.grad = c->grad;
   a.fx = c->fx;
+  a.fx4 = c->fx4;
+  a.fx1 = c->fx1;
   a.scal = c->scal;
   a.dt_ff = c->dt_ff;
   a.stage = stage;
@@ -198,7 +203,7 @@ cudaError_t grad3(mst_ctx3d* c, const mst::Step3Args& a, double* dt_part) {
 
 cudaError_t flux3(mst_ctx3d* c, const mst::Step3Args& a, int mode) {
   Prof3 pr(c, "k3_flux_update");
-  c->last_launches += f32(c) ? 1 : 2;  // FP64: the face / cell kernel pair
+  c->last_launches += 2;  // the face / cell kernel pair
   return exact3(c) ? mst::exact3::flux_update(c->p.precision, c->p.order, c->p.viscous != 0,
                                               mode, c->dm, a, c->stream)
                    : mst::fast3::flux_update(c->p.precision, c->p.order, c->p.viscous != 0,
@@ -325,8 +330,8 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
   mst::DevMesh3& d = c->dm;
   d.n_cells = nC;
   d.n_faces = nF;
-  d.n_tiles = L.n_tiles;
-  d.max_tile_faces = std::max(L.max_tile_faces, 1);
+  c->n_tiles = L.n_tiles;
+  c->max_tile_faces = std::max(L.max_tile_faces, 1);
   std::vector<int2> c0c1(nF);
   for (int f = 0; f < nF; ++f) c0c1[f] = make_int2(L.f_c0c1[2 * (size_t)f], L.f_c0c1[2 * (size_t)f + 1]);
   std::vector<double> ivol(nC);
@@ -337,7 +342,7 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
     ivff[i] = make_float2(hi, (float)(ivol[i] - (double)hi));
   }
   // packed FP32 copies of the geometry
-  std::vector<float4> fde(nF), fr0(nF), fr1(nF), cdw(tot);
+  std::vector<float4> fde(nF), fr0(nF), fr1(nF), fd(nF), cdw(tot);
   std::vector<float> cw1(tot);
   for (int f = 0; f < nF; ++f) {
     const double* dv = &L.f_dir[3 * (size_t)f];
@@ -346,6 +351,7 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
     fde[f] = make_float4((float)dv[0], (float)dv[1], (float)dv[2], (float)L.f_eta[f]);
     fr0[f] = make_float4((float)a0[0], (float)a0[1], (float)a0[2], 0.0f);
     fr1[f] = make_float4((float)a1[0], (float)a1[1], (float)a1[2], 0.0f);
+    fd[f] = make_float4((float)(a0[0] - a1[0]), (float)(a0[1] - a1[1]), (float)(a0[2] - a1[2]), 0.0f);
   }
   for (int k = 0; k < tot; ++k) {
     const double* dv = &L.cf_dir[3 * (size_t)k];
@@ -358,19 +364,16 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
       (st = upload3(c.get(), &d.f_r1, L.f_r1)) || (st = upload3(c.get(), &d.f_eta, L.f_eta)) ||
       (st = upload3(c.get(), &d.f_dir_eta32, fde)) ||
       (st = upload3(c.get(), &d.f_r0_32, fr0)) || (st = upload3(c.get(), &d.f_r1_32, fr1)) ||
+      (st = upload3(c.get(), &d.f_d32, fd)) ||
       (st = upload3(c.get(), &d.c_vol, L.c_vol)) ||
       (st = upload3(c.get(), &d.c_ivol, ivol)) || (st = upload3(c.get(), &d.c_ivol_ff, ivff)) ||
       (st = upload3(c.get(), &d.c_ptr, L.c_ptr)) ||
-      (st = upload3(c.get(), &d.cf_slot, L.cf_slot)) ||
       (st = upload3(c.get(), &d.cf_face, L.cf_face)) ||
       (st = upload3(c.get(), &c->cell_perm, L.cell_perm)) ||
       (st = upload3(c.get(), &c->cell_iperm, L.cell_iperm)) ||
       (st = upload3(c.get(), &d.cf_nb, L.cf_nb)) || (st = upload3(c.get(), &d.cf_w, L.cf_w)) ||
       (st = upload3(c.get(), &d.cf_dir, L.cf_dir)) ||
-      (st = upload3(c.get(), &d.cf_dw32, cdw)) || (st = upload3(c.get(), &d.cf_w1_32, cw1)) ||
-      (st = upload3(c.get(), &d.t_own_ptr, L.t_own_ptr)) ||
-      (st = upload3(c.get(), &d.t_bor_ptr, L.t_bor_ptr)) ||
-      (st = upload3(c.get(), &d.t_bor, L.t_bor))) {
+      (st = upload3(c.get(), &d.cf_dw32, cdw)) || (st = upload3(c.get(), &d.cf_w1_32, cw1))) {
     cleanup();
     return st;
   }
@@ -388,6 +391,7 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
       (st = alloc3(c.get(), (char**)&c->grad,
                    mst::kGrad3 * (size_t)nC * (pairs ? sizeof(float) : sizeof(double)))) ||
       (!pairs && (st = alloc3(c.get(), &c->fx, (exact3(c.get()) ? 16 : 6) * (size_t)nF))) ||
+      (pairs && ((st = alloc3(c.get(), &c->fx4, nF)) || (st = alloc3(c.get(), &c->fx1, nF)))) ||
       (st = alloc3(c.get(), &c->dt_part, nb)) || (st = alloc3(c.get(), &c->scal, 2)) ||
       (st = alloc3(c.get(), &c->dt_ff, 2)) || (st = alloc3(c.get(), &c->ke_part, 2 * (size_t)nb)) ||
       (st = alloc3(c.get(), &c->ke_out, 2))) {
@@ -424,8 +428,8 @@ mst_status mst_ctx3d_info_get(mst_ctx3d* c, mst_ctx3d_info* info) {
   if (!c || !info) return fail3(MST_EINVAL, "NULL argument");
   info->n_cells = c->dm.n_cells;
   info->n_faces = c->dm.n_faces;
-  info->n_tiles = c->dm.n_tiles;
-  info->max_tile_faces = c->dm.max_tile_faces;
+  info->n_tiles = c->n_tiles;
+  info->max_tile_faces = c->max_tile_faces;
   info->n_cell_faces = c->n_cell_faces;
   info->n_borrowed = c->n_borrowed;
   info->device_bytes = c->bytes;
