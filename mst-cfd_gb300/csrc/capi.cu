@@ -265,9 +265,7 @@ mst_status launch_grad(mst_ctx* c, const double4_32a* q, const float4* qf = null
 
 mst_status launch_flux(mst_ctx* c, const mst::StepArgs& a) {
   if (a.fx) c->last_launches++;  // the face / cell kernel pair
-  ProfScope ps(c, c->p.precision != MST_PREC_FP32 ? "k_flux_update<f64>"
-                  : a.tile_grad                   ? "k_flux_update<f32,tg>"
-                                                  : "k_flux_update<f32>");
+  ProfScope ps(c, c->p.precision != MST_PREC_FP32 ? "k_flux_update<f64>" : "k_flux_update<f32>");
   cudaError_t e = (c->p.precision == MST_PREC_FP64_EXACT)
                       ? mst::exact::launch_flux_update(prec_of(c->p), c->p.flux, c->p.order,
                                                        c->dm, a, 0, c->stream)
@@ -279,23 +277,6 @@ mst_status launch_flux(mst_ctx* c, const mst::StepArgs& a) {
 }
 
 bool pairs(const mst_ctx* c) { return c->p.precision == MST_PREC_FP32; }
-
-// The viscous FP32 float-pair path at 2nd order in the corrected mode forms
-// its gradients inside the flux kernel (k_flux_update TG: no gradient pass,
-// no gradient through HBM); measured faster there, while the inviscid stage
-// keeps the gradient pass (its flux kernel alone is issue-bound, and the
-// tile's gradient phases add latency that the pass hides better).  Both
-// schedules give bit-identical states.  MSTCFD_FP32_GRADIENT_PASS=1 / =0 in
-// the environment forces one schedule, to compare them.
-bool tile_grad(const mst_ctx* c) {
-  static const int force = [] {
-    const char* e = std::getenv("MSTCFD_FP32_GRADIENT_PASS");
-    return e ? (e[0] == '1' ? 1 : 0) : -1;
-  }();
-  const bool can = pairs(c) && c->p.order == 2 && c->p.reference_quirks == 0;
-  if (force >= 0) return can && force == 0;
-  return can && c->p.viscous;
-}
 
 // double copies of the float-pair states (device order) for the entry
 // points that read the FP64 buffers
@@ -372,8 +353,7 @@ mst_status run_stage(mst_ctx* c, const StageBufs& b, int stage, bool fixed_dt, b
   double4_32a* qn = b.qn;
   const float4* qf = pairs(c) ? b.qf : nullptr;
   float4* qfn = pairs(c) ? b.qfn : nullptr;
-  const bool tg = tile_grad(c);
-  if (c->p.order == 2 && !grad_ready && !tg) {
+  if (c->p.order == 2 && !grad_ready) {
     mst_status s = launch_grad(c, q, qf);
     if (s) return s;
   }
@@ -381,7 +361,6 @@ mst_status run_stage(mst_ctx* c, const StageBufs& b, int stage, bool fixed_dt, b
   a.q = q;
   a.qf = qf;
   a.qfn = qfn;
-  a.tile_grad = tg ? 1 : 0;
   if (pairs(c)) {
     a.qlo = b.ql;
     a.qlon = b.qln;
@@ -414,16 +393,7 @@ mst_status compute_dt(mst_ctx* c, const double4_32a* q, double t_end,
                       const float4* qf = nullptr, bool* grad_ready = nullptr) {
   const int nC = c->dm.n_cells;
   int mode = 0;
-  if (c->p.dt_mode != MST_DT_FIXED && tile_grad(c)) {
-    // no gradient pass on this schedule: the step from the FP32 state alone
-    ProfScope ps(c, "k_cfl_dt_pairs");
-    cudaError_t e = mst::fast::launch_cfl_dt_pairs(
-        c->dm, qf, c->p.cfl, c->p.dt_mode == MST_DT_CFL_LOCAL ? c->dt_cell_ff : nullptr,
-        c->dt_part, c->stream);
-    c->last_launches++;
-    if (e != cudaSuccess) return fail(MST_ECUDA, std::string("cfl_dt: ") + cudaGetErrorString(e));
-    mode = 1;
-  } else if (c->p.dt_mode != MST_DT_FIXED && c->p.order == 2 && grad_ready) {
+  if (c->p.dt_mode != MST_DT_FIXED && c->p.order == 2 && grad_ready) {
     mst_status st = launch_grad(c, q, qf, c->dt_part, c->p.dt_mode == MST_DT_CFL_LOCAL);
     if (st) return st;
     *grad_ready = true;
@@ -679,7 +649,7 @@ mst_status mst_mesh_get_info(const mst_mesh* m, mst_mesh_info* info) {
   info->n_bond2 = (int)h.bond2.size();
   info->n_tiles = m->lay.n_tiles;
   info->n_borrowed = (int)m->lay.t_bor.size();
-  info->n_halo = (int)m->lay.t_halo.size();
+  info->n_halo = m->lay.n_halo;
   info->n_halo_cells = m->lay.n_halo_cells;
   info->n_halo_cell_faces = m->lay.n_halo_cell_faces;
   return MST_OK;
@@ -756,10 +726,16 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
     CU(up(&d.f_r0, as_d2(L.f_r0)));
     CU(up(&d.f_r1, as_d2(L.f_r1)));
     CU(up(&d.cf_w, as_d2(L.cf_w)));
-    CU(up(&d.f_dir32, as_f2(L.f_dir)));
     CU(up(&d.f_r0_32, as_f2(L.f_r0)));
     CU(up(&d.f_r1_32, as_f2(L.f_r1)));
-    CU(up(&d.cf_w32, as_f2(L.cf_w)));
+    {
+      std::vector<float4> dd(L.n_faces);
+      for (size_t f = 0; f < dd.size(); ++f)
+        dd[f] = make_float4((float)L.f_dir[2 * f], (float)L.f_dir[2 * f + 1],
+                            (float)(L.f_r0[2 * f] - L.f_r1[2 * f]),
+                            (float)(L.f_r0[2 * f + 1] - L.f_r1[2 * f + 1]));
+      CU(up(&d.f_dd32, dd));
+    }
     {
       std::vector<double> cd(2 * L.cf_face.size());
       for (size_t k = 0; k < L.cf_face.size(); ++k) {
@@ -774,6 +750,36 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
       for (size_t k = 0; k < len.size(); ++k)
         len[k] = std::sqrt(cd[2 * k] * cd[2 * k] + cd[2 * k + 1] * cd[2 * k + 1]);
       CU(up(&d.cf_len, len));
+      // the FP32 tables by face position
+      int deg = 0;
+      for (int i = 0; i < L.n_cells; ++i) deg = std::max(deg, L.c_ptr[i + 1] - L.c_ptr[i]);
+      const size_t n = L.n_cells;
+      std::vector<int> nb(deg * n), slot(deg * n, -1);
+      std::vector<float4> wd(deg * n, make_float4(0.f, 0.f, 0.f, 0.f));
+      for (size_t at = 0; at < nb.size(); ++at) nb[at] = (int)(at % n);
+      int4 quirk = make_int4(-1, -1, -1, -1);
+      for (size_t i = 0; i < n; ++i)
+        for (int k = L.c_ptr[i]; k < L.c_ptr[i + 1]; ++k) {
+          const size_t at = (size_t)(k - L.c_ptr[i]) * n + i, k2 = 2 * (size_t)k;
+          const int mode = L.cf_nb_fix[k] >> mst::kFvShift;
+          const int modeq = L.cf_nb[k] >> mst::kFvShift;
+          if (mode != mst::kFvSelf) nb[at] = L.cf_nb_fix[k] & ((1 << mst::kFvShift) - 1);
+          slot[at] = L.cf_slot[k];
+          // a face without interpolation takes one side's value
+          const bool in = mode == mst::kFvInterp;
+          wd[at] = make_float4(in ? (float)L.cf_w[k2] : (mode == mst::kFvSelf ? 1.f : 0.f),
+                               in ? (float)L.cf_w[k2 + 1] : (mode == mst::kFvSelf ? 0.f : 1.f),
+                               (float)cd[k2], (float)cd[k2 + 1]);
+          if (modeq != mode && modeq == mst::kFvSelf)
+            quirk.x = (int)i, quirk.y = k - L.c_ptr[i];
+          if (modeq != mode && modeq == mst::kFvNb)
+            quirk.z = (int)i, quirk.w = k - L.c_ptr[i];
+        }
+      c->dm.quirk_at = quirk;
+      CU(up(&d.e_nb, nb));
+      CU(up(&d.e_slot, slot));
+      CU(up(&d.e_wd, wd));
+      c->dm.e_deg = deg;
     }
     {
       std::vector<double> fe(L.n_faces);
@@ -804,10 +810,6 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
     CU(up(&d.t_own_ptr, L.t_own_ptr));
     CU(up(&d.t_bor_ptr, L.t_bor_ptr));
     CU(up(&d.t_bor, L.t_bor));
-    CU(up(&d.t_halo_ptr, L.t_halo_ptr));
-    CU(up(&d.t_halo, L.t_halo));
-    CU(up(&d.t_slot_loc, L.t_slot_loc));
-    CU(up(&d.cf_nbl, L.cf_nbl));
     CU(up(&d.cell_iperm, L.cell_iperm));
     CU(up(&d.cell_perm, L.cell_perm));
   }
@@ -821,7 +823,7 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
   dm.f_dir = d.f_dir;
   dm.f_r0 = d.f_r0;
   dm.f_r1 = d.f_r1;
-  dm.f_dir32 = d.f_dir32;
+  dm.f_dd32 = d.f_dd32;
   dm.f_r0_32 = d.f_r0_32;
   dm.f_r1_32 = d.f_r1_32;
   dm.f_eta = d.f_eta;
@@ -835,18 +837,15 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
   dm.cf_nb = d.cf_nb;
   dm.cf_nb_fix = d.cf_nb_fix;
   dm.cf_w = d.cf_w;
-  dm.cf_w32 = d.cf_w32;
   dm.cf_dir = d.cf_dir;
   dm.cf_dir32 = d.cf_dir32;
   dm.cf_len = d.cf_len;
   dm.t_own_ptr = d.t_own_ptr;
   dm.t_bor_ptr = d.t_bor_ptr;
   dm.t_bor = d.t_bor;
-  dm.t_halo_ptr = d.t_halo_ptr;
-  dm.t_halo = d.t_halo;
-  dm.t_slot_loc = d.t_slot_loc;
-  dm.cf_nbl = d.cf_nbl;
-  dm.max_halo = L.max_halo;
+  dm.e_nb = d.e_nb;
+  dm.e_wd = d.e_wd;
+  dm.e_slot = d.e_slot;
   dm.deg3 = 1;
   for (int i = 0; i <= L.n_cells && dm.deg3; ++i) dm.deg3 = L.c_ptr[i] == 3 * i;
   const size_t nC = L.n_cells, nB = (nC + 255) / 256;

@@ -31,8 +31,8 @@ struct DevArrays {
   int* f_info = nullptr;
   double2 *f_dir = nullptr, *f_r0 = nullptr, *f_r1 = nullptr, *cf_w = nullptr,
           *cf_dir = nullptr;
-  float2 *f_dir32 = nullptr, *f_r0_32 = nullptr, *f_r1_32 = nullptr, *cf_w32 = nullptr,
-         *cf_dir32 = nullptr;
+  float2 *f_r0_32 = nullptr, *f_r1_32 = nullptr, *cf_dir32 = nullptr;
+  float4 *f_dd32 = nullptr, *e_wd = nullptr;
   double* f_eta = nullptr;
   float* f_eta32 = nullptr;
   double* cf_len = nullptr;
@@ -42,7 +42,7 @@ struct DevArrays {
   int *c_ptr = nullptr, *cf_face = nullptr, *cf_slot = nullptr, *cf_nb = nullptr,
       *cf_nb_fix = nullptr, *t_own_ptr = nullptr, *t_bor_ptr = nullptr,
       *t_bor = nullptr, *cell_iperm = nullptr, *cell_perm = nullptr,
-      *t_halo_ptr = nullptr, *t_halo = nullptr, *t_slot_loc = nullptr, *cf_nbl = nullptr;
+      *e_nb = nullptr, *e_slot = nullptr;
 };
 
 struct mst_node_avg;  // result writer buffers (io.cu)

@@ -18,7 +18,7 @@ struct DevMesh {
   const double2* f_dir;
   const double2* f_r0;
   const double2* f_r1;
-  const float2* f_dir32;
+  const float4* f_dd32;   // (area vector, x_c1 - x_c0)
   const float2* f_r0_32;
   const float2* f_r1_32;
   const double* f_eta;    // eta0 per face (viscous face interpolation)
@@ -32,7 +32,6 @@ struct DevMesh {
   const int* cf_nb;
   const int* cf_nb_fix;
   const double2* cf_w;
-  const float2* cf_w32;
   // area vector of every cell-face, pointing out of the cell (the signed
   // f_dir of cf_face): a contiguous load instead of a gather
   const double2* cf_dir;
@@ -41,13 +40,18 @@ struct DevMesh {
   const int* t_own_ptr;
   const int* t_bor_ptr;
   const int* t_bor;
-  // fused FP32 tile pass (mesh.hpp DevLayout): halo cells per tile, local
-  // cell indices of every tile face slot and of every cell-face neighbour
-  const int* t_halo_ptr;
-  const int* t_halo;
-  const int* t_slot_loc;
-  const int* cf_nbl;
-  int max_halo;
+  // FP32 path: the cell-face tables by face position, [e_deg][n_cells]: the
+  // neighbour (boundary and absent faces: the cell itself), (weights of the
+  // cell and the neighbour, outward area vector; boundary (1, 0, S), absent
+  // zero), tile slot << 1 | sign (absent: -1).  A warp's loads are
+  // contiguous, where the CSR tables' were strided by the faces of a cell.
+  int e_deg;
+  const int* e_nb;
+  const float4* e_wd;
+  const int* e_slot;
+  // the interior face whose value the reference's boundary loop overwrites:
+  // (cell, position) of its c0 side and of its c1 side, -1 where none
+  int4 quirk_at;
   int deg3;  // every cell has three faces and c_ptr[c] = 3c (triangles)
   // batches (nullptr for a single mesh): the case of every device cell and
   // the iteration at which each case converged (-1 while it runs).  The
@@ -126,8 +130,6 @@ struct StepArgs {
   double dt;              // fixed step
   int stage;              // 0: Q - dt/V R;  1: 0.5 Q0 + 0.5 (Q - dt/V R)
   int quirks;             // reproduce the reference's quirks
-  int tile_grad;          // FP32 pairs, 2nd order, corrected mode: the flux
-                          // kernel forms the gradients itself (grad unused)
   int limiter;            // MST_LIMITER_*
   double inlet[4];
   int viscous;            // laminar viscous term on
@@ -274,9 +276,6 @@ enum { kFluxAusm = 0, kFluxRoe = 1 };
                               int threads, bool turn, cudaStream_t s);        \
   cudaError_t lusgs_backward_t(const DevMesh& m, const LusgsArgs& a,         \
                                int threads, cudaStream_t s);                  \
-  cudaError_t launch_cfl_dt_pairs(const DevMesh& m, const float4* qf,        \
-                                  double cfl, float2* dt_cell_ff,             \
-                                  double* dt_part, cudaStream_t s);           \
   cudaError_t case_norms_t(const DevMesh& m, const CaseNormArgs& a,          \
                            int n_cases, cudaStream_t s);                      \
   }

@@ -9,9 +9,10 @@ namespace mst {
 // Gradient record per cell: [3][5] plus one pad, so that a cell's gradient
 // is 64 B (FP32) or 128 B (FP64), loaded and stored as aligned vectors.
 constexpr int kGrad3 = 16;
+constexpr int kNoFace3 = 0x7fffffff;
 
 // 3D mesh in device order (mesh3d.hpp DevLayout3D): FP64 vectors of 3
-// packed (x, y, z) per face or cell-face, and FP32 copies packed in float4
+// packed (x, y, z) per face or cell-face (FP64 paths), FP32 tables (FP32 path)
 struct DevMesh3 {
   int n_cells, n_faces;
   const int2* f_c0c1;
@@ -28,9 +29,15 @@ struct DevMesh3 {
   const int* cf_nb;         // neighbour device cell, -1 on boundary faces
   const double* cf_w;       // [tot][2] face-value weights (self, neighbour)
   const double* cf_dir;     // [tot][3] outward area vector
-  // FP32 copies: (outward S, self weight) and the neighbour weight
-  const float4* cf_dw32;
-  const float* cf_w1_32;
+  // FP32 path: the cell-face tables by face position, [e_deg][n_cells]: the
+  // neighbour (boundary and absent faces: the cell itself), (outward S, self
+  // weight), the neighbour weight (boundary 1 and 0, absent all zero), the
+  // device face as cf_face (absent: kNoFace3).  A warp's loads are contiguous.
+  int e_deg;
+  const int* e_nb;
+  const float4* e_dw;
+  const float* e_w1;
+  const int* e_face;
 };
 
 // One stage of the 3D path.  FP64 state: q [nC][5].  FP32 path: the state

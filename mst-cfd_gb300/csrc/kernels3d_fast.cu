@@ -4,6 +4,7 @@
 #include "launch3d.hpp"
 #include "mesh.hpp"
 #include "physics.cuh"
+#include "vec8.cuh"
 
 namespace mst {
 namespace fast3 {

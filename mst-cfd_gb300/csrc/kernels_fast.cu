@@ -5,6 +5,7 @@
 #include "devtypes.hpp"
 #include "mesh.hpp"
 #include "physics.cuh"
+#include "vec8.cuh"
 
 namespace mst {
 namespace fast {

@@ -8,6 +8,7 @@
 #pragma once
 #include <cstdint>
 #include <string>
+#include <algorithm>
 #include <vector>
 
 namespace mst {
@@ -141,24 +142,37 @@ struct DevLayout {
   std::vector<int> t_own_ptr;   // [nT+1] owned face range (device ids)
   std::vector<int> t_bor_ptr;   // [nT+1] into t_bor
   std::vector<int> t_bor;       // borrowed device face ids
-  // fused FP32 tile pass (gradients formed in shared memory): per tile a
-  // table of its cells (local 0..kTileCells-1) followed by its halo cells
-  // (outside the tile, sharing an interior face with a tile cell)
-  std::vector<int> t_halo_ptr;  // [nT+1] into t_halo
-  std::vector<int> t_halo;      // halo device cells, ascending per tile
-  std::vector<int> t_slot_loc;  // per tile face slot (tile t's slots start at
-                                // t_own_ptr[t] + t_bor_ptr[t]): local index
-                                // of c0 | local index of c1 << 16 (0xFFFF:
-                                // boundary face)
-  std::vector<int> cf_nbl;      // [tot] local index of the neighbour in its
-                                // cell's tile table | corrected face-value
-                                // mode << 16
-  int max_halo = 0;
+  // halo: cells outside a tile that share an interior face with one of its
+  // cells, over all tiles (layout statistics)
+  int n_halo = 0;
   int n_halo_cells = 0;       // distinct cells in some tile's halo
   int n_halo_cell_faces = 0;  // their cell-faces
 };
 
 int build_layout(const HostMesh& m, bool renumber, DevLayout* L,
                  std::string* err);
+
+// Faces in ascending (lower device cell, higher device cell): iperm[i] is the
+// face at place i, low[f] the lower cell of face f.  cell(f, side): device
+// cell of a side, -1 beyond the boundary.  Ties keep the faces' own order.
+template <class Cell>
+void order_faces_by_cell(int nF, int nC, Cell cell, std::vector<int>* iperm,
+                         std::vector<int>* low) {
+  std::vector<int> at((size_t)nC + 1, 0), high(nF);
+  low->resize(nF);
+  for (int f = 0; f < nF; ++f) {
+    const int a = cell(f, 0), b = cell(f, 1);
+    (*low)[f] = b >= 0 ? std::min(a, b) : a;
+    high[f] = std::max(a, b);
+    at[(*low)[f] + 1]++;
+  }
+  for (int c = 0; c < nC; ++c) at[c + 1] += at[c];
+  iperm->resize(nF);
+  std::vector<int> fill(at.begin(), at.end() - 1);
+  for (int f = 0; f < nF; ++f) (*iperm)[fill[(*low)[f]]++] = f;
+  for (int c = 0; c < nC; ++c)
+    std::stable_sort(iperm->begin() + at[c], iperm->begin() + at[c + 1],
+                     [&](int x, int y) { return high[x] < high[y]; });
+}
 
 }  // namespace mst

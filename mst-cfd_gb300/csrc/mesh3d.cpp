@@ -215,27 +215,18 @@ int build_layout3d(const SolverMesh3D& m, DevLayout3D* L, std::string* err) {
   for (int i = 0; i < nC; ++i) L->cell_perm[L->cell_iperm[i]] = i;
   const int nT = (nC + kTileCells - 1) / kTileCells;
   L->n_tiles = nT;
-  std::vector<int> owner(nF);
-  for (int f = 0; f < nF; ++f) {
-    const int a = L->cell_perm[m.face_cells[2 * (size_t)f]];
-    const int c1 = m.face_cells[2 * (size_t)f + 1];
-    const int b = c1 >= 0 ? L->cell_perm[c1] : a;
-    owner[f] = std::min(a, b) / kTileCells;
-  }
-  // device faces grouped by owner tile (counting sort, file order within)
-  L->t_own_ptr.assign(nT + 1, 0);
-  for (int f = 0; f < nF; ++f) L->t_own_ptr[owner[f] + 1]++;
-  for (int t = 0; t < nT; ++t) L->t_own_ptr[t + 1] += L->t_own_ptr[t];
+  // faces by the lower, then the higher device cell (a warp's faces gather
+  // from neighbouring cells); a tile owns those whose lower cell is its own
+  std::vector<int> owner, face_iperm;
+  order_faces_by_cell(nF, nC, [&](int f, int side) {
+    const int c = m.face_cells[2 * (size_t)f + side];
+    return c >= 0 ? L->cell_perm[c] : -1;
+  }, &face_iperm, &owner);
   L->face_perm.assign(nF, 0);
-  std::vector<int> face_iperm(nF);
-  {
-    std::vector<int> fill(L->t_own_ptr.begin(), L->t_own_ptr.end() - 1);
-    for (int f = 0; f < nF; ++f) {
-      const int df = fill[owner[f]]++;
-      L->face_perm[f] = df;
-      face_iperm[df] = f;
-    }
-  }
+  for (int i = 0; i < nF; ++i) L->face_perm[face_iperm[i]] = i;
+  L->t_own_ptr.assign(nT + 1, 0);
+  for (int f = 0; f < nF; ++f) L->t_own_ptr[owner[f] / kTileCells + 1]++;
+  for (int t = 0; t < nT; ++t) L->t_own_ptr[t + 1] += L->t_own_ptr[t];
   // borrowed faces: cut faces owned by the other tile, ascending device id
   L->t_bor_ptr.assign(nT + 1, 0);
   for (int f = 0; f < nF; ++f) {

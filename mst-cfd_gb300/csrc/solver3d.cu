@@ -334,51 +334,75 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
   c->max_tile_faces = std::max(L.max_tile_faces, 1);
   std::vector<int2> c0c1(nF);
   for (int f = 0; f < nF; ++f) c0c1[f] = make_int2(L.f_c0c1[2 * (size_t)f], L.f_c0c1[2 * (size_t)f + 1]);
-  std::vector<double> ivol(nC);
-  std::vector<float2> ivff(nC);
-  for (int i = 0; i < nC; ++i) {
-    ivol[i] = 1.0 / L.c_vol[i];
-    const float hi = (float)ivol[i];
-    ivff[i] = make_float2(hi, (float)(ivol[i] - (double)hi));
-  }
-  // packed FP32 copies of the geometry
-  std::vector<float4> fde(nF), fr0(nF), fr1(nF), fd(nF), cdw(tot);
-  std::vector<float> cw1(tot);
-  for (int f = 0; f < nF; ++f) {
-    const double* dv = &L.f_dir[3 * (size_t)f];
-    const double* a0 = &L.f_r0[3 * (size_t)f];
-    const double* a1 = &L.f_r1[3 * (size_t)f];
-    fde[f] = make_float4((float)dv[0], (float)dv[1], (float)dv[2], (float)L.f_eta[f]);
-    fr0[f] = make_float4((float)a0[0], (float)a0[1], (float)a0[2], 0.0f);
-    fr1[f] = make_float4((float)a1[0], (float)a1[1], (float)a1[2], 0.0f);
-    fd[f] = make_float4((float)(a0[0] - a1[0]), (float)(a0[1] - a1[1]), (float)(a0[2] - a1[2]), 0.0f);
-  }
-  for (int k = 0; k < tot; ++k) {
-    const double* dv = &L.cf_dir[3 * (size_t)k];
-    cdw[k] = make_float4((float)dv[0], (float)dv[1], (float)dv[2], (float)L.cf_w[2 * (size_t)k]);
-    cw1[k] = (float)L.cf_w[2 * (size_t)k + 1];
-  }
   mst_status st = MST_OK;
+  const bool pairs = f32(c.get());
   if ((st = upload3(c.get(), &d.f_c0c1, c0c1)) || (st = upload3(c.get(), &d.f_info, L.f_info)) ||
-      (st = upload3(c.get(), &d.f_dir, L.f_dir)) || (st = upload3(c.get(), &d.f_r0, L.f_r0)) ||
-      (st = upload3(c.get(), &d.f_r1, L.f_r1)) || (st = upload3(c.get(), &d.f_eta, L.f_eta)) ||
-      (st = upload3(c.get(), &d.f_dir_eta32, fde)) ||
-      (st = upload3(c.get(), &d.f_r0_32, fr0)) || (st = upload3(c.get(), &d.f_r1_32, fr1)) ||
-      (st = upload3(c.get(), &d.f_d32, fd)) ||
       (st = upload3(c.get(), &d.c_vol, L.c_vol)) ||
-      (st = upload3(c.get(), &d.c_ivol, ivol)) || (st = upload3(c.get(), &d.c_ivol_ff, ivff)) ||
-      (st = upload3(c.get(), &d.c_ptr, L.c_ptr)) ||
-      (st = upload3(c.get(), &d.cf_face, L.cf_face)) ||
       (st = upload3(c.get(), &c->cell_perm, L.cell_perm)) ||
-      (st = upload3(c.get(), &c->cell_iperm, L.cell_iperm)) ||
-      (st = upload3(c.get(), &d.cf_nb, L.cf_nb)) || (st = upload3(c.get(), &d.cf_w, L.cf_w)) ||
-      (st = upload3(c.get(), &d.cf_dir, L.cf_dir)) ||
-      (st = upload3(c.get(), &d.cf_dw32, cdw)) || (st = upload3(c.get(), &d.cf_w1_32, cw1))) {
+      (st = upload3(c.get(), &c->cell_iperm, L.cell_iperm))) {
     cleanup();
     return st;
   }
+  if (pairs) {
+    // the FP32 path's packed geometry
+    std::vector<float2> ivff(nC);
+    for (int i = 0; i < nC; ++i) {
+      const double iv = 1.0 / L.c_vol[i];
+      const float hi = (float)iv;
+      ivff[i] = make_float2(hi, (float)(iv - (double)hi));
+    }
+    std::vector<float4> fde(nF), fr0(nF), fr1(nF), fd(nF);
+    for (int f = 0; f < nF; ++f) {
+      const double* dv = &L.f_dir[3 * (size_t)f];
+      const double* a0 = &L.f_r0[3 * (size_t)f];
+      const double* a1 = &L.f_r1[3 * (size_t)f];
+      fde[f] = make_float4((float)dv[0], (float)dv[1], (float)dv[2], (float)L.f_eta[f]);
+      fr0[f] = make_float4((float)a0[0], (float)a0[1], (float)a0[2], 0.0f);
+      fr1[f] = make_float4((float)a1[0], (float)a1[1], (float)a1[2], 0.0f);
+      fd[f] = make_float4((float)(a0[0] - a1[0]), (float)(a0[1] - a1[1]), (float)(a0[2] - a1[2]),
+                          0.0f);
+    }
+    int deg = 0;
+    for (int i = 0; i < nC; ++i) deg = std::max(deg, L.c_ptr[i + 1] - L.c_ptr[i]);
+    const size_t n = nC;
+    std::vector<int> nb(deg * n), face(deg * n, mst::kNoFace3);
+    std::vector<float4> dw(deg * n, make_float4(0.f, 0.f, 0.f, 0.f));
+    std::vector<float> w1(deg * n, 0.f);
+    for (size_t at = 0; at < nb.size(); ++at) nb[at] = (int)(at % n);
+    for (int i = 0; i < nC; ++i)
+      for (int k = L.c_ptr[i]; k < L.c_ptr[i + 1]; ++k) {
+        const size_t at = (size_t)(k - L.c_ptr[i]) * n + i;
+        const double* dv = &L.cf_dir[3 * (size_t)k];
+        const bool in = L.cf_nb[k] >= 0;
+        if (in) nb[at] = L.cf_nb[k];
+        face[at] = L.cf_face[k];
+        dw[at] = make_float4((float)dv[0], (float)dv[1], (float)dv[2],
+                             in ? (float)L.cf_w[2 * (size_t)k] : 1.f);
+        w1[at] = in ? (float)L.cf_w[2 * (size_t)k + 1] : 0.f;
+      }
+    d.e_deg = deg;
+    if ((st = upload3(c.get(), &d.c_ivol_ff, ivff)) || (st = upload3(c.get(), &d.f_dir_eta32, fde)) ||
+        (st = upload3(c.get(), &d.f_r0_32, fr0)) || (st = upload3(c.get(), &d.f_r1_32, fr1)) ||
+        (st = upload3(c.get(), &d.f_d32, fd)) || (st = upload3(c.get(), &d.e_nb, nb)) ||
+        (st = upload3(c.get(), &d.e_face, face)) || (st = upload3(c.get(), &d.e_dw, dw)) ||
+        (st = upload3(c.get(), &d.e_w1, w1))) {
+      cleanup();
+      return st;
+    }
+  } else {
+    std::vector<double> ivol(nC);
+    for (int i = 0; i < nC; ++i) ivol[i] = 1.0 / L.c_vol[i];
+    if ((st = upload3(c.get(), &d.f_dir, L.f_dir)) || (st = upload3(c.get(), &d.f_r0, L.f_r0)) ||
+        (st = upload3(c.get(), &d.f_r1, L.f_r1)) || (st = upload3(c.get(), &d.f_eta, L.f_eta)) ||
+        (st = upload3(c.get(), &d.c_ivol, ivol)) || (st = upload3(c.get(), &d.c_ptr, L.c_ptr)) ||
+        (st = upload3(c.get(), &d.cf_face, L.cf_face)) ||
+        (st = upload3(c.get(), &d.cf_nb, L.cf_nb)) || (st = upload3(c.get(), &d.cf_w, L.cf_w)) ||
+        (st = upload3(c.get(), &d.cf_dir, L.cf_dir))) {
+      cleanup();
+      return st;
+    }
+  }
   const int nb = (nC + 63) / 64;  // step minima: FP64 gradient blocks of 64 cells
-  const bool pairs = f32(c.get());
   for (int i = 0; i < 3 && !st; ++i) {
     if (pairs) {
       (st = alloc3(c.get(), &c->h4[i], nC)) || (st = alloc3(c.get(), &c->h1[i], nC)) ||
