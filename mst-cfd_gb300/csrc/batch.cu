@@ -192,7 +192,7 @@ mst_status residual_pass(mst_batch* b, int which, bool lo, const mst::DevMesh& d
     if (exact(b) && !lo) e = mst::exact::launch_gradient(prec, dm, q, grad, 0, s);
     else if (qf)
       e = mst::fast::launch_gradient_dt(prec, dm, q, qf, grad, 0, 0.0, nullptr, nullptr,
-                                        nullptr, s);
+                                        nullptr, mst::FinishDt{}, s);
     else e = mst::fast::launch_gradient(prec, dm, q, grad, 0, s);
     if (e != cudaSuccess)
       return mst_internal_fail(MST_ECUDA, std::string("gradient: ") + cudaGetErrorString(e));
@@ -583,6 +583,9 @@ mst_status mst_batch_create(const mst_mesh* const* meshes, const mst_case_params
     return mst_internal_fail(rc == mst::kEMesh ? MST_EMESH : MST_EINVAL, err);
   }
   mst_status st = mst_ctx_create(b->mesh, p, &b->ctx);
+  // the FP64 sweeps, the FP32 residual phase and the FP32 sweeps
+  if (!st) st = mst_internal_geometry(b->ctx, false);
+  if (!st && (ip->fp32_until > 0 || b->sweep32)) st = mst_internal_geometry(b->ctx, true);
   auto cleanup = [&]() {
     if (b->ctx) mst_ctx_destroy(b->ctx);
     for (void* q : b->allocs) cudaFree(q);

@@ -87,76 +87,84 @@ __global__ void k_from_pairs(const float4* __restrict__ hi, const float4* __rest
                           (double)h.z + (double)l.z, (double)h.w + (double)l.w);
 }
 
-// step length: fixed (mode 0) or min over block partials (mode 1), clipped
-// so that the time reaches t_end; writes scal[0] = dt
-__global__ void k_finalize_dt(const double* __restrict__ part, int n,
-                              int mode, double dt_fixed, double t_end,
-                              double* __restrict__ scal) {
+// the CFL step from the block minima of a launch of many blocks
+__global__ void __launch_bounds__(1024) k_finalize_dt(const double* __restrict__ part, int n,
+                                                      const mst::FinishDt f) {
   __shared__ double red[32];
   double x = 1e300;
-  if (mode == 0) {
-    x = dt_fixed;
-  } else {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) x = (part[i] < x) ? part[i] : x;
-    for (int o = 16; o > 0; o >>= 1) {
-      double w = __shfl_xor_sync(0xffffffffu, x, o);
-      x = (w < x) ? w : x;
-    }
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      x = red[0];
-      for (int i = 1; i < (int)(blockDim.x >> 5); ++i) x = (red[i] < x) ? red[i] : x;
-    }
+  for (int i = threadIdx.x; i < n; i += blockDim.x) x = (part[i] < x) ? part[i] : x;
+  for (int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_xor_sync(0xffffffffu, x, o);
+    x = (w < x) ? w : x;
   }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    double t = scal[1];
-    if (t_end > 0 && t + x > t_end) x = t_end - t;
-    if (x < 0) x = 0;
-    scal[0] = x;
-    scal[1] = t + x;  // the step is always taken with this length
-    // the same step as a float pair for the FP32 path (scal[2] as 2 floats)
-    float* ff = reinterpret_cast<float*>(scal + 2);
-    ff[0] = (float)x;
-    ff[1] = (float)(x - (double)ff[0]);
+    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) x = (red[i] < x) ? red[i] : x;
+    mst::set_step(x, f);
   }
 }
 
-// norms of a step from per-tile partials (fixed order: deterministic).
+// a fixed step, clipped so that the time reaches t_end
+__global__ void k_fixed_dt(double dt, const mst::FinishDt f) { mst::set_step(dt, f); }
+
+// norms of a step from per-tile partials (fixed order: deterministic): block
+// b reduces a slice of the tiles into part2[b], the last block to finish the
+// slices.  (One block for all: 150 us on 15,625 tiles -- 140,000 FP64
+// additions on one SM -- now 9.)
 // out: linf[4], l2[4] (sqrt(mean)), mass, dt, time
-__global__ void k_finalize_norms(const double* __restrict__ part, int n_tiles,
-                                 int n_cells, int advance,
-                                 double* __restrict__ scal,
-                                 double* __restrict__ out) {
-  __shared__ double red[kNormSlots][32];
-  const int j = threadIdx.y;  // one row of threads per norm slot
+constexpr int kNormBlocks = 64;    // most blocks
+constexpr int kNormTiles = 128;    // tiles per block before there are more blocks
+__device__ __forceinline__ double norm_op(int j, double x, double v) {
+  return (j < 4) ? ((x < v) ? v : x) : x + v;
+}
+__device__ double norm_slice(const double* part, int i0, int i1, double (*red)[2]) {
+  const int j = threadIdx.y;  // one row of 64 threads per norm slot
   double x = 0.0;
-  for (int i = threadIdx.x; i < n_tiles; i += blockDim.x) {
-    double v = part[(size_t)i * kNormSlots + j];
-    x = (j < 4) ? ((x < v) ? v : x) : x + v;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    double w = __shfl_xor_sync(0xffffffffu, x, o);
-    x = (j < 4) ? ((x < w) ? w : x) : x + w;
-  }
+  for (int i = i0 + (int)threadIdx.x; i < i1; i += blockDim.x)
+    x = norm_op(j, x, __ldcg(part + (size_t)i * kNormSlots + j));
+  for (int o = 16; o > 0; o >>= 1) x = norm_op(j, x, __shfl_xor_sync(0xffffffffu, x, o));
   if ((threadIdx.x & 31) == 0) red[j][threadIdx.x >> 5] = x;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double acc = red[j][0];
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i)
-      acc = (j < 4) ? ((acc < red[j][i]) ? red[j][i] : acc) : acc + red[j][i];
-    if (j >= 4 && j < 8) acc = sqrt(acc / (double)n_cells);
-    out[j] = acc;
-  }
+  x = norm_op(j, red[j][0], red[j][1]);
   __syncthreads();
+  return x;
+}
+__global__ void __launch_bounds__(64 * kNormSlots)
+    k_finalize_norms(const double* __restrict__ part, int n_tiles, int n_cells,
+                     const double* __restrict__ scal, double* part2, unsigned* ticket,
+                     double* __restrict__ out) {
+  __shared__ double red[kNormSlots][2];
+  __shared__ bool last;
+  const int j = threadIdx.y, nb = (int)gridDim.x;
+  const int per = (n_tiles + nb - 1) / nb;
+  const int i0 = (int)blockIdx.x * per;
+  double x = norm_slice(part, i0, min(n_tiles, i0 + per), red);
+  if (nb > 1) {
+    if (threadIdx.x == 0) part2[blockIdx.x * kNormSlots + j] = x;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && j == 0) {
+      last = atomicInc(ticket, nb - 1) == (unsigned)(nb - 1);
+      __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    x = norm_slice(part2, 0, nb, red);
+  }
+  if (threadIdx.x == 0) out[j] = (j >= 4 && j < 8) ? sqrt(x / (double)n_cells) : x;
   if (threadIdx.x == 0 && j == 0) {
-    (void)advance;
     out[kNormSlots] = scal[0];
     out[kNormSlots + 1] = scal[1];
   }
 }
 
 }  // namespace
+
+cudaError_t mst::launch_finalize_dt(const double* part, int n, const FinishDt& f, cudaStream_t s) {
+  k_finalize_dt<<<1, 1024, 0, s>>>(part, n, f);
+  return cudaGetLastError();
+}
 
 namespace {
 
@@ -244,7 +252,8 @@ void drain_profile(mst_ctx* c) {
 // gradient of q (qf: its FP32 copy on the FP32 path); with dt_part it also
 // writes the CFL step partials (and dt_cell)
 mst_status launch_grad(mst_ctx* c, const double4_32a* q, const float4* qf = nullptr,
-                       double* dt_part = nullptr, bool local_dt = false) {
+                       double* dt_part = nullptr, bool local_dt = false,
+                       const mst::FinishDt& fin = mst::FinishDt{}) {
   ProfScope ps(c, c->p.precision == MST_PREC_FP32 ? "k_gradient<f32>" : "k_gradient<f64>");
   const bool f32 = c->p.precision == MST_PREC_FP32;
   if (!f32) qf = nullptr;
@@ -253,10 +262,10 @@ mst_status launch_grad(mst_ctx* c, const double4_32a* q, const float4* qf = null
   cudaError_t e = (c->p.precision == MST_PREC_FP64_EXACT)
                       ? mst::exact::launch_gradient_dt(prec_of(c->p), c->dm, q, qf, c->grad,
                                                        c->p.reference_quirks, c->p.cfl,
-                                                       dt_cell, dt_cell_ff, dt_part, c->stream)
+                                                       dt_cell, dt_cell_ff, dt_part, fin, c->stream)
                       : mst::fast::launch_gradient_dt(prec_of(c->p), c->dm, q, qf, c->grad,
                                                       c->p.reference_quirks, c->p.cfl,
-                                                      dt_cell, dt_cell_ff, dt_part, c->stream);
+                                                      dt_cell, dt_cell_ff, dt_part, fin, c->stream);
   c->last_launches++;
   if (e != cudaSuccess) return fail(MST_ECUDA, std::string("gradient: ") + cudaGetErrorString(e));
   c->grad_valid = true;
@@ -392,39 +401,52 @@ mst_status run_stage(mst_ctx* c, const StageBufs& b, int stage, bool fixed_dt, b
 mst_status compute_dt(mst_ctx* c, const double4_32a* q, double t_end,
                       const float4* qf = nullptr, bool* grad_ready = nullptr) {
   const int nC = c->dm.n_cells;
-  int mode = 0;
-  if (c->p.dt_mode != MST_DT_FIXED && c->p.order == 2 && grad_ready) {
-    mst_status st = launch_grad(c, q, qf, c->dt_part, c->p.dt_mode == MST_DT_CFL_LOCAL);
+  const mst::FinishDt fin{c->dt_ticket, c->scal, reinterpret_cast<float*>(c->scal + 2), t_end};
+  if (c->p.dt_mode == MST_DT_FIXED) {
+    ProfScope ps(c, "k_fixed_dt");
+    k_fixed_dt<<<1, 1, 0, c->stream>>>(c->p.dt, fin);
+    c->last_launches++;
+    CU(cudaGetLastError());
+    return MST_OK;
+  }
+  // the minima's blocks (gradient FP64: kGrad64Cells cells, else 256): few
+  // enough, the launch sets the step itself
+  const bool grad = c->p.order == 2 && grad_ready;
+  const int bs = grad && !pairs(c) ? mst::kGrad64Cells : 256, nb = (nC + bs - 1) / bs;
+  mst::FinishDt own = fin;
+  if (nb > mst::kFinishBlocks) own.ticket = nullptr;
+  if (grad) {
+    mst_status st =
+        launch_grad(c, q, qf, c->dt_part, c->p.dt_mode == MST_DT_CFL_LOCAL, own);
     if (st) return st;
     *grad_ready = true;
-    mode = 1;
-  } else if (c->p.dt_mode != MST_DT_FIXED) {
+  } else {
     ProfScope ps(c, "k_spectral_dt");
     cudaError_t e = (c->p.precision == MST_PREC_FP64_EXACT)
                         ? mst::exact::launch_spectral_dt(prec_of(c->p), c->dm, q, c->p.cfl,
-                                                         c->dt_cell, c->dt_part, c->stream)
+                                                         c->dt_cell, c->dt_part, own, c->stream)
                         : mst::fast::launch_spectral_dt(prec_of(c->p), c->dm, q, c->p.cfl,
-                                                        c->dt_cell, c->dt_part, c->stream);
+                                                        c->dt_cell, c->dt_part, own, c->stream);
     c->last_launches++;
     if (e != cudaSuccess) return fail(MST_ECUDA, std::string("spectral_dt: ") + cudaGetErrorString(e));
-    if (pairs(c) && c->p.dt_mode == MST_DT_CFL_LOCAL) {
-      k_to_pairs1<<<(nC + 255) / 256, 256, 0, c->stream>>>(c->dt_cell, c->dt_cell_ff, nC);
-      CU(cudaGetLastError());
-    }
-    mode = 1;
   }
-  ProfScope ps(c, "k_finalize_dt");
-  k_finalize_dt<<<1, 1024, 0, c->stream>>>(c->dt_part, (nC + 255) / 256, mode, c->p.dt,
-                                            t_end, c->scal);
-  c->last_launches++;
-  CU(cudaGetLastError());
+  if (!grad && pairs(c) && c->p.dt_mode == MST_DT_CFL_LOCAL) {
+    k_to_pairs1<<<(nC + 255) / 256, 256, 0, c->stream>>>(c->dt_cell, c->dt_cell_ff, nC);
+    CU(cudaGetLastError());
+  }
+  if (!own.ticket) {
+    ProfScope ps(c, "k_finalize_dt");
+    CU(mst::launch_finalize_dt(c->dt_part, nb, fin, c->stream));
+    c->last_launches++;
+  }
   return MST_OK;
 }
 
-mst_status finalize_norms(mst_ctx* c, bool advance) {
+mst_status finalize_norms(mst_ctx* c) {
   ProfScope ps(c, "k_finalize_norms");
-  k_finalize_norms<<<1, dim3(64, kNormSlots), 0, c->stream>>>(
-      c->partials, c->dm.n_tiles, c->dm.n_cells, advance ? 1 : 0, c->scal, c->norms);
+  const int nb = std::min(kNormBlocks, (c->dm.n_tiles + kNormTiles - 1) / kNormTiles);
+  k_finalize_norms<<<std::max(nb, 1), dim3(64, kNormSlots), 0, c->stream>>>(
+      c->partials, c->dm.n_tiles, c->dm.n_cells, c->scal, c->norm_part, c->dt_ticket + 1, c->norms);
   c->last_launches++;
   CU(cudaGetLastError());
   return MST_OK;
@@ -683,6 +705,123 @@ mst_status mst_mesh_get_arrays(const mst_mesh* m, mst_mesh_arrays* a) {
   return MST_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// a device array of the context, its address into *dst
+template <class T>
+cudaError_t ctx_upload(mst_ctx* c, const T** dst, const T* src, size_t n) {
+  void* v = nullptr;
+  cudaError_t e = cudaMalloc(&v, std::max<size_t>(n, 1) * sizeof(T));
+  if (e != cudaSuccess) return e;
+  c->allocs.push_back(v);
+  *dst = static_cast<const T*>(v);
+  return n ? cudaMemcpy(v, src, n * sizeof(T), cudaMemcpyHostToDevice) : cudaSuccess;
+}
+
+// outward area vectors of the cell-faces (the signed f_dir of cf_face)
+std::vector<double2> cell_face_dirs(const mst::DevLayout& L) {
+  std::vector<double2> cd(L.cf_face.size());
+  for (size_t k = 0; k < cd.size(); ++k) {
+    const int fs = L.cf_face[k];
+    const double* v = &L.f_dir[2 * (size_t)(fs < 0 ? ~fs : fs)];
+    cd[k] = fs < 0 ? make_double2(-v[0], -v[1]) : make_double2(v[0], v[1]);
+  }
+  return cd;
+}
+
+}  // namespace
+
+// The geometry that the FP64 (exact and production) or the FP32 kernels
+// read, uploaded once a context runs one of them
+mst_status mst_internal_geometry(mst_ctx* c, bool f32) {
+  if (f32 ? c->geo32 : c->geo64) return MST_OK;
+  const mst::DevLayout& L = c->mesh->lay;
+  mst::DevMesh& dm = c->dm;
+  auto up = [&](auto** dst, const auto& v) { return ctx_upload(c, dst, v.data(), v.size()); };
+  auto up2 = [&](const double2** dst, const std::vector<double>& v) {
+    return ctx_upload(c, dst, reinterpret_cast<const double2*>(v.data()), v.size() / 2);
+  };
+  const std::vector<double2> cd = cell_face_dirs(L);
+  const size_t nF = L.n_faces, n = L.n_cells;
+  std::vector<double> eta(nF);
+  for (size_t i = 0; i < nF; ++i) eta[i] = c->mesh->host.face_eta0[L.face_iperm[i]];
+  if (!f32) {
+    std::vector<double> len(cd.size());
+    for (size_t k = 0; k < len.size(); ++k)
+      len[k] = std::sqrt(cd[k].x * cd[k].x + cd[k].y * cd[k].y);
+    CU(up2(&dm.f_dir, L.f_dir));
+    CU(up2(&dm.f_r0, L.f_r0));
+    CU(up2(&dm.f_r1, L.f_r1));
+    CU(up2(&dm.cf_w, L.cf_w));
+    CU(up(&dm.cf_dir, cd));
+    CU(up(&dm.cf_len, len));
+    CU(up(&dm.f_eta, eta));
+    CU(up(&dm.cf_face, L.cf_face));
+    CU(up(&dm.cf_nb, L.cf_nb));
+    CU(up(&dm.cf_nb_fix, L.cf_nb_fix));
+    c->geo64 = true;
+    return MST_OK;
+  }
+  std::vector<float2> r0(nF), r1(nF), cd32(cd.size()), ivff(n);
+  std::vector<float4> dd(nF);
+  std::vector<float> eta32(nF);
+  for (size_t f = 0; f < nF; ++f) {
+    const double *a = &L.f_r0[2 * f], *b = &L.f_r1[2 * f];
+    r0[f] = make_float2((float)a[0], (float)a[1]);
+    r1[f] = make_float2((float)b[0], (float)b[1]);
+    dd[f] = make_float4((float)L.f_dir[2 * f], (float)L.f_dir[2 * f + 1], (float)(a[0] - b[0]),
+                        (float)(a[1] - b[1]));
+    eta32[f] = (float)eta[f];
+  }
+  for (size_t k = 0; k < cd.size(); ++k) cd32[k] = make_float2((float)cd[k].x, (float)cd[k].y);
+  for (size_t i = 0; i < n; ++i) {
+    const double iv = 1.0 / L.c_vol[i];
+    const float h = (float)iv;
+    ivff[i] = make_float2(h, (float)(iv - (double)h));
+  }
+  // the tables by face position
+  int deg = 0;
+  for (size_t i = 0; i < n; ++i) deg = std::max(deg, L.c_ptr[i + 1] - L.c_ptr[i]);
+  std::vector<int> nb(deg * n), slot(deg * n, -1);
+  std::vector<float4> wd(deg * n, make_float4(0.f, 0.f, 0.f, 0.f));
+  int4 quirk = make_int4(-1, -1, -1, -1);
+  for (size_t i = 0; i < n; ++i) {
+    const int kb = L.c_ptr[i], cnt = L.c_ptr[i + 1] - kb;
+    for (int j = 0; j < deg; ++j) {
+      const size_t at = j * n + i, k = (size_t)kb + j;
+      nb[at] = (int)i;
+      if (j >= cnt) continue;
+      const int mode = L.cf_nb_fix[k] >> mst::kFvShift, modeq = L.cf_nb[k] >> mst::kFvShift;
+      if (mode != mst::kFvSelf) nb[at] = L.cf_nb_fix[k] & ((1 << mst::kFvShift) - 1);
+      slot[at] = L.cf_slot[k];
+      // a face without interpolation takes one side's value
+      const float self = mode == mst::kFvSelf ? 1.f : 0.f;
+      const bool in = mode == mst::kFvInterp;
+      wd[at] = make_float4(in ? (float)L.cf_w[2 * k] : self,
+                           in ? (float)L.cf_w[2 * k + 1] : 1.f - self, cd32[k].x, cd32[k].y);
+      if (modeq != mode && modeq == mst::kFvSelf) quirk.x = (int)i, quirk.y = j;
+      if (modeq != mode && modeq == mst::kFvNb) quirk.z = (int)i, quirk.w = j;
+    }
+  }
+  dm.quirk_at = quirk;
+  dm.e_deg = deg;
+  CU(up(&dm.f_r0_32, r0));
+  CU(up(&dm.f_r1_32, r1));
+  CU(up(&dm.f_dd32, dd));
+  CU(up(&dm.cf_dir32, cd32));
+  CU(up(&dm.f_eta32, eta32));
+  CU(up(&dm.c_ivol_ff, ivff));
+  CU(up(&dm.e_nb, nb));
+  CU(up(&dm.e_slot, slot));
+  CU(up(&dm.e_wd, wd));
+  c->geo32 = true;
+  return MST_OK;
+}
+
+extern "C" {
+
 mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out) {
   if (!m || !out) return fail(MST_EINVAL, "NULL argument");
   *out = nullptr;
@@ -702,153 +841,31 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
   CU(cudaEventCreate(&c->ev1));
   const auto& L = m->lay;
   DevArrays& d = c->d;
-  auto up = [&](auto** dst, const auto& v) -> cudaError_t {
-    cudaError_t r = upload(dst, v);
-    c->allocs.push_back((void*)*dst);
-    return r;
-  };
-  {
-    std::vector<int2> c0c1(L.n_faces);
-    for (int i = 0; i < L.n_faces; ++i) c0c1[i] = make_int2(L.f_c0c1[2 * i], L.f_c0c1[2 * i + 1]);
-    auto as_d2 = [](const std::vector<double>& v) {
-      std::vector<double2> o(v.size() / 2);
-      for (size_t i = 0; i < o.size(); ++i) o[i] = make_double2(v[2 * i], v[2 * i + 1]);
-      return o;
-    };
-    auto as_f2 = [](const std::vector<double>& v) {
-      std::vector<float2> o(v.size() / 2);
-      for (size_t i = 0; i < o.size(); ++i) o[i] = make_float2((float)v[2 * i], (float)v[2 * i + 1]);
-      return o;
-    };
-    CU(up(&d.f_c0c1, c0c1));
-    CU(up(&d.f_info, L.f_info));
-    CU(up(&d.f_dir, as_d2(L.f_dir)));
-    CU(up(&d.f_r0, as_d2(L.f_r0)));
-    CU(up(&d.f_r1, as_d2(L.f_r1)));
-    CU(up(&d.cf_w, as_d2(L.cf_w)));
-    CU(up(&d.f_r0_32, as_f2(L.f_r0)));
-    CU(up(&d.f_r1_32, as_f2(L.f_r1)));
-    {
-      std::vector<float4> dd(L.n_faces);
-      for (size_t f = 0; f < dd.size(); ++f)
-        dd[f] = make_float4((float)L.f_dir[2 * f], (float)L.f_dir[2 * f + 1],
-                            (float)(L.f_r0[2 * f] - L.f_r1[2 * f]),
-                            (float)(L.f_r0[2 * f + 1] - L.f_r1[2 * f + 1]));
-      CU(up(&d.f_dd32, dd));
-    }
-    {
-      std::vector<double> cd(2 * L.cf_face.size());
-      for (size_t k = 0; k < L.cf_face.size(); ++k) {
-        const int fs = L.cf_face[k];
-        const int f = fs < 0 ? ~fs : fs;
-        cd[2 * k] = fs < 0 ? -L.f_dir[2 * (size_t)f] : L.f_dir[2 * (size_t)f];
-        cd[2 * k + 1] = fs < 0 ? -L.f_dir[2 * (size_t)f + 1] : L.f_dir[2 * (size_t)f + 1];
-      }
-      CU(up(&d.cf_dir, as_d2(cd)));
-      CU(up(&d.cf_dir32, as_f2(cd)));
-      std::vector<double> len(cd.size() / 2);
-      for (size_t k = 0; k < len.size(); ++k)
-        len[k] = std::sqrt(cd[2 * k] * cd[2 * k] + cd[2 * k + 1] * cd[2 * k + 1]);
-      CU(up(&d.cf_len, len));
-      // the FP32 tables by face position
-      int deg = 0;
-      for (int i = 0; i < L.n_cells; ++i) deg = std::max(deg, L.c_ptr[i + 1] - L.c_ptr[i]);
-      const size_t n = L.n_cells;
-      std::vector<int> nb(deg * n), slot(deg * n, -1);
-      std::vector<float4> wd(deg * n, make_float4(0.f, 0.f, 0.f, 0.f));
-      for (size_t at = 0; at < nb.size(); ++at) nb[at] = (int)(at % n);
-      int4 quirk = make_int4(-1, -1, -1, -1);
-      for (size_t i = 0; i < n; ++i)
-        for (int k = L.c_ptr[i]; k < L.c_ptr[i + 1]; ++k) {
-          const size_t at = (size_t)(k - L.c_ptr[i]) * n + i, k2 = 2 * (size_t)k;
-          const int mode = L.cf_nb_fix[k] >> mst::kFvShift;
-          const int modeq = L.cf_nb[k] >> mst::kFvShift;
-          if (mode != mst::kFvSelf) nb[at] = L.cf_nb_fix[k] & ((1 << mst::kFvShift) - 1);
-          slot[at] = L.cf_slot[k];
-          // a face without interpolation takes one side's value
-          const bool in = mode == mst::kFvInterp;
-          wd[at] = make_float4(in ? (float)L.cf_w[k2] : (mode == mst::kFvSelf ? 1.f : 0.f),
-                               in ? (float)L.cf_w[k2 + 1] : (mode == mst::kFvSelf ? 0.f : 1.f),
-                               (float)cd[k2], (float)cd[k2 + 1]);
-          if (modeq != mode && modeq == mst::kFvSelf)
-            quirk.x = (int)i, quirk.y = k - L.c_ptr[i];
-          if (modeq != mode && modeq == mst::kFvNb)
-            quirk.z = (int)i, quirk.w = k - L.c_ptr[i];
-        }
-      c->dm.quirk_at = quirk;
-      CU(up(&d.e_nb, nb));
-      CU(up(&d.e_slot, slot));
-      CU(up(&d.e_wd, wd));
-      c->dm.e_deg = deg;
-    }
-    {
-      std::vector<double> fe(L.n_faces);
-      std::vector<float> fe32(L.n_faces);
-      for (int i = 0; i < L.n_faces; ++i) {
-        fe[i] = m->host.face_eta0[L.face_iperm[i]];
-        fe32[i] = (float)fe[i];
-      }
-      CU(up(&d.f_eta, fe));
-      CU(up(&d.f_eta32, fe32));
-    }
-    CU(up(&d.c_vol, L.c_vol));
-    for (double v : L.c_vol) c->volumes_ok = c->volumes_ok && std::isfinite(v) && v > 0.0;
-    std::vector<double> ivol(L.c_vol.size());
-    for (size_t i = 0; i < ivol.size(); ++i) ivol[i] = 1.0 / L.c_vol[i];
-    CU(up(&d.c_ivol, ivol));
-    std::vector<float2> ivff(ivol.size());
-    for (size_t i = 0; i < ivol.size(); ++i) {
-      const float h = (float)ivol[i];
-      ivff[i] = make_float2(h, (float)(ivol[i] - (double)h));
-    }
-    CU(up(&d.c_ivol_ff, ivff));
-    CU(up(&d.c_ptr, L.c_ptr));
-    CU(up(&d.cf_face, L.cf_face));
-    CU(up(&d.cf_slot, L.cf_slot));
-    CU(up(&d.cf_nb, L.cf_nb));
-    CU(up(&d.cf_nb_fix, L.cf_nb_fix));
-    CU(up(&d.t_own_ptr, L.t_own_ptr));
-    CU(up(&d.t_bor_ptr, L.t_bor_ptr));
-    CU(up(&d.t_bor, L.t_bor));
-    CU(up(&d.cell_iperm, L.cell_iperm));
-    CU(up(&d.cell_perm, L.cell_perm));
-  }
   mst::DevMesh& dm = c->dm;
+  auto up = [&](auto** dst, const auto& v) { return ctx_upload(c.get(), dst, v.data(), v.size()); };
   dm.n_cells = L.n_cells;
   dm.n_faces = L.n_faces;
   dm.n_tiles = L.n_tiles;
   dm.max_tile_faces = L.max_tile_faces;
-  dm.f_c0c1 = d.f_c0c1;
-  dm.f_info = d.f_info;
-  dm.f_dir = d.f_dir;
-  dm.f_r0 = d.f_r0;
-  dm.f_r1 = d.f_r1;
-  dm.f_dd32 = d.f_dd32;
-  dm.f_r0_32 = d.f_r0_32;
-  dm.f_r1_32 = d.f_r1_32;
-  dm.f_eta = d.f_eta;
-  dm.f_eta32 = d.f_eta32;
-  dm.c_vol = d.c_vol;
-  dm.c_ivol = d.c_ivol;
-  dm.c_ivol_ff = d.c_ivol_ff;
-  dm.c_ptr = d.c_ptr;
-  dm.cf_face = d.cf_face;
-  dm.cf_slot = d.cf_slot;
-  dm.cf_nb = d.cf_nb;
-  dm.cf_nb_fix = d.cf_nb_fix;
-  dm.cf_w = d.cf_w;
-  dm.cf_dir = d.cf_dir;
-  dm.cf_dir32 = d.cf_dir32;
-  dm.cf_len = d.cf_len;
-  dm.t_own_ptr = d.t_own_ptr;
-  dm.t_bor_ptr = d.t_bor_ptr;
-  dm.t_bor = d.t_bor;
-  dm.e_nb = d.e_nb;
-  dm.e_wd = d.e_wd;
-  dm.e_slot = d.e_slot;
+  // int pairs lie as int2
+  CU(ctx_upload(c.get(), &dm.f_c0c1, reinterpret_cast<const int2*>(L.f_c0c1.data()), L.n_faces));
+  CU(up(&dm.f_info, L.f_info));
+  CU(up(&dm.c_vol, L.c_vol));
+  for (double v : L.c_vol) c->volumes_ok = c->volumes_ok && std::isfinite(v) && v > 0.0;
+  std::vector<double> ivol(L.c_vol.size());
+  for (size_t i = 0; i < ivol.size(); ++i) ivol[i] = 1.0 / L.c_vol[i];
+  CU(up(&dm.c_ivol, ivol));
+  CU(up(&dm.c_ptr, L.c_ptr));
+  CU(up(&dm.cf_slot, L.cf_slot));
+  CU(up(&dm.t_own_ptr, L.t_own_ptr));
+  CU(up(&dm.t_bor_ptr, L.t_bor_ptr));
+  CU(up(&dm.t_bor, L.t_bor));
+  CU(up(&d.cell_iperm, L.cell_iperm));
+  CU(up(&d.cell_perm, L.cell_perm));
+  if ((st = mst_internal_geometry(c.get(), p->precision == MST_PREC_FP32))) return st;
   dm.deg3 = 1;
   for (int i = 0; i <= L.n_cells && dm.deg3; ++i) dm.deg3 = L.c_ptr[i] == 3 * i;
-  const size_t nC = L.n_cells, nB = (nC + 255) / 256;
+  const size_t nC = L.n_cells, nB = (nC + mst::kGrad64Cells - 1) / mst::kGrad64Cells;
   const size_t qbytes = nC * sizeof(double4_32a);
   if ((st = dalloc(c.get(), &c->q_old, qbytes)) || (st = dalloc(c.get(), &c->q_new, qbytes)) ||
       (st = dalloc(c.get(), &c->q_stage, qbytes)) || (st = dalloc(c.get(), &c->r, qbytes)) ||
@@ -861,7 +878,9 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
       (st = dalloc(c.get(), &c->ql_stage, nC * sizeof(float4))) ||
       (st = dalloc(c.get(), (char**)&c->grad, nC * 8 * sizeof(double))) ||
       (st = dalloc(c.get(), &c->partials,
-                   std::max<size_t>(L.n_tiles, nB) * kNormSlots * sizeof(double))) ||
+                   (size_t)L.n_tiles * kNormSlots * sizeof(double))) ||
+      (st = dalloc(c.get(), &c->norm_part, kNormBlocks * kNormSlots * sizeof(double))) ||
+      (st = dalloc(c.get(), &c->dt_ticket, 2 * sizeof(unsigned))) ||
       (st = dalloc(c.get(), &c->dt_part, nB * sizeof(double))) ||
       (st = dalloc(c.get(), &c->dt_cell, nC * sizeof(double))) ||
       (st = dalloc(c.get(), &c->dt_cell_ff, nC * sizeof(float2))) ||
@@ -872,6 +891,7 @@ mst_status mst_ctx_create(const mst_mesh* m, const mst_params* p, mst_ctx** out)
   CU(cudaMemset(c->q_old, 0, qbytes));
   CU(cudaMemset(c->q_new, 0, qbytes));
   CU(cudaMemset(c->r, 0, qbytes));
+  CU(cudaMemset(c->dt_ticket, 0, 2 * sizeof(unsigned)));
   CU(cudaMemset(c->scal, 0, 4 * sizeof(double)));
   CU(cudaMemset(c->norms, 0, (kNormSlots + 2) * sizeof(double)));
   CU(cudaDeviceSynchronize());
@@ -901,7 +921,9 @@ mst_status mst_ctx_set_params(mst_ctx* c, const mst_params* p) {
   if (!c) return fail(MST_EINVAL, "NULL context");
   mst_status st = check_params(p);
   if (st) return st;
-  if ((st = ensure_face_buffer(c, p->precision))) return st;
+  if ((st = mst_internal_geometry(c, p->precision == MST_PREC_FP32)) ||
+      (st = ensure_face_buffer(c, p->precision)))
+    return st;
   const bool was = pairs(c);
   const bool to_pairs = p->precision == MST_PREC_FP32 && !was;
   if (was && p->precision != MST_PREC_FP32) {  // the FP64 buffers were not kept
@@ -982,7 +1004,7 @@ mst_status mst_solve(mst_ctx* c) {
   b.qln = c->ql_new;
   mst_status s = run_stage(c, b, 0, true, true, true);
   if (s) return s;
-  if ((s = finalize_norms(c, false))) return s;
+  if ((s = finalize_norms(c))) return s;
   CU(cudaEventRecord(c->ev1, c->stream));
   c->timed = true;
   CU(cudaStreamSynchronize(c->stream));
@@ -1110,7 +1132,7 @@ mst_status enqueue_steps(mst_ctx* c, int nsteps, double t_end, bool last_norms =
       if (!st) st = run_stage(c, b1, 1, false, norms, false);
     }
     if (st) return st;
-    if (norms && (st = finalize_norms(c, true))) return st;
+    if (norms && (st = finalize_norms(c))) return st;
     std::swap(c->q_old, c->q_new);
     std::swap(c->qf_old, c->qf_new);
     std::swap(c->ql_old, c->ql_new);

@@ -27,23 +27,13 @@ struct mst_mesh3d {
 };
 
 struct DevArrays {
-  int2* f_c0c1 = nullptr;
-  int* f_info = nullptr;
-  double2 *f_dir = nullptr, *f_r0 = nullptr, *f_r1 = nullptr, *cf_w = nullptr,
-          *cf_dir = nullptr;
-  float2 *f_r0_32 = nullptr, *f_r1_32 = nullptr, *cf_dir32 = nullptr;
-  float4 *f_dd32 = nullptr, *e_wd = nullptr;
-  double* f_eta = nullptr;
-  float* f_eta32 = nullptr;
-  double* cf_len = nullptr;
-  double* c_vol = nullptr;
-  double* c_ivol = nullptr;
-  float2* c_ivol_ff = nullptr;
-  int *c_ptr = nullptr, *cf_face = nullptr, *cf_slot = nullptr, *cf_nb = nullptr,
-      *cf_nb_fix = nullptr, *t_own_ptr = nullptr, *t_bor_ptr = nullptr,
-      *t_bor = nullptr, *cell_iperm = nullptr, *cell_perm = nullptr,
-      *e_nb = nullptr, *e_slot = nullptr;
+  const int *cell_iperm = nullptr, *cell_perm = nullptr;
 };
+
+struct mst_ctx;
+// Uploads the geometry the FP64 or the FP32 kernels read, if the context
+// does not hold it yet (capi.cu).
+mst_status mst_internal_geometry(mst_ctx* c, bool f32);
 
 struct mst_node_avg;  // result writer buffers (io.cu)
 void mst_io_release(struct mst_ctx* c);
@@ -56,6 +46,7 @@ struct mst_ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   DevArrays d;
   mst::DevMesh dm{};
+  bool geo64 = false, geo32 = false;  // geometry uploaded (mst_internal_geometry)
   double4_32a *q_old = nullptr, *q_new = nullptr, *q_stage = nullptr,
               *r = nullptr, *stage_in = nullptr;
   // FP32 path: state as float pairs, hi parts (qf_*) and lo parts (ql_*)
@@ -67,7 +58,9 @@ struct mst_ctx {
   // per face; allocated once a context runs one of them
   double* fx = nullptr;
   size_t fx_words = 0;
-  double* partials = nullptr;  // [max(nT, nBlocks)][kNormSlots]
+  double* partials = nullptr;  // [nT][kNormSlots]
+  double* norm_part = nullptr; // their sums over slices of the tiles
+  unsigned* dt_ticket = nullptr;  // [0] step minima, [1] norms: blocks arrived
   double* dt_part = nullptr;   // [nBlocks]
   double* dt_cell = nullptr;   // [nC]
   float2* dt_cell_ff = nullptr;  // [nC] local steps as float pairs (FP32 path)

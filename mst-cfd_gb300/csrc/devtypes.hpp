@@ -104,6 +104,73 @@ __device__ __forceinline__ bool range_cases_done(const DevMesh& m, int c0, int c
   return true;
 }
 
+// Most blocks of a launch that sets the step itself (finish_dt).
+constexpr int kFinishBlocks = 1024;
+
+// Cells per block of the FP64 gradient kernels.
+constexpr int kGrad64Cells = 64;
+
+// The step length of a CFL step, set by the last block of the launch that
+// forms the cells' steps (ticket: blocks that have arrived, 0 between
+// launches; nullptr: not by this launch).
+struct FinishDt {
+  unsigned* ticket = nullptr;
+  double* scal = nullptr;  // [0] step, [1] time
+  float* ff = nullptr;     // the step as a float pair
+  double t_end = 0.0;
+};
+
+// the step from the n minima in part, by a launch of its own (capi.cu)
+cudaError_t launch_finalize_dt(const double* part, int n, const FinishDt& f, cudaStream_t s);
+
+// step x, cut to reach t_end (> 0); the time advances by it
+__device__ __forceinline__ void set_step(double x, const FinishDt& f) {
+  const double t = f.scal[1];
+  if (f.t_end > 0.0 && t + x > f.t_end) x = f.t_end - t;
+  if (!(x > 0.0)) x = 0.0;
+  f.scal[0] = x;
+  f.scal[1] = t + x;
+  const float hi = (float)x;
+  f.ff[0] = hi;
+  f.ff[1] = (float)(x - (double)hi);
+}
+
+// The minima that this launch's blocks leave in part, reduced by the last
+// block to arrive (every block calls it after its thread 0 stored its own
+// minimum).  Saves the launch of a one-block reduction (6 us) where the
+// launch is about one wave of blocks; beyond kFinishBlocks the atomics on one
+// address and the blocks that wait for them cost more than that launch
+// (7,813 blocks: gradient 48 -> 76 us, the launch 7).
+__device__ __forceinline__ void finish_dt(const double* part, const FinishDt& f) {
+  if (!f.ticket) return;
+  __shared__ bool last_block;
+  __shared__ double red_dt[32];
+  const unsigned n = gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last_block = atomicInc(f.ticket, n - 1) == n - 1;  // wraps to 0 for the next launch
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last_block) return;
+  double x = 1e300;
+  for (unsigned i = threadIdx.x; i < n; i += blockDim.x) {
+    const double p = __ldcg(part + i);
+    x = (p < x) ? p : x;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_xor_sync(0xffffffffu, x, o);
+    x = (w < x) ? w : x;
+  }
+  if ((threadIdx.x & 31) == 0) red_dt[threadIdx.x >> 5] = x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) x = (red_dt[i] < x) ? red_dt[i] : x;
+    set_step(x, f);
+  }
+}
+
 // Number of doubles of per-tile partial norms: linf[4], l2[4], mass.
 constexpr int kNormSlots = 9;
 
@@ -259,7 +326,8 @@ enum { kFluxAusm = 0, kFluxRoe = 1 };
                                  const double4_32a* q, const float4* qf,      \
                                  void* grad, int quirks, double cfl,          \
                                  double* dt_cell, float2* dt_cell_ff,         \
-                                 double* dt_part, cudaStream_t s);            \
+                                 double* dt_part, const FinishDt& fin,        \
+                                 cudaStream_t s);                             \
   cudaError_t launch_to_f32(const double4_32a* q, float4* qf, int n,         \
                             cudaStream_t s);                                  \
   cudaError_t launch_flux_update(int prec, int flux, int order,              \
@@ -271,7 +339,7 @@ enum { kFluxAusm = 0, kFluxRoe = 1 };
   cudaError_t launch_spectral_dt(int prec, const DevMesh& m,                 \
                                  const double4_32a* q, double cfl,            \
                                  double* dt_cell, double* partials,           \
-                                 cudaStream_t s);                             \
+                                 const FinishDt& fin, cudaStream_t s);        \
   cudaError_t lusgs_forward_t(const DevMesh& m, const LusgsArgs& a,          \
                               int threads, bool turn, cudaStream_t s);        \
   cudaError_t lusgs_backward_t(const DevMesh& m, const LusgsArgs& a,         \

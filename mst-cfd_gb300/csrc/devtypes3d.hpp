@@ -2,7 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include "smem_limit.hpp"
+#include "devtypes.hpp"
 
 namespace mst {
 

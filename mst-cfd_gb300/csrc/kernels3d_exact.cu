@@ -12,17 +12,13 @@ constexpr bool kExactArith = true;
 #include "kernels3d.inc"
 
 cudaError_t gradient(int, const DevMesh3& m, const Step3Args& a, void* grad, double cfl,
-                     double* dt_part, cudaStream_t s) {
-  return gradient3_t<double, 0>(m, a, grad, cfl, dt_part, s);
+                     double* dt_part, const FinishDt& fin, cudaStream_t s) {
+  return gradient3_t<double, 0>(m, a, grad, cfl, dt_part, fin, s);
 }
 cudaError_t flux_update(int, int order, bool visc, int mode, const DevMesh3& m,
                         const Step3Args& a, cudaStream_t s) {
   if (mode == 3) return flux3_dispatch<false, 3>(order, visc, m, a, s);
   return flux3_dispatch<false, 0>(order, visc, m, a, s);
-}
-cudaError_t finalize_dt(const double* part, int n, double t_end, double* scal, float* dt_ff,
-                        cudaStream_t s) {
-  return finalize_dt3(part, n, t_end, scal, dt_ff, s);
 }
 cudaError_t kinetic(int, const DevMesh3& m, const Step3Args& a, double* part, double* out,
                     cudaStream_t s) {

@@ -12,9 +12,9 @@ constexpr bool kExactArith = false;
 #include "kernels3d.inc"
 
 cudaError_t gradient(int prec, const DevMesh3& m, const Step3Args& a, void* grad, double cfl,
-                     double* dt_part, cudaStream_t s) {
-  if (prec == 2) return gradient3_t<float, 1>(m, a, grad, cfl, dt_part, s);
-  return gradient3_t<double, 0>(m, a, grad, cfl, dt_part, s);
+                     double* dt_part, const FinishDt& fin, cudaStream_t s) {
+  if (prec == 2) return gradient3_t<float, 1>(m, a, grad, cfl, dt_part, fin, s);
+  return gradient3_t<double, 0>(m, a, grad, cfl, dt_part, fin, s);
 }
 cudaError_t flux_update(int prec, int order, bool visc, int mode, const DevMesh3& m,
                         const Step3Args& a, cudaStream_t s) {
@@ -24,10 +24,6 @@ cudaError_t flux_update(int prec, int order, bool visc, int mode, const DevMesh3
   }
   if (mode == 3) return flux3_dispatch<false, 3>(order, visc, m, a, s);
   return flux3_dispatch<false, 0>(order, visc, m, a, s);
-}
-cudaError_t finalize_dt(const double* part, int n, double t_end, double* scal, float* dt_ff,
-                        cudaStream_t s) {
-  return finalize_dt3(part, n, t_end, scal, dt_ff, s);
 }
 cudaError_t kinetic(int prec, const DevMesh3& m, const Step3Args& a, double* part, double* out,
                     cudaStream_t s) {

@@ -16,16 +16,16 @@ constexpr bool kExactArith = false;
 cudaError_t launch_gradient(int prec, const DevMesh& m, const double4_32a* q,
                             void* grad, int quirks, cudaStream_t s) {
   if (prec == kPrecF32)
-    return gradient_t<float>(m, q, nullptr, grad, quirks, 0.0, nullptr, nullptr, nullptr, s);
-  return gradient_t<double>(m, q, nullptr, grad, quirks, 0.0, nullptr, nullptr, nullptr, s);
+    return gradient_t<float>(m, q, nullptr, grad, quirks, 0.0, nullptr, nullptr, nullptr, FinishDt{}, s);
+  return gradient_t<double>(m, q, nullptr, grad, quirks, 0.0, nullptr, nullptr, nullptr, FinishDt{}, s);
 }
 cudaError_t launch_gradient_dt(int prec, const DevMesh& m, const double4_32a* q,
                                const float4* qf, void* grad, int quirks, double cfl,
                                double* dt_cell, float2* dt_cell_ff, double* dt_part,
-                               cudaStream_t s) {
+                               const FinishDt& fin, cudaStream_t s) {
   if (prec == kPrecF32)
-    return gradient_t<float>(m, q, qf, grad, quirks, cfl, dt_cell, dt_cell_ff, dt_part, s);
-  return gradient_t<double>(m, q, nullptr, grad, quirks, cfl, dt_cell, nullptr, dt_part, s);
+    return gradient_t<float>(m, q, qf, grad, quirks, cfl, dt_cell, dt_cell_ff, dt_part, fin, s);
+  return gradient_t<double>(m, q, nullptr, grad, quirks, cfl, dt_cell, nullptr, dt_part, fin, s);
 }
 cudaError_t launch_to_f32(const double4_32a* q, float4* qf, int n, cudaStream_t s) {
   k_to_f32<<<(n + 255) / 256, 256, 0, s>>>(q, qf, n);
@@ -43,12 +43,12 @@ cudaError_t launch_face_flux(int prec, int flux, int order, const DevMesh& m,
 }
 cudaError_t launch_spectral_dt(int prec, const DevMesh& m, const double4_32a* q,
                                double cfl, double* dt_cell, double* partials,
-                               cudaStream_t s) {
+                               const FinishDt& fin, cudaStream_t s) {
   const int nb = (m.n_cells + 255) / 256;
   if (prec == kPrecF32)
-    k_spectral_dt<float><<<nb, 256, 0, s>>>(m, q, cfl, dt_cell, partials);
+    k_spectral_dt<float><<<nb, 256, 0, s>>>(m, q, cfl, dt_cell, partials, fin);
   else
-    k_spectral_dt<double><<<nb, 256, 0, s>>>(m, q, cfl, dt_cell, partials);
+    k_spectral_dt<double><<<nb, 256, 0, s>>>(m, q, cfl, dt_cell, partials, fin);
   return cudaGetLastError();
 }
 }  // namespace fast

@@ -51,6 +51,7 @@ struct mst_ctx3d {
   double* dt_part = nullptr;
   double* scal = nullptr;  // [0] dt, [1] time
   float* dt_ff = nullptr;
+  unsigned* dt_ticket = nullptr;
   double* ke_part = nullptr;
   double* ke_out = nullptr;
   int cur = 0;
@@ -192,13 +193,14 @@ mst::Step3Args args3(mst_ctx3d* c, int in, int out, int prev, int stage) {
   return a;
 }
 
-cudaError_t grad3(mst_ctx3d* c, const mst::Step3Args& a, double* dt_part) {
+cudaError_t grad3(mst_ctx3d* c, const mst::Step3Args& a, double* dt_part,
+                  const mst::FinishDt& fin = mst::FinishDt{}) {
   Prof3 pr(c, "k3_gradient");
   ++c->last_launches;
   return exact3(c) ? mst::exact3::gradient(c->p.precision, c->dm, a, c->grad, c->p.cfl, dt_part,
-                                           c->stream)
+                                           fin, c->stream)
                    : mst::fast3::gradient(c->p.precision, c->dm, a, c->grad, c->p.cfl, dt_part,
-                                          c->stream);
+                                          fin, c->stream);
 }
 
 cudaError_t flux3(mst_ctx3d* c, const mst::Step3Args& a, int mode) {
@@ -417,12 +419,14 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
       (!pairs && (st = alloc3(c.get(), &c->fx, (exact3(c.get()) ? 16 : 6) * (size_t)nF))) ||
       (pairs && ((st = alloc3(c.get(), &c->fx4, nF)) || (st = alloc3(c.get(), &c->fx1, nF)))) ||
       (st = alloc3(c.get(), &c->dt_part, nb)) || (st = alloc3(c.get(), &c->scal, 2)) ||
+      (st = alloc3(c.get(), &c->dt_ticket, 1)) ||
       (st = alloc3(c.get(), &c->dt_ff, 2)) || (st = alloc3(c.get(), &c->ke_part, 2 * (size_t)nb)) ||
       (st = alloc3(c.get(), &c->ke_out, 2))) {
     cleanup();
     return st;
   }
-  if (cudaMemset(c->scal, 0, 2 * sizeof(double)) != cudaSuccess) {
+  if (cudaMemset(c->scal, 0, 2 * sizeof(double)) != cudaSuccess ||
+      cudaMemset(c->dt_ticket, 0, sizeof(unsigned)) != cudaSuccess) {
     cleanup();
     return fail3(MST_ECUDA, "memset failed");
   }
@@ -508,17 +512,20 @@ mst_status mst_ctx3d_gradient(mst_ctx3d* c, double* g) {
 mst_status mst_ctx3d_step(mst_ctx3d* c, int nsteps, double t_end, double* time) {
   if (!c || nsteps < 0) return fail3(MST_EINVAL, "bad arguments");
   c->last_launches = 0;
-  const int bs = f32(c) ? 256 : 64;  // cells per block of the gradient kernel
+  const mst::FinishDt fin{c->dt_ticket, c->scal, c->dt_ff, t_end};
+  const int bs = f32(c) ? 256 : mst::kGrad64Cells;  // cells per block of the gradient kernel
   const int nb = (c->dm.n_cells + bs - 1) / bs;
+  mst::FinishDt own = fin;  // few enough blocks: the gradient launch sets the step
+  if (nb > mst::kFinishBlocks) own.ticket = nullptr;
   C3(cudaEventRecord(c->ev0, c->stream));
   for (int s = 0; s < nsteps; ++s) {
     const int in = c->cur, stg = (c->cur + 1) % 3, nxt = (c->cur + 2) % 3;
     mst::Step3Args a0 = args3(c, in, stg, -1, 0);
-    C3(grad3(c, a0, c->dt_part));
-    {
+    C3(grad3(c, a0, c->dt_part, own));
+    if (!own.ticket) {
       Prof3 pr(c, "k3_finalize_dt");
       ++c->last_launches;
-      C3(mst::fast3::finalize_dt(c->dt_part, nb, t_end, c->scal, c->dt_ff, c->stream));
+      C3(mst::launch_finalize_dt(c->dt_part, nb, fin, c->stream));
     }
     C3(flux3(c, a0, f32(c) ? 1 : 0));
     mst::Step3Args a1 = args3(c, stg, nxt, in, 1);
