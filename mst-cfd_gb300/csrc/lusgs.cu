@@ -11,10 +11,12 @@
 // in the same order when a row's entries are sorted by (column ascending,
 // insertion order) -- or (column descending, insertion order) for the
 // backward sweep.  Rows whose dependencies are all in earlier levels are
-// independent, so each level is one parallel launch and every row adds its
-// terms sequentially in that order: the results are bit-identical to the
+// independent, so each level is one parallel launch -- or, for scalar
+// systems, a phase of one launch -- and every row adds
+// its terms sequentially in that order: the results are bit-identical to the
 // reference's (compiled with --fmad=false; 4x4 blocks use the adjugate
 // inverse and left-to-right products of the oracle's Eigen shim).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -24,6 +26,9 @@
 #include <vector>
 
 #include "ctx.hpp"
+#include "smem_limit.hpp"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -206,6 +211,200 @@ __global__ void k_invert_blocks(int dim, const double* __restrict__ D, double* _
   if (r < dim) inv4(D + 16 * (size_t)r, Di + 16 * (size_t)r);
 }
 
+// ---- scalar systems: the whole solve in one launch ----------------------------
+// The levels of a sweep are small (800 rows of an 18k-row mesh system) and
+// depend on each other, so a launch per level pays launch and memory latency
+// 230 times a solve.  Here one thread-block cluster runs all iterations and the
+// exit test.  The swept vector lies in the CTAs' shared memory, 512 rows in turn
+// to each CTA; a row's dependent values are read from the owner (distributed
+// shared memory: two thirds of the latency of the same vector in L2), and a
+// level ends with the hardware cluster barrier.  A row's columns and weights
+// are fetched a level ahead, 32 rows a warp.  The FP64 pipe takes 64 cycles a
+// warp instruction on each SM sub-partition, so the cluster is the largest the
+// device places.  ILUSGS, 5 iterations, call included: 200 / 18,240 / 228,488
+// rows 195 / 449 / 1,919 us (a launch per level 869 / 1,580 / 2,228; clusters of
+// 1 / 4 / 8 at 18,240 rows 1,549 / 722 / 534).
+constexpr int kLuThreads = 512;
+constexpr int kLuMaxCta = 16;
+
+// Rows of a sweep in level order, or of a product in row order.  The first four
+// entries stand at fixed places, so that all of a row's loads can be issued at
+// once; rows with more find the rest at meta.z.  A sweep's weight is
+// L (1 / D[column]).
+struct LuRows {
+  const int* lev;
+  const int4* meta;  // row, entries, first of the entries past the fourth, -
+  const int4* col4;
+  const double4_32a* w4;
+  const int* col;
+  const double* w;
+  int n_levels;
+};
+struct LuSolve {
+  int dim, gs, shift, rows;  // 2^shift CTAs, rows of the vector in each
+  LuRows up, lo, fwd, bwd;
+  const double *D, *rD, *b;  // rD = 1 / D
+  double* x;
+  unsigned* part;  // [kLuMaxCta]
+  int* its;
+};
+
+// a vector over the cluster's shared memory
+struct LuVec {
+  double* base;
+  int shift;
+  __device__ __forceinline__ double* at(int r) const {
+    const int chunk = r / kLuThreads;
+    return cg::this_cluster().map_shared_rank(base, chunk & ((1 << shift) - 1)) +
+           ((chunk >> shift) * kLuThreads + r % kLuThreads);
+  }
+  __device__ __forceinline__ double operator[](int r) const { return *(volatile double*)at(r); }
+};
+
+struct LuRow {
+  int4 meta, c;
+  double4_32a w;
+};
+__device__ __forceinline__ void lu_fetch(LuRow& r, const LuRows& s, int i, int end) {
+  r.meta.x = -1;
+  if (i >= end) return;
+  r.meta = s.meta[i];
+  r.c = s.col4[i];
+  r.w = s.w4[i];
+}
+// acc - sum w v (or + : the products), entries in order
+template <bool SUB, class V>
+__device__ __forceinline__ double lu_row(const LuRow& r, const LuRows& s, const V& v, double acc) {
+  const int n = r.meta.y;
+  const double v0 = n > 0 ? v[r.c.x] : 0., v1 = n > 1 ? v[r.c.y] : 0., v2 = n > 2 ? v[r.c.z] : 0.,
+               v3 = n > 3 ? v[r.c.w] : 0.;
+  auto add = [&](double p) { acc = SUB ? acc - p : acc + p; };
+  if (n > 0) add(r.w.x * v0);
+  if (n > 1) add(r.w.y * v1);
+  if (n > 2) add(r.w.z * v2);
+  if (n > 3) add(r.w.w * v3);
+  for (int k = 0; k < n - 4; ++k) add(s.w[r.meta.z + k] * v[s.col[r.meta.z + k]]);
+  return acc;
+}
+
+struct LuGlobal {  // written by other CTAs of the cluster: read from L2
+  const double* p;
+  __device__ __forceinline__ double operator[](int r) const { return __ldcg(p + r); }
+};
+
+__device__ void lu_sweep(const LuRows& s, const LuVec& v, int first, int stride) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int n = s.n_levels;
+  if (n < 2) return;
+  // rows [b, e) of this level, [e, e1) of the next, [e1, e2) after it; the
+  // rows of level 0 have no entries
+  int b = s.lev[1], e = s.lev[2], e1 = s.lev[min(3, n)], e2 = s.lev[min(4, n)];
+  LuRow cur, nxt;
+  lu_fetch(cur, s, b + first, e);
+  for (int l = 1; l < n; ++l) {
+    lu_fetch(nxt, s, e + first, e1);
+    const int e3 = s.lev[min(l + 4, n)];
+    for (int i = b + first;;) {
+      if (cur.meta.x >= 0) {
+        double* p = v.at(cur.meta.x);
+        *p = lu_row<true>(cur, s, v, *(volatile double*)p);
+      }
+      i += stride;
+      if (i >= e) break;
+      lu_fetch(cur, s, i, e);
+    }
+    cl.sync();
+    cur = nxt;
+    b = e;
+    e = e1;
+    e1 = e2;
+    e2 = e3;
+  }
+}
+
+// A row's |X - X'| / X against the bounds of the exit test: bit 0, not below
+// 1e-7; bit 1, above 1e-20 (the test of SparseSolverNUM.cpp:194-205 on the
+// largest quotient, started at 0, NaN never taken).  The quotient lies within a
+// factor of two of the power of two that the exponents give; it is formed where
+// that does not decide.
+__device__ __forceinline__ unsigned lu_change(double xo, double xn) {
+  const double d = fabs(xo - xn);
+  const int ex = (__double2hiint(xo) >> 20) & 0x7ff, ed = __double2hiint(d) >> 20;
+  if (ex > 0 && ex < 0x7ff && ed > 0 && ed < 0x7ff) {
+    if (__double2hiint(xo) < 0) return 0;
+    if (ed - ex >= -22) return 3;                    // > 2^-23 > 1e-7
+    if (ed - ex <= -25 && ed - ex >= -65) return 2;  // < 2^-24 < 1e-7, > 2^-66 > 1e-20
+  }
+  const double q = d / xo;
+  return (q >= 1e-7 ? 1u : 0u) | (q > 1e-10 * 1e-10 ? 2u : 0u);
+}
+
+__global__ void __launch_bounds__(kLuThreads, 1) k_lu_solve(const LuSolve S) {
+  extern __shared__ double sm[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), n_cta = (int)cl.num_blocks();
+  const LuVec y{sm, S.shift}, v{sm + S.rows, S.shift};
+  // this thread's rows of the row-parallel phases lie in its own CTA
+  const int r0 = rank * kLuThreads + threadIdx.x, stride = kLuThreads * n_cta;
+  // its rows of a level: the warps' groups of 32 go to the CTAs in turn
+  const int first = ((int)(threadIdx.x / 32) * n_cta + rank) * 32 + (int)(threadIdx.x % 32);
+  cl.sync();  // every CTA runs before its shared memory is used
+  int it = 0;
+  for (it = 0; it < kLuInterval; ++it) {
+    LuRow cur, nxt;
+    // ILUSGS: y = D^-1 sum_U U X; GS: v = b - sum_U U X
+    const LuGlobal x{S.x};
+    lu_fetch(cur, S.up, r0, S.dim);
+    for (int r = r0, j = threadIdx.x; r < S.dim; r += stride, j += kLuThreads) {
+      lu_fetch(nxt, S.up, r + stride, S.dim);
+      const double s = lu_row<false>(cur, S.up, x, 0.);
+      if (S.gs) v.base[j] = S.b[r] - s;
+      else y.base[j] = s / S.D[r];
+      cur = nxt;
+    }
+    if (!S.gs) {
+      // v = b + sum_L L y
+      lu_fetch(cur, S.lo, r0, S.dim);
+      cl.sync();
+      for (int r = r0, j = threadIdx.x; r < S.dim; r += stride, j += kLuThreads) {
+        lu_fetch(nxt, S.lo, r + stride, S.dim);
+        v.base[j] = S.b[r] + lu_row<false>(cur, S.lo, y, 0.);
+        cur = nxt;
+      }
+    }
+    cl.sync();
+    lu_sweep(S.fwd, v, first, stride);
+    if (!S.gs) {
+      for (int r = r0, j = threadIdx.x; r < S.dim; r += stride, j += kLuThreads) {
+        const double x1 = S.rD[r] * v.base[j];
+        v.base[j] = S.D[r] * x1;
+      }
+      cl.sync();
+      lu_sweep(S.bwd, v, first, stride);
+    }
+    // X = D^-1 v
+    unsigned ch = 0;
+    for (int r = r0, j = threadIdx.x; r < S.dim; r += stride, j += kLuThreads) {
+      const double xn = S.rD[r] * v.base[j];
+      ch |= lu_change(__ldcg(S.x + r), xn);
+      S.x[r] = xn;
+    }
+    const unsigned big = __syncthreads_or(ch & 1u), any = __syncthreads_or(ch & 2u);
+    if (threadIdx.x == 0) S.part[rank] = (big ? 1u : 0u) | (any ? 2u : 0u);
+    cl.sync();
+    ch = 0;
+    for (int q = 0; q < n_cta; ++q) ch |= __ldcg(S.part + q);
+    // the reference's exit test (:205, :245); the same value in every thread
+    if (ch == 2u) {
+      ++it;
+      break;
+    }
+  }
+  if (rank == 0 && threadIdx.x == 0) *S.its = it;
+  // (every access to another CTA's shared memory is followed by a cluster
+  // barrier above, so no CTA leaves too early)
+}
+
 // ---- host-side structure -----------------------------------------------------
 struct Csr {
   std::vector<int> ptr, col;
@@ -227,6 +426,12 @@ struct mst_lu {
   double *b = nullptr, *x = nullptr, *t1 = nullptr, *rhs = nullptr, *rhs1 = nullptr,
          *part = nullptr;
   std::vector<void*> allocs;
+  // the one-launch solve of scalar systems (cluster = 0: not used)
+  int cluster = 0;
+  LuRows r_up{}, r_lo{}, r_fwd{}, r_bwd{};
+  double* rD = nullptr;
+  unsigned* change = nullptr;
+  int* its = nullptr;
 };
 
 namespace {
@@ -292,6 +497,115 @@ cudaError_t up(mst_lu* s, T** dst, const std::vector<T>& v) {
   s->allocs.push_back(*dst);
   if (!v.empty()) e = cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
   return e;
+}
+
+// Rows in the given order with their first four entries at fixed places; a
+// sweep's entries times 1 / D[column] (the quotient and product the reference
+// forms at every use), a product's (rD = null) as they are
+cudaError_t up_rows(mst_lu* s, LuRows* out, const Csr& c, const std::vector<int>& rows,
+                    const std::vector<int>& lev, const std::vector<double>* rD) {
+  std::vector<int4> meta(rows.size()), col4(rows.size(), int4{0, 0, 0, 0});
+  std::vector<double4_32a> w4(rows.size(), double4_32a{0., 0., 0., 0.});
+  std::vector<int> col;
+  std::vector<double> w;
+  for (size_t i = 0; i < rows.size(); ++i) {
+    const int k0 = c.ptr[rows[i]], n = c.ptr[rows[i] + 1] - k0;
+    meta[i] = int4{rows[i], n, (int)col.size(), 0};
+    for (int k = 0; k < n; ++k) {
+      const int j = c.col[k0 + k];
+      const double q = rD ? c.val[k0 + k] * (*rD)[j] : c.val[k0 + k];
+      if (k < 4) {
+        (&col4[i].x)[k] = j;
+        (&w4[i].x)[k] = q;
+      } else {
+        col.push_back(j);
+        w.push_back(q);
+      }
+    }
+  }
+  int *d_lev = nullptr, *d_col = nullptr;
+  int4 *d_meta = nullptr, *d_col4 = nullptr;
+  double4_32a* d_w4 = nullptr;
+  double* d_w = nullptr;
+  cudaError_t e = up(s, &d_lev, lev);
+  if (e == cudaSuccess) e = up(s, &d_meta, meta);
+  if (e == cudaSuccess) e = up(s, &d_col4, col4);
+  if (e == cudaSuccess) e = up(s, &d_w4, w4);
+  if (e == cudaSuccess) e = up(s, &d_col, col);
+  if (e == cudaSuccess) e = up(s, &d_w, w);
+  *out = LuRows{d_lev, d_meta, d_col4, d_w4, d_col, d_w, (int)lev.size() - 1};
+  return e;
+}
+
+int lu_cta_rows(int cluster, int dim) {
+  const int span = cluster * kLuThreads;
+  return (dim + span - 1) / span * kLuThreads;
+}
+
+void lu_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int cluster, int dim,
+               cudaStream_t stream) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3(cluster);
+  cfg->blockDim = dim3(kLuThreads);
+  cfg->dynamicSmemBytes = 2 * sizeof(double) * (size_t)lu_cta_rows(cluster, dim);
+  cfg->stream = stream;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = cluster;
+  at->val.clusterDim.y = 1;
+  at->val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+}
+
+// The cluster of the one-launch solve: the largest the device places.  0, a
+// launch per level on the whole device, where the vectors do not fit the
+// cluster's shared memory (229,376 rows on 16 CTAs: still the faster there)
+int lu_pick_cluster(int dim) {
+  constexpr size_t kMaxSmem = 224 * 1024;
+  static std::atomic<uint64_t> attr_done{0};
+  if (mst::ensure_smem_limit(k_lu_solve, (int)kMaxSmem, attr_done) != cudaSuccess ||
+      cudaFuncSetAttribute(k_lu_solve, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  for (int nb = kLuMaxCta; nb >= 1; nb /= 2) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    lu_config(&cfg, &at, nb, dim, nullptr);
+    if (cfg.dynamicSmemBytes > kMaxSmem) break;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_lu_solve, &cfg) == cudaSuccess && n > 0) return nb;
+    cudaGetLastError();
+  }
+  return 0;
+}
+
+mst_status lu_solve_cluster(mst_lu* s, int gs, int* iterations) {
+  LuSolve a{};
+  a.dim = s->dim;
+  a.gs = gs;
+  while ((1 << a.shift) < s->cluster) ++a.shift;
+  a.rows = lu_cta_rows(s->cluster, s->dim);
+  a.up = s->r_up;
+  a.lo = s->r_lo;
+  a.fwd = s->r_fwd;
+  a.bwd = s->r_bwd;
+  a.D = s->D;
+  a.rD = s->rD;
+  a.b = s->b;
+  a.x = s->x;
+  a.part = s->change;
+  a.its = s->its;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  lu_config(&cfg, &at, s->cluster, s->dim, s->stream);
+  LU_CU(cudaLaunchKernelEx(&cfg, k_lu_solve, a));
+  int it = 0;
+  LU_CU(cudaMemcpyAsync(&it, s->its, sizeof it, cudaMemcpyDeviceToHost, s->stream));
+  LU_CU(cudaStreamSynchronize(s->stream));
+  if (iterations) *iterations = it;
+  return MST_OK;
 }
 
 template <int B>
@@ -379,21 +693,38 @@ mst_status mst_lu_create(int block, int dim, int n, const int* rows, const int* 
   levels(Ud, dim, false, &br, &s->bwd_ptr, &s->n_bwd_levels);
   cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = up(s, &s->D, D);
-  if (e == cudaSuccess) e = up(s, &s->l_ptr, L.ptr);
-  if (e == cudaSuccess) e = up(s, &s->l_col, L.col);
-  if (e == cudaSuccess) e = up(s, &s->l_val, L.val);
-  if (e == cudaSuccess) e = up(s, &s->ua_ptr, Ua.ptr);
-  if (e == cudaSuccess) e = up(s, &s->ua_col, Ua.col);
-  if (e == cudaSuccess) e = up(s, &s->ua_val, Ua.val);
-  if (e == cudaSuccess) e = up(s, &s->ud_ptr, Ud.ptr);
-  if (e == cudaSuccess) e = up(s, &s->ud_col, Ud.col);
-  if (e == cudaSuccess) e = up(s, &s->ud_val, Ud.val);
-  if (e == cudaSuccess) e = up(s, &s->fwd_rows, fr);
-  if (e == cudaSuccess) e = up(s, &s->bwd_rows, br);
   const std::vector<double> zero((size_t)dim * block, 0.0);
-  for (double** p : {&s->b, &s->x, &s->t1, &s->rhs, &s->rhs1})
+  for (double** p : {&s->b, &s->x})
     if (e == cudaSuccess) e = up(s, p, zero);
-  if (e == cudaSuccess) e = up(s, &s->part, std::vector<double>((dim + 127) / 128 + 1, 0.0));
+  if (block == 1) s->cluster = lu_pick_cluster(dim);
+  if (e == cudaSuccess && s->cluster > 0) {
+    std::vector<double> rD(dim);
+    std::vector<int> order(dim);
+    for (int r = 0; r < dim; ++r) rD[r] = 1. / D[r];
+    std::iota(order.begin(), order.end(), 0);
+    e = up_rows(s, &s->r_up, Ua, order, {0, dim}, nullptr);
+    if (e == cudaSuccess) e = up_rows(s, &s->r_lo, L, order, {0, dim}, nullptr);
+    if (e == cudaSuccess) e = up_rows(s, &s->r_fwd, L, fr, s->fwd_ptr, &rD);
+    if (e == cudaSuccess) e = up_rows(s, &s->r_bwd, Ud, br, s->bwd_ptr, &rD);
+    if (e == cudaSuccess) e = up(s, &s->rD, rD);
+    if (e == cudaSuccess) e = up(s, &s->change, std::vector<unsigned>(kLuMaxCta, 0u));
+    if (e == cudaSuccess) e = up(s, &s->its, std::vector<int>(1, 0));
+  } else {
+    if (e == cudaSuccess) e = up(s, &s->l_ptr, L.ptr);
+    if (e == cudaSuccess) e = up(s, &s->l_col, L.col);
+    if (e == cudaSuccess) e = up(s, &s->l_val, L.val);
+    if (e == cudaSuccess) e = up(s, &s->ua_ptr, Ua.ptr);
+    if (e == cudaSuccess) e = up(s, &s->ua_col, Ua.col);
+    if (e == cudaSuccess) e = up(s, &s->ua_val, Ua.val);
+    if (e == cudaSuccess) e = up(s, &s->ud_ptr, Ud.ptr);
+    if (e == cudaSuccess) e = up(s, &s->ud_col, Ud.col);
+    if (e == cudaSuccess) e = up(s, &s->ud_val, Ud.val);
+    if (e == cudaSuccess) e = up(s, &s->fwd_rows, fr);
+    if (e == cudaSuccess) e = up(s, &s->bwd_rows, br);
+    for (double** p : {&s->t1, &s->rhs, &s->rhs1})
+      if (e == cudaSuccess) e = up(s, p, zero);
+    if (e == cudaSuccess) e = up(s, &s->part, std::vector<double>((dim + 127) / 128 + 1, 0.0));
+  }
   if (e == cudaSuccess && block == 4) {
     e = up(s, &s->Di, std::vector<double>((size_t)dim * 16, 0.0));
     // D^-1 once: the reference re-inverts D[i] at every use, always to the
@@ -421,7 +752,8 @@ mst_status mst_lu_solve(mst_lu* s, int method, const double* b, double* x, int* 
   const size_t bytes = (size_t)s->dim * s->block * sizeof(double);
   LU_CU(cudaMemcpyAsync(s->b, b, bytes, cudaMemcpyHostToDevice, s->stream));
   LU_CU(cudaMemcpyAsync(s->x, x, bytes, cudaMemcpyHostToDevice, s->stream));
-  mst_status st = (s->block == 1) ? lu_iterate<1>(s, method == MST_LU_GS, iterations)
+  mst_status st = s->cluster      ? lu_solve_cluster(s, method == MST_LU_GS, iterations)
+                  : s->block == 1 ? lu_iterate<1>(s, method == MST_LU_GS, iterations)
                                   : lu_iterate<4>(s, 0, iterations);
   if (st) return st;
   LU_CU(cudaMemcpyAsync(x, s->x, bytes, cudaMemcpyDeviceToHost, s->stream));
