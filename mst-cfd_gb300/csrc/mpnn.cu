@@ -15,6 +15,7 @@
 #include "ctx.hpp"
 #include "tc_gemm.cuh"
 #include "tc_gemm_tma.cuh"
+#include "vec8.cuh"
 
 namespace mst {
 namespace tc {
@@ -47,17 +48,46 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// tensor map of a row-major [rows][K] BF16 matrix in 128-row x 64-K boxes,
-// 128-byte swizzle; rows beyond the matrix read as zeros
-bool bf16_tile_map(CUtensorMap* map, const void* base, int rows, int K) {
+// tensor map of a row-major [rows][cols] BF16 matrix in boxes of box_rows rows
+// x 64 columns, 128-byte swizzle; what lies beyond the matrix reads as zeros
+bool bf16_tile_map(CUtensorMap* map, const void* base, int rows, int cols, int box_rows) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)kBM};
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
   const cuuint32_t es[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
             box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+         CUDA_SUCCESS;
+}
+
+// MSTCFD_GEMM_TMA=0 keeps every GEMM on k_gemm_bf16 (for comparisons)
+bool use_tma() {
+  static const bool on = [] {
+    const char* v = std::getenv("MSTCFD_GEMM_TMA");
+    return !v || std::atoi(v) != 0;
+  }();
+  return on;
+}
+
+unsigned spin_limit() {
+  const long long lim = g_wait_limit.load(std::memory_order_relaxed);
+  return lim < 0 ? kSpinLimit : (unsigned)std::min<long long>(lim, 0xFFFFFFFFll);
+}
+
+// tensor map of an FP32 [rows][ld] matrix's first cols columns in boxes of 32 x
+// 32, 128-byte swizzle: the staged result tiles (stores clip at the matrix)
+bool f32_tile_map(CUtensorMap* map, const float* base, int rows, int cols, int ld) {
+  EncodeTiledFn fn = encode_tiled();
+  if (!fn || (ld & 3) || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  const cuuint32_t box[2] = {32, 32};
+  const cuuint32_t es[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box,
+            es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
          CUDA_SUCCESS;
 }
@@ -72,7 +102,8 @@ bool gemm_tma(const GemmArgs& a, cudaStream_t s, cudaError_t* err) {
       (reinterpret_cast<uintptr_t>(a.A) & 15) || (reinterpret_cast<uintptr_t>(a.B) & 15))
     return false;
   CUtensorMap ma, mb;
-  if (!bf16_tile_map(&ma, a.A, a.M, a.K) || !bf16_tile_map(&mb, a.B, a.N, a.K)) return false;
+  if (!bf16_tile_map(&ma, a.A, a.M, a.K, kBM) || !bf16_tile_map(&mb, a.B, a.N, a.K, kBM))
+    return false;
   static std::atomic<uint64_t> attr_done{0};
   const int kt = a.K / kBK;
   *err = ensure_smem_limit(k_gemm_tma, tma_smem_bytes(kTmaMaxKT), attr_done);
@@ -94,14 +125,31 @@ bool gemm_tma(const GemmArgs& a, cudaStream_t s, cudaError_t* err) {
   TmaGemm t;
   t.g = a;
   t.kt = kt;
+  CUtensorMap mc = ma, mi = ma;  // (not used unless staged)
+  t.staged = (!a.C || f32_tile_map(&mc, a.C, a.M, a.N, a.ldc)) &&
+             (!a.Cin || f32_tile_map(&mi, a.Cin, a.M, a.N, a.ldc)) &&
+             (!a.Cb || ((a.ldcb & 7) == 0 && (reinterpret_cast<uintptr_t>(a.Cb) & 15) == 0 &&
+                        a.N % 32 == 0)) &&
+             (!a.gate || a.N % 32 == 0);
   t.n_ntiles = (a.N + kBN - 1) / kBN;
   t.m_tiles = (a.M + kBM - 1) / kBM;
   // one wave of resident CTAs, each column block with the same number
   int grid = std::min(slots, t.n_ntiles * t.m_tiles);
   grid = std::max(t.n_ntiles, grid / t.n_ntiles * t.n_ntiles);
-  k_gemm_tma<<<grid, kTmaThreads, tma_smem_bytes(kt), s>>>(ma, mb, t);
+  k_gemm_tma<<<grid, kTmaThreads, tma_smem_bytes(kt), s>>>(ma, mb, mc, mi, t);
   *err = cudaGetLastError();
   return true;
+}
+
+template <bool ROWS>
+cudaError_t launch_split(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& a,
+                         cudaStream_t s) {
+  static std::atomic<uint64_t> attr_done{0};
+  const cudaError_t e = ensure_smem_limit(k_gemm_tma_split<ROWS>, split_smem_bytes(), attr_done);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((a.M + kBM - 1) / kBM, (a.N + kBN - 1) / kBN, (a.K + a.k_chunk - 1) / a.k_chunk);
+  k_gemm_tma_split<ROWS><<<grid, kSplitThreads, split_smem_bytes(), s>>>(ma, mb, a);
+  return cudaGetLastError();
 }
 
 // The split-K TMA kernel where it applies (K and the chunk in tiles of 64,
@@ -112,13 +160,28 @@ bool gemm_tma_split(const GemmArgs& a, cudaStream_t s, cudaError_t* err) {
       (reinterpret_cast<uintptr_t>(a.A) & 15) || (reinterpret_cast<uintptr_t>(a.B) & 15))
     return false;
   CUtensorMap ma, mb;
-  if (!bf16_tile_map(&ma, a.A, a.M, a.K) || !bf16_tile_map(&mb, a.B, a.N, a.K)) return false;
-  static std::atomic<uint64_t> attr_done{0};
-  *err = ensure_smem_limit(k_gemm_tma_split, split_smem_bytes(), attr_done);
-  if (*err != cudaSuccess) return true;
-  const dim3 grid((a.M + kBM - 1) / kBM, (a.N + kBN - 1) / kBN, (a.K + a.k_chunk - 1) / a.k_chunk);
-  k_gemm_tma_split<<<grid, kSplitThreads, split_smem_bytes(), s>>>(ma, mb, a);
-  *err = cudaGetLastError();
+  if (!bf16_tile_map(&ma, a.A, a.M, a.K, kBM) || !bf16_tile_map(&mb, a.B, a.N, a.K, kBM))
+    return false;
+  *err = launch_split<false>(ma, mb, a, s);
+  return true;
+}
+
+// The same with operands [n_rows][a_cols] and [n_rows][b_cols] (K = the rows,
+// M <= a_cols, N <= b_cols); false: the caller transposes
+bool gemm_tma_rows(const GemmArgs& a, int n_rows, int a_cols, int b_cols, cudaStream_t s,
+                   cudaError_t* err) {
+  *err = cudaSuccess;
+  if (!use_tma() || a.k_chunk <= 0 || a.k_chunk % kBK != 0 || a.K % kBK != 0 ||
+      a_cols % 8 != 0 || b_cols % 8 != 0 || (reinterpret_cast<uintptr_t>(a.A) & 15) ||
+      (reinterpret_cast<uintptr_t>(a.B) & 15))
+    return false;
+  CUtensorMap ma, mb;
+  if (!bf16_tile_map(&ma, a.A, n_rows, a_cols, kBK) ||
+      !bf16_tile_map(&mb, a.B, n_rows, b_cols, kBK))
+    return false;
+  GemmArgs g = a;
+  g.spin_limit = spin_limit();
+  *err = launch_split<true>(ma, mb, g, s);
   return true;
 }
 
@@ -129,14 +192,8 @@ cudaError_t gemm(const GemmArgs& a0, cudaStream_t s) {
                          : ensure_smem_limit(k_gemm_bf16<kBN>, kSmemBytes, attr_done);
   if (e != cudaSuccess) return e;
   GemmArgs a = a0;
-  const long long lim = g_wait_limit.load(std::memory_order_relaxed);
-  a.spin_limit = lim < 0 ? kSpinLimit : (unsigned)std::min<long long>(lim, 0xFFFFFFFFll);
-  // MSTCFD_GEMM_TMA=0 keeps every GEMM on k_gemm_bf16 (for comparisons)
-  static const bool use_tma = [] {
-    const char* v = std::getenv("MSTCFD_GEMM_TMA");
-    return !v || std::atoi(v) != 0;
-  }();
-  if (a.lbo == 0 && use_tma) {
+  a.spin_limit = spin_limit();
+  if (a.lbo == 0 && use_tma()) {
     cudaError_t te;
     if (a.k_chunk > 0 ? gemm_tma_split(a, s, &te) : gemm_tma(a, s, &te)) return te;
   }
@@ -155,14 +212,32 @@ cudaError_t gemm(const GemmArgs& a0, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// C[M][N] = sum over z of part[z][M][N], in z order (deterministic)
-__global__ void k_reduce_splits(const float* __restrict__ part, int splits, size_t mn,
-                                float* __restrict__ c) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= mn) return;
+// C[M][N] = sum over z of part[z][M][N], in a fixed order (deterministic): the
+// kReduceRows threads of an output each add a run of z, then the runs are added
+// in order.  (One thread an output: a chain of 293 loads, 16 us.)
+constexpr int kReduceRows = 8;
+__global__ void __launch_bounds__(32 * kReduceRows)
+    k_reduce_splits(const float* __restrict__ part, int splits, size_t mn, float* __restrict__ c) {
+  __shared__ float red[kReduceRows][32];
+  const size_t i = blockIdx.x * (size_t)32 + threadIdx.x;
+  const int run = (splits + kReduceRows - 1) / kReduceRows;
+  const int z1 = min(splits, (int)(threadIdx.y + 1) * run);
   float s = 0.f;
-  for (int z = 0; z < splits; ++z) s += part[(size_t)z * mn + i];
-  c[i] = s;
+  if (i < mn) {
+#pragma unroll 8
+    for (int z = threadIdx.y * run; z < z1; ++z) s += part[(size_t)z * mn + i];
+  }
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && i < mn) {
+    for (int q = 1; q < kReduceRows; ++q) s += red[q][threadIdx.x];
+    c[i] = s;
+  }
+}
+
+cudaError_t reduce_splits(const float* part, int splits, size_t mn, float* c) {
+  k_reduce_splits<<<(unsigned)((mn + 31) / 32), dim3(32, kReduceRows)>>>(part, splits, mn, c);
+  return cudaGetLastError();
 }
 
 }  // namespace tc
@@ -187,48 +262,129 @@ constexpr int kLayers = 3;
 constexpr int kZ = 2 * kW;    // [h, mean of neighbours]
 constexpr int kMaxSplits = 320;  // split-K CTAs of a weight-gradient GEMM
 
-__global__ void k_to_bf16(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, size_t n) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) y[i] = __float2bfloat16_rn(x[i]);
-}
+// Cells are walked by half warps, each lane eight of the 128 columns (32-byte
+// loads; four columns a lane and a warp a cell took twice the instructions: 49
+// and 82 us where this takes 41 and 72).  A block takes a run of consecutive
+// cells (neighbours' rows meet in its L1), its kCellWarps warps in turn, so that a
+// cell's neighbour ids are there when its rows are read.
+constexpr int kCellWarps = 8;
+constexpr int kHalf = 16;  // lanes of a cell
+constexpr unsigned kFull = 0xffffffffu;
 
-// Z = [bf16(h_c), bf16(mean_{j in N(c)} h_j)] (rows >= n: zero); one warp
-// per cell, each lane four features (16-byte loads, 8-byte stores), the
-// neighbours summed in list order
-constexpr int kCellsPerBlock = 8;
 __device__ __forceinline__ uint2 bf16x4(float4 v) {
   const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
   return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
-__global__ void __launch_bounds__(32 * kCellsPerBlock)
-    k_build_z(const float* __restrict__ h, const int* __restrict__ ptr,
-              const int* __restrict__ nbr, int n, int n_pad, __nv_bfloat16* __restrict__ z) {
-  const int c = blockIdx.x * kCellsPerBlock + (threadIdx.x >> 5), k = (threadIdx.x & 31) * 4;
-  if (c >= n_pad) return;
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), hc = a;
-  if (c < n) {
-    hc = *reinterpret_cast<const float4*>(h + (size_t)c * kW + k);
-    const int b = ptr[c], e = ptr[c + 1];
-    for (int i = b; i < e; ++i) {
-      const float4 v = *reinterpret_cast<const float4*>(h + (size_t)nbr[i] * kW + k);
-      a.x += v.x;
-      a.y += v.y;
-      a.z += v.z;
-      a.w += v.w;
-    }
-    if (e > b) {
-      const float d = (float)(e - b);
-      a.x /= d;
-      a.y /= d;
-      a.z /= d;
-      a.w /= d;
-    }
-  }
-  *reinterpret_cast<uint2*>(z + (size_t)c * kZ + k) = bf16x4(hc);
-  *reinterpret_cast<uint2*>(z + (size_t)c * kZ + kW + k) = bf16x4(a);
+struct F8 {
+  float x[8];
+};
+__device__ __forceinline__ F8 ld8(const float* p) {
+  F8 r;
+  mst::load8(p, r.x);
+  return r;
+}
+__device__ __forceinline__ void st_bf16x8(__nv_bfloat16* p, const F8& v) {
+  const uint2 lo = bf16x4(make_float4(v.x[0], v.x[1], v.x[2], v.x[3])),
+              hi = bf16x4(make_float4(v.x[4], v.x[5], v.x[6], v.x[7]));
+  *reinterpret_cast<uint4*>(p) = make_uint4(lo.x, lo.y, hi.x, hi.y);
 }
 
-// dst[w][n_pad] = transpose of src[n][w] (BF16), zero for rows >= n
+// x / d for a cell's degree d, r = 1 / d: the product with the reciprocal and
+// one residual correction (Markstein 1990), equal to the correctly rounded
+// quotient for every x of normal range and d = 1..256 (all significands
+// compared).  The division itself takes four times the instructions, and its
+// slow path wherever a numerator is zero, as relu outputs often are: 20 us of
+// k_build_z's 75 at 168,594 cells.
+__device__ __forceinline__ F8 div_deg(F8 v, float d, float r) {
+  float m = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v.x[i]));
+  if (m == __int_as_float(0x7f800000) || d > 256.f) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v.x[i] /= d;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float q = v.x[i] * r;
+      v.x[i] = fmaf(fmaf(-q, d, v.x[i]), r, q);
+    }
+  }
+  return v;
+}
+
+// The cells of one half warp, every 2 kCellWarps-th: their neighbour ranges and
+// ids (lane i the i-th) read one cell ahead
+struct CellWalk {
+  const int *ptr, *nbr;
+  int n, sub, b, e, id, nb, ne, nid;
+  __device__ __forceinline__ void fetch(int c) {
+    nb = ne = 0;
+    if (c < n) {
+      nb = ptr[c];
+      ne = ptr[c + 1];
+    }
+    nid = nb + sub < ne ? nbr[nb + sub] : 0;
+  }
+  __device__ __forceinline__ void next() {
+    b = nb;
+    e = ne;
+    id = nid;
+  }
+};
+
+// add(k, whether the cell has a k-th neighbour, it, its row) in list order; both
+// halves of a warp go through the longer list.  (Rows loaded two or three at a
+// time cost registers and with them warps: 78 and 85 us for 72 in k_back.)
+template <class Load, class Add>
+__device__ __forceinline__ void walk_neighbours(const CellWalk& w, Load load, Add add) {
+  const int deg = w.e - w.b, most = max(deg, __shfl_xor_sync(kFull, deg, kHalf));
+  for (int k = 0; k < most; ++k) {
+    int id = __shfl_sync(kFull, w.id, k & (kHalf - 1), kHalf);
+    if (k >= kHalf && k < deg) id = w.nbr[w.b + k];
+    F8 v{};
+    if (k < deg) v = load(id);
+    add(k, k < deg, id, v);
+  }
+}
+
+// Z = [bf16(h_c), bf16(mean_{j in N(c)} h_j)] (rows >= n: zero), the neighbours
+// summed in list order
+__global__ void __launch_bounds__(32 * kCellWarps, 4)
+    k_build_z(const float* __restrict__ h, const int* __restrict__ ptr,
+              const int* __restrict__ nbr, int n, int n_pad, __nv_bfloat16* __restrict__ z) {
+  const int sub = threadIdx.x & (kHalf - 1), k = sub * 8;
+  const int chunk = (n_pad + gridDim.x - 1) / gridDim.x;
+  const int last = min(n_pad, (int)(blockIdx.x + 1) * chunk);
+  int c = blockIdx.x * chunk + threadIdx.x / kHalf;
+  CellWalk w{ptr, nbr, n, sub};
+  w.fetch(c);
+  // (a warp leaves together)
+  for (; c - (int)(threadIdx.x / kHalf & 1) < last; c += 2 * kCellWarps) {
+    w.next();
+    w.fetch(c + 2 * kCellWarps);
+    F8 a{}, hc{};
+    if (c < min(n, last)) hc = ld8(h + (size_t)c * kW + k);
+    walk_neighbours(
+        w, [&](int j) { return ld8(h + (size_t)j * kW + k); },
+        [&](int, bool there, int, const F8& v) {
+          if (there) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a.x[i] += v.x[i];
+          }
+        });
+    if (w.e > w.b) {
+      const float d = (float)(w.e - w.b);
+      a = div_deg(a, d, 1.f / d);
+    }
+    if (c < last) {
+      st_bf16x8(z + (size_t)c * kZ + k, hc);
+      st_bf16x8(z + (size_t)c * kZ + kW + k, a);
+    }
+  }
+}
+
+// dst[w][n_pad] = transpose of src[n][w] (BF16), zero for rows >= n: the
+// operands of the GEMMs that k_gemm_bf16 takes over
 __global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ src, int n, int w,
                                  int n_pad, __nv_bfloat16* __restrict__ dst) {
   __shared__ __nv_bfloat16 t[32][33];
@@ -244,106 +400,180 @@ __global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ src, int n, i
   }
 }
 
-// loss and dY = 2 (y - t) / (n * kOut); per-block partial losses
-__global__ void k_mse(const float* __restrict__ y, const float* __restrict__ t, int n,
-                      float* __restrict__ dy, double* __restrict__ part) {
+// loss and dY = 2 (y - t) / (n * kOut), the latter as the BF16 operand [np][64]
+// (columns >= 4 and rows >= n zero); per-block partial losses and column sums.
+// 64 cells a block.
+__global__ void __launch_bounds__(256)
+    k_mse(const float* __restrict__ y, const float* __restrict__ t, int n,
+          __nv_bfloat16* __restrict__ dyb, double* __restrict__ part, float* __restrict__ cpart) {
   __shared__ double red[256];
+  __shared__ float dy[256];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double l = 0.0;
+  float g = 0.f;
   if (i < n * kOut) {
     const float d = y[i] - t[i];
-    dy[i] = 2.f * d / (float)(n * kOut);
+    g = 2.f * d / (float)(n * kOut);
     l = (double)d * d;
   }
   red[threadIdx.x] = l;
+  dy[threadIdx.x] = g;
+  __syncthreads();
+  for (int q = threadIdx.x; q < 64 * (kInK / 8); q += 256) {
+    const int r = q / (kInK / 8), c = q % (kInK / 8);
+    uint4 o = make_uint4(0u, 0u, 0u, 0u);
+    if (c == 0) {
+      const uint2 b = bf16x4(make_float4(dy[4 * r], dy[4 * r + 1], dy[4 * r + 2], dy[4 * r + 3]));
+      o.x = b.x;
+      o.y = b.y;
+    }
+    reinterpret_cast<uint4*>(dyb)[((size_t)blockIdx.x * 64 + r) * (kInK / 8) + c] = o;
+  }
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    if ((int)threadIdx.x < w) {
+      red[threadIdx.x] += red[threadIdx.x + w];
+      if (w >= kOut) dy[threadIdx.x] += dy[threadIdx.x + w];
+    }
     __syncthreads();
   }
   if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+  if (threadIdx.x < kOut) cpart[(size_t)blockIdx.x * kOut + threadIdx.x] = dy[threadIdx.x];
 }
 
-// dP = dH (.) [r > 0] with r = h_next - h_prev (the relu output), FP32 and a
-// BF16 copy; pad rows zero
-__global__ void k_relu_back(const float* __restrict__ dh, const float* __restrict__ hn,
-                            const float* __restrict__ hp, int n, int n_pad,
-                            float* __restrict__ dp, __nv_bfloat16* __restrict__ dpb) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= (size_t)n_pad * kW) return;
-  float v = 0.f;
-  if (i < (size_t)n * kW) {
-    const float r = hp ? hn[i] - hp[i] : hn[i];
-    v = r > 0.f ? dh[i] : 0.f;
+// One backward step between two dense products.  AGG: dH_l = dH_{l+1} +
+// dZ[:, :kW] + sum_{c in N(j)} dZ[c, kW:] / |N(c)| (neighbours in list order),
+// stored to dh if a further layer needs it; otherwise dH is read.  Then dP =
+// dH (.) [relu output > 0] (the gate bits of the forward product) as the BF16
+// operand (rows >= n zero), and its FP32 column sums per block -- the bias
+// gradient -- without an FP32 dP in memory.  Bound by its bytes: dH and dZ in,
+// dH and dP out.
+template <bool AGG>
+__global__ void __launch_bounds__(32 * kCellWarps, 4)
+    k_back(const float* __restrict__ dhn, const float* __restrict__ dz,
+           const int* __restrict__ ptr, const int* __restrict__ nbr,
+           const uint8_t* __restrict__ gate, int n, int n_pad, float* __restrict__ dh,
+           __nv_bfloat16* __restrict__ dpb, float* __restrict__ cpart) {
+  __shared__ float red[2 * kCellWarps][kW];
+  const int sub = threadIdx.x & (kHalf - 1), k = sub * 8;
+  const int chunk = (n_pad + gridDim.x - 1) / gridDim.x;
+  const int last = min(n_pad, (int)(blockIdx.x + 1) * chunk);
+  int j = blockIdx.x * chunk + threadIdx.x / kHalf;
+  F8 s{};
+  CellWalk w{ptr, nbr, n, sub};
+  if (AGG) w.fetch(j);
+  // (a warp leaves together)
+  for (; j - (int)(threadIdx.x / kHalf & 1) < last; j += 2 * kCellWarps) {
+    F8 v{};
+    unsigned g = 0;
+    const bool live = j < min(n, last);
+    if (AGG) {
+      w.next();
+      w.fetch(j + 2 * kCellWarps);
+    }
+    if (live) {
+      g = gate[(size_t)j * (kW / 8) + sub];
+      v = ld8(dhn + (size_t)j * kW + k);
+    }
+    if (AGG) {
+      // lane i: the degree of the i-th neighbour and its reciprocal
+      const float dl = sub < w.e - w.b ? (float)(ptr[w.id + 1] - ptr[w.id]) : 1.f, rl = 1.f / dl;
+      if (live) {
+        const F8 y = ld8(dz + (size_t)j * kZ + k);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v.x[i] += y.x[i];
+      }
+      walk_neighbours(
+          w, [&](int c) { return ld8(dz + (size_t)c * kZ + kW + k); },
+          [&](int i, bool there, int c, const F8& u) {
+            float d = __shfl_sync(kFull, dl, i & (kHalf - 1), kHalf);
+            float r = __shfl_sync(kFull, rl, i & (kHalf - 1), kHalf);
+            if (!there) return;
+            if (i >= kHalf) {
+              d = (float)(ptr[c + 1] - ptr[c]);
+              r = 1.f / d;
+            }
+            const F8 q = div_deg(u, d, r);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) v.x[t] += q.x[t];
+          });
+      if (dh && live) mst::store8(dh + (size_t)j * kW + k, v.x);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v.x[i] = (g >> i & 1u) ? v.x[i] : 0.f;
+      s.x[i] += v.x[i];
+    }
+    if (j < last) st_bf16x8(dpb + (size_t)j * kW + k, v);
   }
-  dp[i] = v;
-  dpb[i] = __float2bfloat16_rn(v);
-}
-
-// dH_l = dH_{l+1} + dZ[:, :kW] + sum_{c in N(j)} dZ[c, kW:] / |N(c)|; one
-// warp per cell, each lane four features, the neighbours in list order
-__global__ void __launch_bounds__(32 * kCellsPerBlock)
-    k_agg_back(const float* __restrict__ dhn, const float* __restrict__ dz,
-               const int* __restrict__ ptr, const int* __restrict__ nbr, int n,
-               float* __restrict__ dh) {
-  const int j = blockIdx.x * kCellsPerBlock + (threadIdx.x >> 5), k = (threadIdx.x & 31) * 4;
-  if (j >= n) return;
-  const float4 x = *reinterpret_cast<const float4*>(dhn + (size_t)j * kW + k);
-  const float4 y = *reinterpret_cast<const float4*>(dz + (size_t)j * kZ + k);
-  float4 v = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
-  for (int i = ptr[j]; i < ptr[j + 1]; ++i) {
-    const int c = nbr[i];
-    const float deg = (float)(ptr[c + 1] - ptr[c]);
-    const float4 u = *reinterpret_cast<const float4*>(dz + (size_t)c * kZ + kW + k);
-    v.x += u.x / deg;
-    v.y += u.y / deg;
-    v.z += u.z / deg;
-    v.w += u.w / deg;
-  }
-  *reinterpret_cast<float4*>(dh + (size_t)j * kW + k) = v;
-}
-
-// Column sums of g[n][w] (bias gradients), w dividing 256, in a fixed order
-// (deterministic): block b sums rows [b*chunk, (b+1)*chunk), its 256 threads
-// reading whole rows (thread t: column t % w, row offset t / w), into
-// part[b][w]; k_colsum_parts then adds the blocks' partials in block order.
-__global__ void __launch_bounds__(256) k_colsum(const float* __restrict__ g, int n, int w,
-                                                int chunk, float* __restrict__ part) {
-  __shared__ float red[256];
-  const int t = threadIdx.x, col = t % w, rows = 256 / w;
-  const int r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
-  float s = 0.f;
-  for (int r = r0 + t / w; r < r1; r += rows) s += g[(size_t)r * w + col];
-  red[t] = s;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) red[threadIdx.x / kHalf][k + i] = s.x[i];
   __syncthreads();
-  if (t < w) {
-    float acc = red[t];
-    for (int k = 1; k < rows; ++k) acc += red[t + k * w];
-    part[(size_t)blockIdx.x * w + t] = acc;
+  if (threadIdx.x < kW) {
+    float a = red[0][threadIdx.x];
+    for (int q = 1; q < 2 * kCellWarps; ++q) a += red[q][threadIdx.x];
+    cpart[(size_t)blockIdx.x * kW + threadIdx.x] = a;
   }
 }
-__global__ void k_colsum_parts(const float* __restrict__ part, int blocks, int w,
-                               float* __restrict__ out) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= w) return;
+
+// out[w] = column sums of the blocks' partials part[blocks][w], w <= 128, in a
+// fixed order: thread (r, c) of a block takes every 32nd partial of column c
+__global__ void __launch_bounds__(1024) k_colsum_parts(const float* __restrict__ part, int blocks,
+                                                       int w, float* __restrict__ out) {
+  __shared__ float red[32][33];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), r = threadIdx.x >> 5;
   float acc = 0.f;
-  for (int b = 0; b < blocks; ++b) acc += part[(size_t)b * w + col];
-  out[col] = acc;
+  if (c < w) {
+#pragma unroll 8
+    for (int b = r; b < blocks; b += 32) acc += part[(size_t)b * w + c];
+  }
+  red[r][threadIdx.x & 31] = acc;
+  __syncthreads();
+  if (r == 0 && c < w) {
+    for (int q = 1; q < 32; ++q) acc += red[q][threadIdx.x];
+    out[c] = acc;
+  }
 }
 
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, int n, float lr, float b1, float b2, float c1,
-                       float c2, __nv_bfloat16* __restrict__ wb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float x = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
-  w[i] = x;
-  if (wb) wb[i] = __float2bfloat16_rn(x);
+// the transposes of the weights that the data gradients need, in one launch
+// (blockIdx.z: which); dst[cols][rows_pad], zero for rows >= rows
+struct WeightT {
+  const __nv_bfloat16* src[kLayers + 1];
+  __nv_bfloat16* dst[kLayers + 1];
+  int rows[kLayers + 1], cols[kLayers + 1], pad[kLayers + 1];
+};
+__global__ void k_transpose_weights(const WeightT t) {
+  __shared__ __nv_bfloat16 s[32][33];
+  const int z = blockIdx.z, r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  const int R = t.rows[z], W = t.cols[z], pad = t.pad[z];
+  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
+    const int r = r0 + i, c = c0 + threadIdx.x;
+    s[i][threadIdx.x] = (r < R && c < W) ? t.src[z][(size_t)r * W + c] : __float2bfloat16_rn(0.f);
+  }
+  __syncthreads();
+  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
+    const int c = c0 + i, r = r0 + threadIdx.x;
+    if (c < W && r < pad) t.dst[z][(size_t)c * pad + r] = s[threadIdx.x][i];
+  }
+}
+
+struct AdamTensors {  // blockIdx.y: which
+  float *w[2 * (kLayers + 2)], *m[2 * (kLayers + 2)], *v[2 * (kLayers + 2)];
+  const float* g[2 * (kLayers + 2)];
+  __nv_bfloat16* wb[2 * (kLayers + 2)];
+  int n[2 * (kLayers + 2)];
+};
+__global__ void k_adam(const AdamTensors t, float lr, float b1, float b2, float c1, float c2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  if (i >= t.n[q]) return;
+  const float gi = t.g[q][i];
+  const float mi = b1 * t.m[q][i] + (1.f - b1) * gi;
+  const float vi = b2 * t.v[q][i] + (1.f - b2) * gi * gi;
+  t.m[q][i] = mi;
+  t.v[q][i] = vi;
+  const float x = t.w[q][i] - lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
+  t.w[q][i] = x;
+  t.wb[q][i] = __float2bfloat16_rn(x);
 }
 
 }  // namespace
@@ -360,18 +590,21 @@ struct MpnnParam {
 
 struct mst_mpnn {
   MpnnParam W[2 * (kLayers + 2)];  // We, be, Wl0, bl0, ..., Wd, bd
+  // the tensors of W lie one after another in these
+  float *w = nullptr, *g = nullptr, *m1 = nullptr, *v1 = nullptr;
+  __nv_bfloat16* wb = nullptr;
   int step = 0;
   // work buffers for up to cap cells
   int cap = 0;
   int* err = nullptr;
   double* lpart = nullptr;
   std::vector<void*> bufs;
-  float* H[kLayers + 1] = {};      // FP32 residual stream
+  float* H[kLayers] = {};          // FP32 residual stream (the last only as Hb)
   __nv_bfloat16 *X = nullptr, *Z[kLayers] = {}, *Hb = nullptr;
-  float *Y = nullptr, *T = nullptr, *dY = nullptr, *dH = nullptr, *dHn = nullptr,
-        *dP = nullptr, *dZ = nullptr;
-  __nv_bfloat16 *dPb = nullptr, *tA = nullptr, *tB = nullptr, *dYb = nullptr, *WdT = nullptr,
-                *WlT = nullptr;
+  uint16_t* gate[kLayers + 1] = {};  // [cap][8] bits: the layer's relu output > 0
+  float *Y = nullptr, *T = nullptr, *dH = nullptr, *dHn = nullptr, *dZ = nullptr;
+  __nv_bfloat16 *dPb = nullptr, *dYb = nullptr, *WdT = nullptr, *WlT[kLayers] = {};
+  __nv_bfloat16 *tA = nullptr, *tB = nullptr;  // transposed operands, where they are needed
   float* part = nullptr;  // split-K partial products of the weight gradients
   float* feat = nullptr;  // the graph's FP32 features [cap][16]
   int *ptr = nullptr, *nbr = nullptr;
@@ -420,28 +653,28 @@ cudaError_t ensure_cap(mst_mpnn* m, int n, int n_nbr) {
   // grow: free the old work buffers (parameters live in m->W)
   for (void* p : m->bufs) cudaFree(p);
   m->bufs.clear();
-  const int np = pad128(n), nk = pad64(n);
+  const int np = pad128(n);
   m->cap = n;
-  for (int l = 0; l <= kLayers && e == cudaSuccess; ++l) e = nalloc(m, &m->H[l], (size_t)np * kW);
+  m->tA = m->tB = nullptr;
+  for (int l = 0; l < kLayers && e == cudaSuccess; ++l) e = nalloc(m, &m->H[l], (size_t)np * kW);
   for (int l = 0; l < kLayers && e == cudaSuccess; ++l) e = nalloc(m, &m->Z[l], (size_t)np * kZ);
+  for (int l = 0; l <= kLayers && e == cudaSuccess; ++l)
+    e = nalloc(m, &m->gate[l], (size_t)np * (kW / 16));
   if (e == cudaSuccess) e = nalloc(m, &m->X, (size_t)np * kInK);
   if (e == cudaSuccess) e = nalloc(m, &m->Hb, (size_t)np * kW);
   if (e == cudaSuccess) e = nalloc(m, &m->Y, (size_t)np * kOut);
   if (e == cudaSuccess) e = nalloc(m, &m->T, (size_t)np * kOut);
-  if (e == cudaSuccess) e = nalloc(m, &m->dY, (size_t)np * kOut);
   if (e == cudaSuccess) e = nalloc(m, &m->dYb, (size_t)np * kInK);
   if (e == cudaSuccess) e = nalloc(m, &m->dH, (size_t)np * kW);
   if (e == cudaSuccess) e = nalloc(m, &m->dHn, (size_t)np * kW);
-  if (e == cudaSuccess) e = nalloc(m, &m->dP, (size_t)np * kW);
   if (e == cudaSuccess) e = nalloc(m, &m->dPb, (size_t)np * kW);
   if (e == cudaSuccess) e = nalloc(m, &m->dZ, (size_t)np * kZ);
-  if (e == cudaSuccess) e = nalloc(m, &m->tA, (size_t)kZ * nk);
-  if (e == cudaSuccess) e = nalloc(m, &m->tB, (size_t)kZ * nk);
   if (e == cudaSuccess) e = nalloc(m, &m->ptr, (size_t)n + 1);
   if (e == cudaSuccess) e = nalloc(m, &m->lpart, (size_t)(np * kOut + 255) / 256 + 1);
   if (e == cudaSuccess) e = nalloc(m, &m->err, 1);
   if (e == cudaSuccess) e = nalloc(m, &m->WdT, (size_t)kW * kInK);
-  if (e == cudaSuccess) e = nalloc(m, &m->WlT, (size_t)kZ * kW);
+  for (int l = 0; l < kLayers && e == cudaSuccess; ++l)
+    e = nalloc(m, &m->WlT[l], (size_t)kZ * kW);
   if (e == cudaSuccess) e = nalloc(m, &m->part, (size_t)kMaxSplits * kW * kZ);
   if (e == cudaSuccess) e = nalloc(m, &m->feat, (size_t)n * kIn);
   return e;
@@ -468,40 +701,62 @@ struct GemmTimer {
   }
 };
 
+// what a product writes beside (or instead of) C
+struct Side {
+  const float* Cin = nullptr;  // residual added
+  __nv_bfloat16* Cb = nullptr;
+  uint16_t* gate = nullptr;
+};
+
 cudaError_t gemm(mst_mpnn* m, const __nv_bfloat16* A, const __nv_bfloat16* B, float* C, int M,
-                 int N, int K, int ldc, const float* bias, int relu, int acc) {
+                 int N, int K, int ldc, const float* bias, int relu, const Side& side = Side()) {
   GemmTimer timer(m, 2.0 * M * N * K,
-                  2.0 * ((double)M * K + (double)N * K) + 4.0 * M * N * (acc ? 2 : 1));
+                  2.0 * ((double)M * K + (double)N * K) + (C ? 4.0 * M * N : 0.0) +
+                      (side.Cin ? 4.0 * M * N : 0.0) + (side.Cb ? 2.0 * M * N : 0.0) +
+                      (side.gate ? M * N / 8.0 : 0.0));
   mst::tc::GemmArgs g{};
   g.A = A;
   g.B = B;
   g.C = C;
+  g.Cin = side.Cin;
+  g.Cb = side.Cb;
+  g.gate = side.gate;
   g.bias = bias;
   g.M = M;
   g.N = N;
   g.K = K;
   g.ldc = ldc;
+  g.ldcb = ldc;
   g.relu = relu;
-  g.accumulate_c = acc;
   g.err = m->err;
   return mst::tc::gemm(g, 0);
 }
 
-// Weight gradients: M, N small (<= 256), K = the number of cells.  Split K
-// over up to kMaxSplits CTAs per output tile, then add the partial products
-// in a fixed order.
-cudaError_t gemm_wgrad(mst_mpnn* m, const __nv_bfloat16* A, const __nv_bfloat16* B, float* C,
-                       int M, int N, int K, int ldc) {
+cudaError_t transpose(const __nv_bfloat16* src, int n, int w, int n_pad, __nv_bfloat16* dst) {
+  dim3 grid((n_pad + 31) / 32, (w + 31) / 32), block(32, 8);
+  k_transpose_bf16<<<grid, block>>>(src, n, w, n_pad, dst);
+  return cudaGetLastError();
+}
+
+// SMs of the device (read once, thread-safe; it only sizes grids)
+int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    n = 152;
+  return n;
+}
+
+// Weight gradients C[M][N] = A^T B over the n cells: A [n][a_cols], B
+// [n][b_cols] with M <= a_cols, N <= b_cols (<= 256).  Split over up to
+// kMaxSplits CTAs per output tile, then add the partial products in a fixed
+// order.
+cudaError_t gemm_wgrad(mst_mpnn* m, const __nv_bfloat16* A, int a_cols, const __nv_bfloat16* B,
+                       int b_cols, float* C, int M, int N, int n, int ldc) {
+  const int K = pad64(n);
   const int kt = K / mst::tc::kBK;  // K tiles
-  // about two CTAs per SM over the output tiles, each with at least 4 K
-  // tiles (the SM count read once, thread-safe; it only sizes the split)
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      n = 148;
-    return n;
-  }();
+  // about two CTAs per SM over the output tiles, each with at least 4 K tiles
+  static const int sms = sm_count();
   const int n_tiles = ((M + mst::tc::kBM - 1) / mst::tc::kBM) * ((N + mst::tc::kBN - 1) / mst::tc::kBN);
   const int splits =
       std::min(kMaxSplits, std::max(1, std::min(2 * sms / std::max(1, n_tiles), kt / 4)));
@@ -521,129 +776,131 @@ cudaError_t gemm_wgrad(mst_mpnn* m, const __nv_bfloat16* A, const __nv_bfloat16*
   {
     GemmTimer timer(m, 2.0 * M * N * K,
                     2.0 * ((double)M * K + (double)N * K) + 4.0 * used * M * N);
-    e = mst::tc::gemm(g, 0);
+    if (!mst::tc::gemm_tma_rows(g, n, a_cols, b_cols, 0, &e)) {
+      // k_gemm_bf16 reads [M][K] and [N][K]
+      const size_t nk = pad64(m->cap);
+      e = cudaSuccess;
+      if (!m->tA) e = nalloc(m, &m->tA, kZ * nk);
+      if (e == cudaSuccess && !m->tB) e = nalloc(m, &m->tB, kZ * nk);
+      if (e == cudaSuccess) e = transpose(A, n, a_cols, K, m->tA);
+      if (e == cudaSuccess) e = transpose(B, n, b_cols, K, m->tB);
+      g.A = m->tA;
+      g.B = m->tB;
+      if (e == cudaSuccess) e = mst::tc::gemm(g, 0);
+    }
   }
   if (e != cudaSuccess) return e;
   const size_t mn = (size_t)M * ldc;
-  mst::tc::k_reduce_splits<<<(unsigned)((mn + 255) / 256), 256>>>(m->part, used, mn, C);
-  return cudaGetLastError();
+  return mst::tc::reduce_splits(m->part, used, mn, C);
 }
 
-// bias gradient out[w] = column sums of g[n][w], through the split-K
-// partial buffer (free between weight-gradient GEMMs)
-void colsum(mst_mpnn* m, const float* g, int n, int w, float* out) {
-  const int blocks = std::max(1, std::min(296, (n + 255) / 256));
-  const int chunk = (n + blocks - 1) / blocks;
-  k_colsum<<<blocks, 256>>>(g, n, w, chunk, m->part);
-  k_colsum_parts<<<(w + 127) / 128, 128>>>(m->part, blocks, w, out);
+// bias gradient from the blocks' column sums in the split-K partial buffer
+// (free between weight-gradient GEMMs)
+void colsum(mst_mpnn* m, int blocks, int w, float* out) {
+  k_colsum_parts<<<(w + 31) / 32, 1024>>>(m->part, blocks, w, out);
 }
 
-cudaError_t transpose(const __nv_bfloat16* src, int n, int w, int n_pad, __nv_bfloat16* dst) {
-  dim3 grid((n_pad + 31) / 32, (w + 31) / 32), block(32, 8);
-  k_transpose_bf16<<<grid, block>>>(src, n, w, n_pad, dst);
-  return cudaGetLastError();
+// blocks of the kernels that walk cells by warps: up to 8 an SM, so that a warp
+// has several cells where there are many
+int cell_blocks(int n_pad) {
+  static const int sms = sm_count();
+  return std::min((n_pad + 2 * kCellWarps - 1) / (2 * kCellWarps), 8 * sms);
 }
 
 // forward over the graph loaded in m (n cells); Y = outputs
 cudaError_t forward(mst_mpnn* m, int n) {
   const int np = pad128(n);
-  cudaError_t e = gemm(m, m->X, P(m, kWe).wb, m->H[0], np, kW, kInK, kW, P(m, kBe).w, 1, 0);
+  Side side;
+  side.gate = m->gate[0];
+  cudaError_t e =
+      gemm(m, m->X, P(m, kWe).wb, m->H[0], np, kW, kInK, kW, P(m, kBe).w, 1, side);
   for (int l = 0; l < kLayers && e == cudaSuccess; ++l) {
-    k_build_z<<<(np + kCellsPerBlock - 1) / kCellsPerBlock, 32 * kCellsPerBlock>>>(
-        m->H[l], m->ptr, m->nbr, n, np, m->Z[l]);
-    e = cudaMemcpyAsync(m->H[l + 1], m->H[l], sizeof(float) * (size_t)np * kW,
-                        cudaMemcpyDeviceToDevice, 0);
-    if (e == cudaSuccess)
-      e = gemm(m, m->Z[l], P(m, wl(l)).wb, m->H[l + 1], np, kW, kZ, kW, P(m, bl(l)).w, 1, 1);
+    k_build_z<<<cell_blocks(np), 32 * kCellWarps>>>(m->H[l], m->ptr, m->nbr, n, np, m->Z[l]);
+    // h_{l+1}: the next layer reads it in FP32, the decoder as its BF16 operand
+    const bool last = l + 1 == kLayers;
+    side.Cin = m->H[l];
+    side.gate = m->gate[l + 1];
+    side.Cb = last ? m->Hb : nullptr;
+    e = gemm(m, m->Z[l], P(m, wl(l)).wb, last ? nullptr : m->H[l + 1], np, kW, kZ, kW,
+             P(m, bl(l)).w, 1, side);
   }
-  if (e == cudaSuccess) {
-    const size_t cnt = (size_t)np * kW;
-    k_to_bf16<<<(unsigned)((cnt + 255) / 256), 256>>>(m->H[kLayers], m->Hb, cnt);
-    e = gemm(m, m->Hb, P(m, kWd).wb, m->Y, np, kOut, kW, kOut, P(m, kBd).w, 0, 0);
-  }
+  if (e == cudaSuccess)
+    e = gemm(m, m->Hb, P(m, kWd).wb, m->Y, np, kOut, kW, kOut, P(m, kBd).w, 0);
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 // backward of the mean squared error against m->T; gradients into W[].g;
 // returns the loss through *loss
 cudaError_t backward(mst_mpnn* m, int n, double* loss) {
-  const int np = pad128(n), nk = pad64(n);
-  const int nb = (n * kOut + 255) / 256;
-  k_mse<<<nb, 256>>>(m->Y, m->T, n, m->dY, m->lpart);
-  cudaError_t e = cudaGetLastError();
+  const int np = pad128(n), nb = np / 64, cb = cell_blocks(np);
+  cudaError_t e = cudaSuccess;
+  {
+    WeightT t;
+    for (int l = 0; l < kLayers; ++l) {  // Wl^T [256][128]
+      t.src[l] = P(m, wl(l)).wb;
+      t.dst[l] = m->WlT[l];
+      t.rows[l] = t.pad[l] = kW;
+      t.cols[l] = kZ;
+    }
+    t.src[kLayers] = P(m, kWd).wb;  // Wd^T [128][64], K = 4 padded with zeros
+    t.dst[kLayers] = m->WdT;
+    t.rows[kLayers] = kOut;
+    t.cols[kLayers] = kW;
+    t.pad[kLayers] = kInK;
+    k_transpose_weights<<<dim3(kW / 32, kZ / 32, kLayers + 1), dim3(32, 8)>>>(t);
+  }
+  // decoder: dWd = dY^T H3, dbd = colsum dY, dH3 = dY Wd
+  k_mse<<<nb, 256>>>(m->Y, m->T, n, m->dYb, m->lpart, m->part);
+  colsum(m, nb, kOut, P(m, kBd).g);
+  e = gemm_wgrad(m, m->dYb, kInK, m->Hb, kW, P(m, kWd).g, kOut, kW, n, kW);
+  if (e == cudaSuccess) e = gemm(m, m->dYb, m->WdT, m->dH, np, kW, kInK, kW, nullptr, 0);
+  if (e == cudaSuccess)
+    k_back<false><<<cb, 32 * kCellWarps>>>(m->dH, nullptr, nullptr, nullptr,
+                                           reinterpret_cast<const uint8_t*>(m->gate[kLayers]), n,
+                                           np, nullptr, m->dPb, m->part);
+  for (int l = kLayers - 1; l >= 0 && e == cudaSuccess; --l) {
+    // dbl, dWl = dP^T Z, dZ = dP Wl, then dH_l and the dP below it
+    colsum(m, cb, kW, P(m, bl(l)).g);
+    e = gemm_wgrad(m, m->dPb, kW, m->Z[l], kZ, P(m, wl(l)).g, kW, kZ, n, kZ);
+    if (e == cudaSuccess) e = gemm(m, m->dPb, m->WlT[l], m->dZ, np, kZ, kW, kZ, nullptr, 0);
+    if (e != cudaSuccess) break;
+    std::swap(m->dH, m->dHn);  // dHn = dH_{l+1}
+    k_back<true><<<cb, 32 * kCellWarps>>>(m->dHn, m->dZ, m->ptr, m->nbr,
+                                          reinterpret_cast<const uint8_t*>(m->gate[l]), n, np,
+                                          l > 0 ? m->dH : nullptr, m->dPb, m->part);
+    e = cudaGetLastError();
+  }
+  // encoder: dbe, dWe = dP0^T X
+  if (e == cudaSuccess) {
+    colsum(m, cb, kW, P(m, kBe).g);
+    e = gemm_wgrad(m, m->dPb, kW, m->X, kInK, P(m, kWe).g, kW, kInK, n, kInK);
+  }
   if (e != cudaSuccess) return e;
   std::vector<double> part(nb);
   e = cudaMemcpy(part.data(), m->lpart, sizeof(double) * nb, cudaMemcpyDeviceToHost);
   double l = 0.0;
   for (double x : part) l += x;
   *loss = l / (double)(n * kOut);
-  // decoder: dWd = dY^T H3, dbd = colsum dY, dH3 = dY Wd.  dY as BF16:
-  // compact [n][4] (in dPb) for the transpose, and widened to a [np][64]
-  // A operand (columns >= 4 zero) for dH3
-  e = cudaMemset(m->dYb, 0, sizeof(__nv_bfloat16) * (size_t)np * kInK);
-  if (e != cudaSuccess) return e;
-  {
-    const size_t cnt = (size_t)n * kOut;
-    k_to_bf16<<<(unsigned)((cnt + 255) / 256), 256>>>(m->dY, m->dPb, cnt);
-    e = cudaMemcpy2DAsync(m->dYb, kInK * sizeof(__nv_bfloat16), m->dPb,
-                          kOut * sizeof(__nv_bfloat16), kOut * sizeof(__nv_bfloat16), n,
-                          cudaMemcpyDeviceToDevice, 0);
-    if (e != cudaSuccess) return e;
-  }
-  e = transpose(m->dPb, n, kOut, nk, m->tA);  // dY^T [4][nk]
-  if (e == cudaSuccess) e = transpose(m->Hb, n, kW, nk, m->tB);  // H3^T [128][nk]
-  if (e == cudaSuccess)
-    e = gemm_wgrad(m, m->tA, m->tB, P(m, kWd).g, kOut, kW, nk, kW);
-  if (e != cudaSuccess) return e;
-  colsum(m, m->dY, n, kOut, P(m, kBd).g);
-  // dH3 = dY . Wd : B operand = Wd^T [128][64] (K = 4 padded with zeros)
-  e = transpose(P(m, kWd).wb, kOut, kW, kInK, m->WdT);
-  if (e == cudaSuccess) e = gemm(m, m->dYb, m->WdT, m->dH, np, kW, kInK, kW, nullptr, 0, 0);
-  for (int l = kLayers - 1; l >= 0 && e == cudaSuccess; --l) {
-    // dP = dH_{l+1} (.) relu'
-    const size_t cnt = (size_t)np * kW;
-    k_relu_back<<<(unsigned)((cnt + 255) / 256), 256>>>(m->dH, m->H[l + 1], m->H[l], n, np,
-                                                         m->dP, m->dPb);
-    e = transpose(m->dPb, n, kW, nk, m->tA);            // dP^T [128][nk]
-    if (e == cudaSuccess) e = transpose(m->Z[l], n, kZ, nk, m->tB);  // Z^T [256][nk]
-    if (e == cudaSuccess)
-      e = gemm_wgrad(m, m->tA, m->tB, P(m, wl(l)).g, kW, kZ, nk, kZ);
-    if (e != cudaSuccess) break;
-    colsum(m, m->dP, n, kW, P(m, bl(l)).g);
-    // dZ = dP . Wl : B operand = Wl^T [256][128]
-    e = transpose(P(m, wl(l)).wb, kW, kZ, kW, m->WlT);
-    if (e == cudaSuccess) e = gemm(m, m->dPb, m->WlT, m->dZ, np, kZ, kW, kZ, nullptr, 0, 0);
-    if (e != cudaSuccess) break;
-    std::swap(m->dH, m->dHn);  // dHn = dH_{l+1}
-    k_agg_back<<<(n + kCellsPerBlock - 1) / kCellsPerBlock, 32 * kCellsPerBlock>>>(
-        m->dHn, m->dZ, m->ptr, m->nbr, n, m->dH);
-    e = cudaGetLastError();
-  }
-  if (e != cudaSuccess) return e;
-  // encoder: dP0 = dH0 (.) [H0 > 0]; dWe = dP0^T X; dbe
-  {
-    const size_t cnt = (size_t)np * kW;
-    k_relu_back<<<(unsigned)((cnt + 255) / 256), 256>>>(m->dH, m->H[0], nullptr, n, np, m->dP,
-                                                         m->dPb);
-    e = transpose(m->dPb, n, kW, nk, m->tA);
-    if (e == cudaSuccess) e = transpose(m->X, n, kInK, nk, m->tB);
-    if (e == cudaSuccess)
-      e = gemm_wgrad(m, m->tA, m->tB, P(m, kWe).g, kW, kInK, nk, kInK);
-    if (e == cudaSuccess) colsum(m, m->dP, n, kW, P(m, kBe).g);
-  }
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace
 namespace {
 
-// features [n][16] FP32 -> X [np][64] BF16 (zero padding)
+// features [n][16] FP32 -> X [np][64] BF16 (zero padding), eight columns a thread
 __global__ void k_features(const float* __restrict__ f, int n, int np,
                            __nv_bfloat16* __restrict__ x) {
+  constexpr int kPer = kInK / 8;
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= (size_t)np * kInK) return;
-  const int r = (int)(i / kInK), c = (int)(i % kInK);
-  x[i] = __float2bfloat16_rn((r < n && c < kIn) ? f[(size_t)r * kIn + c] : 0.f);
+  if (i >= (size_t)np * kPer) return;
+  const int r = (int)(i / kPer), c = (int)(i % kPer) * 8;
+  uint2 lo = make_uint2(0u, 0u), hi = lo;
+  if (r < n && c < kIn) {
+    const float4* p = reinterpret_cast<const float4*>(f + (size_t)r * kIn + c);
+    lo = bf16x4(p[0]);
+    hi = bf16x4(p[1]);
+  }
+  reinterpret_cast<uint4*>(x)[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
 }
 
 // xorshift64* uniform in [-1, 1)
@@ -669,7 +926,14 @@ mst_status mst_mpnn_create(uint64_t seed, mst_mpnn** out) {
   const int shapes[2 * (kLayers + 2)][2] = {{kW, kInK}, {1, kW}, {kW, kZ}, {1, kW}, {kW, kZ},
                                             {1, kW},   {kW, kZ}, {1, kW}, {kOut, kW}, {1, kOut}};
   uint64_t st = seed * 0x9E3779B97F4A7C15ull + 1;
+  const size_t all = (size_t)mst_mpnn_num_params();
   cudaError_t e = cudaSuccess;
+  for (float** q : {&m->w, &m->g, &m->m1, &m->v1}) {
+    if (e == cudaSuccess) e = cudaMalloc(q, all * 4);
+    if (e == cudaSuccess) e = cudaMemset(*q, 0, all * 4);
+  }
+  if (e == cudaSuccess) e = cudaMalloc(&m->wb, all * 2);
+  size_t off = 0;
   for (int i = 0; i < 2 * (kLayers + 2) && e == cudaSuccess; ++i) {
     MpnnParam& p = m->W[i];
     p.rows = shapes[i][0];
@@ -686,16 +950,15 @@ mst_status mst_mpnn_create(uint64_t seed, mst_mpnn** out) {
     }
     std::vector<__nv_bfloat16> wb(n);
     for (size_t k = 0; k < n; ++k) wb[k] = __float2bfloat16_rn(w[k]);
-    e = cudaMalloc(&p.w, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&p.g, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&p.m, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&p.v, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&p.wb, n * 2);
-    if (e == cudaSuccess) e = cudaMemcpy(p.w, w.data(), n * 4, cudaMemcpyHostToDevice);
+    // (every tensor but the last is a multiple of 8 values: 16-byte operands)
+    p.w = m->w + off;
+    p.g = m->g + off;
+    p.m = m->m1 + off;
+    p.v = m->v1 + off;
+    p.wb = m->wb + off;
+    off += n;
+    e = cudaMemcpy(p.w, w.data(), n * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(p.wb, wb.data(), n * 2, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(p.g, 0, n * 4);
-    if (e == cudaSuccess) e = cudaMemset(p.m, 0, n * 4);
-    if (e == cudaSuccess) e = cudaMemset(p.v, 0, n * 4);
   }
   if (e != cudaSuccess) {
     mst_mpnn_destroy(m);
@@ -708,13 +971,8 @@ mst_status mst_mpnn_create(uint64_t seed, mst_mpnn** out) {
 mst_status mst_mpnn_destroy(mst_mpnn* m) {
   if (!m) return MST_OK;
   cudaDeviceSynchronize();
-  for (auto& p : m->W) {
-    cudaFree(p.w);
-    cudaFree(p.g);
-    cudaFree(p.m);
-    cudaFree(p.v);
-    cudaFree(p.wb);
-  }
+  for (float* p : {m->w, m->g, m->m1, m->v1}) cudaFree(p);
+  cudaFree(m->wb);
   for (void* p : m->bufs) cudaFree(p);
   cudaFree(m->nbr);
   for (auto& r : m->recs) {
@@ -760,10 +1018,11 @@ mst_status mst_mpnn_set_graph(mst_mpnn* m, int n, const float* features, const i
   if (!m || n <= 0 || !features || !nbr_ptr || !nbr)
     return mst_internal_fail(MST_EINVAL, "bad graph arguments");
   const int n_nbr = nbr_ptr[n];
-  for (int i = 0; i < n; ++i)
-    if (nbr_ptr[i + 1] < nbr_ptr[i]) return mst_internal_fail(MST_EINVAL, "nbr_ptr not ascending");
-  for (int i = 0; i < n_nbr; ++i)
-    if (nbr[i] < 0 || nbr[i] >= n) return mst_internal_fail(MST_EINVAL, "neighbour id out of range");
+  int bad = 0;  // (no early exit: the loops vectorise)
+  for (int i = 0; i < n; ++i) bad |= nbr_ptr[i + 1] < nbr_ptr[i];
+  if (bad) return mst_internal_fail(MST_EINVAL, "nbr_ptr not ascending");
+  for (int i = 0; i < n_nbr; ++i) bad |= (unsigned)nbr[i] >= (unsigned)n;
+  if (bad) return mst_internal_fail(MST_EINVAL, "neighbour id out of range");
   cudaError_t e = ensure_cap(m, n, std::max(n_nbr, 1));
   float* df = m->feat;
   if (e == cudaSuccess)
@@ -774,7 +1033,7 @@ mst_status mst_mpnn_set_graph(mst_mpnn* m, int n, const float* features, const i
     e = cudaMemcpy(m->nbr, nbr, sizeof(int) * (size_t)n_nbr, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
     const int np = pad128(n);
-    const size_t cnt = (size_t)np * kInK;
+    const size_t cnt = (size_t)np * (kInK / 8);
     k_features<<<(unsigned)((cnt + 255) / 256), 256>>>(df, n, np, m->X);
     e = cudaGetLastError();
   }
@@ -824,13 +1083,9 @@ mst_status mst_mpnn_backward(mst_mpnn* m, double* loss) {
 // W1, b1, W2, b2, Wd, bd, each row-major [outputs][inputs]
 mst_status mst_mpnn_get(mst_mpnn* m, int which, float* out) {
   if (!m || !out) return mst_internal_fail(MST_EINVAL, "NULL argument");
-  size_t off = 0;
-  for (auto& p : m->W) {
-    const size_t n = (size_t)p.size();
-    cudaError_t e = cudaMemcpy(out + off, which ? p.g : p.w, n * 4, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return mst_internal_fail(MST_ECUDA, cudaGetErrorString(e));
-    off += n;
-  }
+  const cudaError_t e = cudaMemcpy(out, which ? m->g : m->w, sizeof(float) * mst_mpnn_num_params(),
+                                   cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return mst_internal_fail(MST_ECUDA, cudaGetErrorString(e));
   return MST_OK;
 }
 
@@ -854,10 +1109,19 @@ mst_status mst_mpnn_adam_step(mst_mpnn* m, float lr) {
   m->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-  for (auto& p : m->W) {
-    const int n = p.size();
-    k_adam<<<(n + 255) / 256, 256>>>(p.w, p.g, p.m, p.v, n, lr, b1, b2, c1, c2, p.wb);
+  AdamTensors t;
+  int most = 0;
+  for (int i = 0; i < 2 * (kLayers + 2); ++i) {
+    const MpnnParam& p = m->W[i];
+    t.w[i] = p.w;
+    t.m[i] = p.m;
+    t.v[i] = p.v;
+    t.g[i] = p.g;
+    t.wb[i] = p.wb;
+    t.n[i] = p.size();
+    most = std::max(most, p.size());
   }
+  k_adam<<<dim3((most + 255) / 256, 2 * (kLayers + 2)), 256>>>(t, lr, b1, b2, c1, c2);
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return mst_internal_fail(MST_ECUDA, cudaGetErrorString(e));
   return MST_OK;
@@ -918,8 +1182,7 @@ mst_status mst_tc_gemm_check(const uint16_t* A, const uint16_t* B, const float* 
         g.k_chunk = layout;
         e = mst::tc::gemm(g, 0);
         const size_t mn = (size_t)M * N;
-        if (e == cudaSuccess)
-          mst::tc::k_reduce_splits<<<(unsigned)((mn + 255) / 256), 256>>>(part, splits, mn, dC);
+        if (e == cudaSuccess) e = mst::tc::reduce_splits(part, splits, mn, dC);
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         cudaFree(part);
       }

@@ -4,7 +4,8 @@
 // project.
 //
 //   C[M, N] (FP32) = A[M, K] (BF16, row-major) . B[N, K]^T (BF16, row-major)
-//                    (+ bias[N]) (ReLU) ; optional BF16 copy of C
+//                    (+ bias[N]) (ReLU) (+ Cin) ; optional BF16 copy of C and
+//                    one bit per value, result > Cin
 //
 // One CTA of 128 threads per 128 x BN tile (BN = 128, or 16 when N <= 16).  K is walked in
 // 64-wide tiles through two shared-memory stages filled with cp.async in
@@ -59,9 +60,10 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return d;                // base offset 0, layout type 0 (no swizzle)
 }
 
-// instruction descriptor of kind::f16: BF16 x BF16 -> FP32, both K-major
-__host__ __device__ constexpr uint32_t instr_desc(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+// instruction descriptor of kind::f16: BF16 x BF16 -> FP32, both K-major or
+// (rows) both with M / N contiguous
+__host__ __device__ constexpr uint32_t instr_desc(int m, int n, bool rows = false) {
+  return (rows ? 3u << 15 : 0u) | (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(m >> 4) << 24);
 }
 
@@ -132,11 +134,12 @@ struct GemmArgs {
   const __nv_bfloat16* A;  // [M][K]
   const __nv_bfloat16* B;  // [N][K]
   float* C;                // [M][ldc] or nullptr
-  __nv_bfloat16* Cb;       // [M][ldcb] BF16 copy or nullptr
+  const float* Cin;        // [M][ldc] added to the result (not C itself) or nullptr
+  __nv_bfloat16* Cb;       // [M][ldcb] BF16 copy of C or nullptr
+  uint16_t* gate;          // [M][N / 16] bits: C > Cin (> 0 without Cin); N in 16s; or nullptr
   const float* bias;       // [N] or nullptr
   int M, N, K, ldc, ldcb;
   int relu;
-  int accumulate_c;        // C += result (FP32 output only)
   uint32_t lbo, sbo;       // descriptor strides (bytes)
   int* err;                // set on a timed-out wait
   unsigned spin_limit;     // polls of each main-loop wait (0: give up at once)
@@ -147,35 +150,41 @@ struct GemmArgs {
 };
 
 // Epilogue of 16 accumulator columns of one row: bias, ReLU, the residual
-// add (accumulate_c) and the stores of C and its BF16 copy (16-byte stores
-// where the row allows them; vc / vb: C / Cb rows 16-byte aligned).  prev:
-// the 16 values of C already loaded for the residual add (or nullptr).
+// add and the stores of C, its BF16 copy and the gate bits (16-byte stores
+// where the row allows them; vc / vb: C and Cin / Cb rows 16-byte aligned).
 __device__ __forceinline__ void store16(const GemmArgs& g, bool split, float* Cout, int row,
-                                        int n0, int c0, float v[16], bool vc, bool vb,
-                                        const float4* prev = nullptr) {
+                                        int n0, int c0, float v[16], bool vc, bool vb) {
   if (row < g.M && vc && vb && n0 + c0 + 16 <= g.N) {
     const int col0 = n0 + c0;
+    unsigned bits = 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       float x = v[i];
       if (!split && g.bias) x += g.bias[col0 + i];
       if (!split && g.relu) x = fmaxf(x, 0.f);
       v[i] = x;
+      if (x > 0.f) bits |= 1u << i;
     }
+    if (g.Cin) {
+      const float4* p = reinterpret_cast<const float4*>(g.Cin + (size_t)row * g.ldc + col0);
+      bits = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 w4 = p[j];
+        const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          v[4 * j + k] += w[k];
+          if (v[4 * j + k] > w[k]) bits |= 1u << (4 * j + k);
+        }
+      }
+    }
+    if (g.gate) g.gate[(size_t)row * (g.N / 16) + col0 / 16] = (uint16_t)bits;
     if (Cout) {
       float4* p = reinterpret_cast<float4*>(Cout + (size_t)row * g.ldc + col0);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float4 o = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        if (!split && g.accumulate_c) {
-          const float4 w = prev ? prev[j] : p[j];
-          o.x += w.x;
-          o.y += w.y;
-          o.z += w.z;
-          o.w += w.w;
-        }
-        p[j] = o;
-      }
+      for (int j = 0; j < 4; ++j)
+        p[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     }
     if (g.Cb) {
       uint4* pb = reinterpret_cast<uint4*>(g.Cb + (size_t)row * g.ldcb + col0);
@@ -191,6 +200,7 @@ __device__ __forceinline__ void store16(const GemmArgs& g, bool split, float* Co
       }
     }
   } else if (row < g.M) {
+    unsigned bits = 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int col = n0 + c0 + i;
@@ -198,13 +208,14 @@ __device__ __forceinline__ void store16(const GemmArgs& g, bool split, float* Co
       if (!split && g.bias && col < g.N) x += g.bias[col];
       if (!split && g.relu) x = fmaxf(x, 0.f);
       if (col < g.N) {
-        if (Cout) {
-          float* p = Cout + (size_t)row * g.ldc + col;
-          *p = (!split && g.accumulate_c) ? *p + x : x;
-        }
+        const float w = g.Cin ? g.Cin[(size_t)row * g.ldc + col] : 0.f;
+        if (g.Cin) x += w;
+        if (x > w) bits |= 1u << i;
+        if (Cout) Cout[(size_t)row * g.ldc + col] = x;
         if (g.Cb) g.Cb[(size_t)row * g.ldcb + col] = __float2bfloat16_rn(x);
       }
     }
+    if (g.gate && n0 + c0 < g.N) g.gate[(size_t)row * (g.N / 16) + (n0 + c0) / 16] = (uint16_t)bits;
   }
 }
 
@@ -327,7 +338,8 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16(const GemmArgs g) {
   if (ok) {
     const int row = m0 + warp * 32 + lane;
     // 16-byte stores where the rows allow them (4 floats of C, 8 BF16 of Cb)
-    const bool vc = !Cout || ((g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(Cout) & 15) == 0);
+    const bool vc = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(Cout) & 15) == 0 &&
+                    (reinterpret_cast<uintptr_t>(g.Cin) & 15) == 0;
     const bool vb = !g.Cb || ((g.ldcb & 7) == 0 && (reinterpret_cast<uintptr_t>(g.Cb) & 15) == 0);
     for (int c0 = 0; c0 < kBN; c0 += 16) {
       float v[16];

@@ -2,7 +2,8 @@
 // network's large-M layers (M = cells, N <= 256, K <= 256):
 //
 //   C[M, N] (FP32) = A[M, K] (BF16, row-major) . B[N, K]^T (BF16, row-major)
-//                    (+ bias[N]) (ReLU) (+ C) ; optional BF16 copy of C
+//                    (+ bias[N]) (ReLU) (+ Cin) ; optional BF16 copy of C and
+//                    one bit per value, C > Cin
 //
 // Each CTA keeps one 128-wide column block of B (all of K) resident in shared
 // memory and walks its share of the 128-row tiles of A.  Warp 0 (one lane)
@@ -11,11 +12,14 @@
 // kTmaStages stages; warp 1 (one lane) issues tcgen05.mma (kind::f16, BF16 x
 // BF16 -> FP32) into one of two tensor-memory accumulators and commits each
 // stage back to the copier; warps 2-9 read the other accumulator with
-// tcgen05.ld and store the tile (each warp 32 rows x 64 columns in two
-// loads, released to the MMA thread once both are in registers; whole
-// 32-byte sectors per store; the C values of a residual add loaded before the
-// accumulator is waited for), so a tile's epilogue overlaps the next
-// tile's copies and products.  Every wait is bounded (GemmArgs.spin_limit
+// tcgen05.ld (each warp 32 rows x 64 columns in two loads, released to the MMA
+// thread once both are in registers) and store it through swizzled 32 x 32
+// staging tiles with TMA; the values of a residual add arrive in the same
+// tiles, asked for before the accumulator is waited for.  So a tile's epilogue
+// overlaps the next tile's copies and products, and memory sees whole lines: a
+// thread storing its own row 32 bytes at a time took 73 us for C[168704][256]
+// with K = 128 (215 MB) and 65 us for N = 128, K = 256 with the residual (260
+// MB); this takes 42 and 45 us.  Every wait is bounded (GemmArgs.spin_limit
 // polls): on timeout a role flags the CTA and the error word, the others
 // stop, the copier waits for its copies in flight and the MMA thread for its
 // products (full limit), and the tensor memory is freed before the CTA ends.
@@ -27,21 +31,19 @@
 namespace mst {
 namespace tc {
 
-constexpr int kTmaStages = 6;                // A ring
+constexpr int kTmaStages = 5;                // A ring
 constexpr int kTmaEpiWarps = 8;              // 4 row quarters x 2 column halves
 constexpr int kTmaThreads = 64 + 32 * kTmaEpiWarps;  // copier, MMA, epilogue
 constexpr int kTmaTile = kBM * kBK * 2;      // one 128-row x 64-K BF16 tile: 16 KB
 constexpr int kTmaMaxKT = 4;                 // K <= 256
-// dynamic shared memory: B (kt tiles) + the A ring + barriers, from a
-// 1024-byte-aligned base (the 128-byte swizzle repeats every 1024 bytes; the
-// kernel checks the base and reports a misaligned one instead of copying);
-// at least 80 KB so that at most two CTAs share an SM (two double
-// accumulators of 128 columns fill its 512 TMEM columns).  The epilogue's
-// registers (the C values of the residual add held across the wait) keep
-// it to one CTA per SM in practice; the launch asks the occupancy.
+// an epilogue warp's staging: two 32-row x 32-column FP32 tiles
+constexpr int kStageTile = 32 * 32 * 4;
+// dynamic shared memory: B (kt tiles) + the A ring + the epilogue's staging +
+// barriers, from a 1024-byte-aligned base (the 128-byte swizzle repeats every
+// 1024 bytes; the kernel checks the base and reports a misaligned one instead of
+// copying): 210 KB at K = 256, one CTA per SM.
 __host__ __device__ constexpr int tma_smem_bytes(int kt) {
-  return ((kt + kTmaStages) * kTmaTile + 256) < 80 * 1024 ? 80 * 1024
-                                                          : (kt + kTmaStages) * kTmaTile + 256;
+  return (kt + kTmaStages) * kTmaTile + 2 * kTmaEpiWarps * kStageTile + 512;
 }
 
 // bounded wait that also gives up once another role has flagged the CTA
@@ -63,6 +65,18 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
   d |= (uint64_t)(1024 >> 4) << 32;   // stride byte offset: 8 rows x 128 B
   d |= (uint64_t)1 << 46;             // descriptor version of this architecture
   d |= (uint64_t)2 << 61;             // layout: 128-byte swizzle
+  return d;
+}
+
+// the same with M / N contiguous (rows of 64 columns = 128 bytes): 8-row groups
+// 1024 bytes apart, 64-column blocks half a tile apart
+__device__ __forceinline__ uint64_t smem_desc_sw128_rows(uint32_t addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr >> 4) & 0x3FFF);
+  d |= (uint64_t)((kTmaTile / 2) >> 4) << 16;  // leading byte offset: 64 columns
+  d |= (uint64_t)(1024 >> 4) << 32;            // stride byte offset: 8 rows
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
   return d;
 }
 
@@ -102,18 +116,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32]) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 32-byte (one sector) global load / store of 8 floats; the address is
-// 32-byte aligned
-__device__ __forceinline__ void ld8(const float* p, float x[8]) {
-  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]),
-                 "=f"(x[6]), "=f"(x[7])
-               : "l"(p));
+// 2D tiled copy shared -> global in the issuing thread's bulk group
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];\n\t"
+      "cp.async.bulk.commit_group;" ::"l"(reinterpret_cast<uint64_t>(map)),
+      "r"(x), "r"(y), "r"(src)
+      : "memory");
 }
-__device__ __forceinline__ void st8(float* p, const float x[8]) {
-  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(x[0]),
-               "f"(x[1]), "f"(x[2]), "f"(x[3]), "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7])
-               : "memory");
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_wait() {
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 struct TmaGemm {
@@ -121,24 +136,28 @@ struct TmaGemm {
   int kt;        // K / 64
   int n_ntiles;  // 128-wide column blocks of N
   int m_tiles;   // 128-row tiles of M
+  int staged;    // C and Cin through shared memory and TMA
 };
 
 __global__ void __launch_bounds__(kTmaThreads, 1)
     k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+               const __grid_constant__ CUtensorMap mapC, const __grid_constant__ CUtensorMap mapI,
                const TmaGemm t) {
   constexpr int S = kTmaStages;
   extern __shared__ __align__(1024) uint8_t smem[];
   const GemmArgs& g = t.g;
   uint8_t* sB = smem;
   uint8_t* sA = smem + t.kt * kTmaTile;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sA + S * kTmaTile);
+  uint8_t* sC = sA + S * kTmaTile;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sC + 2 * kTmaEpiWarps * kStageTile);
   uint64_t* full = bars;             // [S] a stage's copy landed
   uint64_t* empty = bars + S;        // [S] a stage's products are done
   uint64_t* bfull = bars + 2 * S;    // B landed
   uint64_t* accf = bars + 2 * S + 1; // [2] an accumulator holds a finished tile
   uint64_t* acce = bars + 2 * S + 3; // [2] an accumulator was read out
   uint64_t* drain = bars + 2 * S + 5;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2 * S + 6);
+  uint64_t* cinf = bars + 2 * S + 6; // [2 kTmaEpiWarps] a staged Cin tile landed
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(cinf + 2 * kTmaEpiWarps);
   volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (blockIdx.x % t.n_ntiles) * kBN;
@@ -162,6 +181,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
       mbar_init(&acce[b], kTmaEpiWarps);
     }
     mbar_init(drain, 1);
+    for (int q = 0; q < 2 * kTmaEpiWarps; ++q) mbar_init(&cinf[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     // the swizzled layout needs a 1024-byte-aligned base: otherwise report
     // it and copy nothing
@@ -264,33 +284,42 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
     }
   } else {
     // epilogue warps 2-9: warp w reads TMEM lanes 32 (w % 4).. (its rows),
-    // columns [64 h, 64 h + 64) with h = (w - 2) / 4
+    // columns [64 h, 64 h + 64) with h = (w - 2) / 4, 32 at a time
     const int q = warp & 3, h = (warp - 2) >> 2;
-    const int cb = h * (kBN / 2);
-    const bool vc = !g.C || ((g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0);
+    const int col0 = n0 + h * (kBN / 2);
+    const int halves = min(2, max(0, (g.N - col0 + 31) / 32));  // with columns inside N
+    uint8_t* stage = sC + 2 * (warp - 2) * kStageTile;
+    uint64_t* cin = cinf + 2 * (warp - 2);
+    const uintptr_t cp = reinterpret_cast<uintptr_t>(g.C) | reinterpret_cast<uintptr_t>(g.Cin);
+    const bool vc = (g.ldc & 3) == 0 && (cp & 15) == 0;
     const bool vb = !g.Cb || ((g.ldcb & 7) == 0 && (reinterpret_cast<uintptr_t>(g.Cb) & 15) == 0);
-    // whole sectors: C rows 32-byte aligned
-    const bool v32 = !g.C || ((g.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 31) == 0);
+    const bool read_cin = t.staged && g.Cin && halves > 0 && !*abort;
     int i = 0;
     for (int m = m_first; m < t.m_tiles; m += m_step, ++i) {
       const int b = i & 1;
       const uint32_t aph = (uint32_t)(i >> 1) & 1;
-      const int row = m * kBM + q * 32 + lane;
-      // warp-uniform (the TMEM loads below are .sync.aligned): every row of
-      // the warp inside M, all 64 columns inside N, aligned rows
-      const bool fast =
-          __all_sync(0xffffffffu, row < g.M && n0 + cb + kBN / 2 <= g.N && v32 && vb) != 0;
-      // the residual add's C values do not depend on the products: their
-      // loads are in flight while the accumulator is still being formed
-      const bool pre = fast && g.accumulate_c && g.C;
-      float prev[kBN / 2];
-      if (pre) {
-        const float* p = g.C + (size_t)row * g.ldc + n0 + cb;
-#pragma unroll
-        for (int j = 0; j < kBN / 16; ++j) ld8(p + 8 * j, &prev[8 * j]);
+      const int row0 = m * kBM + q * 32, row = row0 + lane;
+      // the residual add's values do not depend on the products: they are
+      // copied into the staging tiles, once the last tile's stores have read
+      // these, while the accumulator is still being formed
+      __syncwarp();  // (and the last tile's values were read by every lane)
+      if (lane == 0) {
+        bulk_wait_read();
+        if (read_cin)
+          for (int k = 0; k < halves; ++k) {
+            mbar_expect_tx(&cin[k], kStageTile);
+            tma_load_2d(smem_u32(stage + k * kStageTile), &mapI, col0 + 32 * k, row0, &cin[k]);
+          }
       }
+      __syncwarp();
       int go = 0;
-      if (lane == 0) go = mbar_wait_or_abort(&accf[b], aph, lim, abort) ? 1 : 0;
+      if (lane == 0) {
+        go = mbar_wait_or_abort(&accf[b], aph, lim, abort) ? 1 : 0;
+        if (read_cin)
+          for (int k = 0; k < halves; ++k)
+            if (!mbar_wait(&cin[k], (uint32_t)i & 1, kSpinLimit)) go = 0;
+      }
+      __syncwarp();
       go = __shfl_sync(0xffffffffu, go, 0);
       if (!go) {
         if (lane == 0) {
@@ -300,62 +329,76 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kBN + cb);
-      if (fast) {
-        const int col0 = n0 + cb;
+      const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kBN + col0 - n0);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          float v[32];
-          tmem_ld32(acc + 32 * half, v);
-          if (half == 1) {
-            // the accumulator is in registers: the MMA thread may reuse it
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acce[b]);
+      for (int half = 0; half < 2; ++half) {
+        float v[32];
+        if (half < halves) tmem_ld32(acc + 32 * half, v);
+        if (half == 1) {
+          // the accumulator is in registers: the MMA thread may reuse it
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acce[b]);
+        }
+        if (half >= halves) continue;
+        const int c0 = col0 + 32 * half;
+        if (!t.staged) {
+          store16(g, false, g.C, row, n0, c0 - n0, &v[0], vc, vb);
+          store16(g, false, g.C, row, n0, c0 - n0 + 16, &v[16], vc, vb);
+          continue;
+        }
+        // this thread's row of the staging tile: 16-byte chunk j at j ^ (row % 8)
+        float4* srow = reinterpret_cast<float4*>(stage + half * kStageTile + lane * 128);
+        unsigned bits = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float4* s4 = srow + (j ^ (lane & 7));
+          float w[4] = {0.f, 0.f, 0.f, 0.f}, x[4];
+          if (g.Cin) {
+            const float4 p = *s4;
+            w[0] = p.x;
+            w[1] = p.y;
+            w[2] = p.z;
+            w[3] = p.w;
           }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            float y = v[4 * j + k];
+            if (g.bias && c0 + 4 * j + k < g.N) y += __ldg(g.bias + c0 + 4 * j + k);
+            if (g.relu) y = fmaxf(y, 0.f);
+            x[k] = g.Cin ? y + w[k] : y;
+            if (x[k] > w[k]) bits |= 1u << (4 * j + k);
+            v[4 * j + k] = x[k];
+          }
+          if (g.C) *s4 = make_float4(x[0], x[1], x[2], x[3]);
+        }
+        if (g.C) {
+          // (rows and columns beyond C are clipped by the copy)
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0 && row0 < g.M)
+            tma_store_2d(&mapC, c0, row0, smem_u32(stage + half * kStageTile));
+        }
+        if (g.gate && row < g.M)
+          *reinterpret_cast<uint32_t*>(g.gate + (size_t)row * (g.N / 16) + c0 / 16) = bits;
+        if (g.Cb && row < g.M) {
+          uint4* pb = reinterpret_cast<uint4*>(g.Cb + (size_t)row * g.ldcb + c0);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const int c = 32 * half + 8 * j;  // column within the warp's 64
-            float x[8];
+            uint32_t w[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              float y = v[8 * j + k];
-              if (g.bias) y += __ldg(g.bias + col0 + c + k);
-              if (g.relu) y = fmaxf(y, 0.f);
-              x[k] = y;
+            for (int k = 0; k < 4; ++k) {
+              const __nv_bfloat162 b2 =
+                  __floats2bfloat162_rn(v[8 * j + 2 * k], v[8 * j + 2 * k + 1]);
+              w[k] = *reinterpret_cast<const uint32_t*>(&b2);
             }
-            if (g.C) {
-              float o[8];
-#pragma unroll
-              for (int k = 0; k < 8; ++k) o[k] = pre ? x[k] + prev[c + k] : x[k];
-              st8(g.C + (size_t)row * g.ldc + col0 + c, o);
-            }
-            if (g.Cb) {
-              uint32_t w[4];
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const __nv_bfloat162 b2 = __floats2bfloat162_rn(x[2 * k], x[2 * k + 1]);
-                w[k] = *reinterpret_cast<const uint32_t*>(&b2);
-              }
-              *reinterpret_cast<uint4*>(g.Cb + (size_t)row * g.ldcb + col0 + c) =
-                  make_uint4(w[0], w[1], w[2], w[3]);
-            }
+            pb[j] = make_uint4(w[0], w[1], w[2], w[3]);
           }
         }
-      } else {
-        // ragged columns, rows past M or unaligned rows: 16 at a time
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          float v[32];
-          tmem_ld32(acc + 32 * half, v);
-          store16(g, false, g.C, row, n0, cb + 32 * half, &v[0], vc, vb);
-          store16(g, false, g.C, row, n0, cb + 32 * half + 16, &v[16], vc, vb);
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acce[b]);
       }
     }
+    // the staging tiles are read before the CTA ends
+    if (lane == 0) bulk_wait();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -364,7 +407,13 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
                  "r"(2 * kBN));
 }
 
-// Split-K variant for the weight gradients (M, N <= 256, K = the cells):
+// Split-K variant for the weight gradients (M, N <= 256, K = the cells).
+// ROWS: the operands lie as [K][columns of A] and [K][columns of B] -- one row
+// per cell, as the layers' kernels write them, so that no transposed copy is
+// made: a tile is two 64-column boxes (8 KB) of 64 rows, read with M / N
+// contiguous (64 columns x 8 rows per 1024-byte swizzle atom, the next 8 rows
+// 1024 bytes on, the next 64 columns 8192); rows past K and columns past an
+// operand's width arrive as zeros.  Otherwise [M][K] and [N][K].
 // CTA (m, n, z) forms the 128x128 partial product of its K chunk and stores
 // it to C + z * M * ldc (no bias / ReLU; the caller adds the chunks in
 // order).  Warp 0 copies A and B tiles (128 x 64 each) with
@@ -375,6 +424,7 @@ constexpr int kSplitStages = 3;
 constexpr int kSplitThreads = 192;
 __host__ __device__ constexpr int split_smem_bytes() { return kSplitStages * 2 * kTmaTile + 256; }
 
+template <bool ROWS>
 __global__ void __launch_bounds__(kSplitThreads)
     k_gemm_tma_split(const __grid_constant__ CUtensorMap mapA,
                      const __grid_constant__ CUtensorMap mapB, const GemmArgs g) {
@@ -432,8 +482,17 @@ __global__ void __launch_bounds__(kSplitThreads)
           break;
         }
         mbar_expect_tx(&full[st], (uint32_t)(2 * kTmaTile));
-        tma_load_2d(smem_u32(sA + st * kTmaTile), &mapA, kbase + k * kBK, m0, &full[st]);
-        tma_load_2d(smem_u32(sB + st * kTmaTile), &mapB, kbase + k * kBK, n0, &full[st]);
+        const uint32_t a0 = smem_u32(sA + st * kTmaTile), b0 = smem_u32(sB + st * kTmaTile);
+        const int k0 = kbase + k * kBK;
+        if (ROWS) {
+          tma_load_2d(a0, &mapA, m0, k0, &full[st]);
+          tma_load_2d(a0 + kTmaTile / 2, &mapA, m0 + 64, k0, &full[st]);
+          tma_load_2d(b0, &mapB, n0, k0, &full[st]);
+          tma_load_2d(b0 + kTmaTile / 2, &mapB, n0 + 64, k0, &full[st]);
+        } else {
+          tma_load_2d(a0, &mapA, k0, m0, &full[st]);
+          tma_load_2d(b0, &mapB, k0, n0, &full[st]);
+        }
         used[st] = true;
         last_ph[st] = ph;
         if (++st == S) {
@@ -450,7 +509,7 @@ __global__ void __launch_bounds__(kSplitThreads)
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = instr_desc(kBM, kBN);
+      const uint32_t idesc = instr_desc(kBM, kBN, ROWS);
       bool ok = !*abort, any = false;
       int st = 0;
       uint32_t ph = 0;
@@ -463,8 +522,9 @@ __global__ void __launch_bounds__(kSplitThreads)
         const uint32_t a0 = smem_u32(sA + st * kTmaTile), b0 = smem_u32(sB + st * kTmaTile);
 #pragma unroll
         for (int kk = 0; kk < kBK / 16; ++kk)
-          mma_bf16(tmem, smem_desc_sw128(a0 + kk * 32), smem_desc_sw128(b0 + kk * 32), idesc,
-                   (k > 0 || kk > 0) ? 1u : 0u);
+          mma_bf16(tmem, ROWS ? smem_desc_sw128_rows(a0 + kk * 2048) : smem_desc_sw128(a0 + kk * 32),
+                   ROWS ? smem_desc_sw128_rows(b0 + kk * 2048) : smem_desc_sw128(b0 + kk * 32),
+                   idesc, (k > 0 || kk > 0) ? 1u : 0u);
         any = true;
         mma_commit(&empty[st]);
         if (++st == S) {
