@@ -21,7 +21,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <numeric>
 #include <string>
 #include <vector>
 
@@ -229,17 +228,42 @@ constexpr int kLuMaxCta = 16;
 
 // Rows of a sweep in level order, or of a product in row order.  The first four
 // entries stand at fixed places, so that all of a row's loads can be issued at
-// once; rows with more find the rest at meta.z.  A sweep's weight is
-// L (1 / D[column]).
+// once; rows with more find the rest in the matrix itself, from meta.z.  A
+// sweep's weight is L (1 / D[column]): the quotient and product the reference
+// forms at every use.
 struct LuRows {
   const int* lev;
-  const int4* meta;  // row, entries, first of the entries past the fourth, -
+  const int4* meta;  // row, entries, the fifth's place in col / val, -
   const int4* col4;
   const double4_32a* w4;
   const int* col;
-  const double* w;
+  const double *val, *rD;  // rD = 1 / D, or null: a product
   int n_levels;
 };
+// lays them out (rows: the order, or null)
+__global__ void k_lu_rows(int dim, const int* __restrict__ rows, const int* __restrict__ ptr,
+                          const int* __restrict__ col, const double* __restrict__ val,
+                          const double* __restrict__ rD, int4* __restrict__ meta,
+                          int4* __restrict__ col4, double4_32a* __restrict__ w4) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= dim) return;
+  const int r = rows ? rows[i] : i, k0 = ptr[r], n = ptr[r + 1] - k0;
+  int c[4];
+  double w[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    c[k] = k < n ? col[k0 + k] : 0;
+    w[k] = k < n ? (rD ? val[k0 + k] * rD[c[k]] : val[k0 + k]) : 0.;
+  }
+  meta[i] = make_int4(r, n, k0 + 4, 0);
+  col4[i] = make_int4(c[0], c[1], c[2], c[3]);
+  w4[i] = double4_32a{w[0], w[1], w[2], w[3]};
+}
+__global__ void k_lu_reciprocal(int dim, const double* __restrict__ D, double* __restrict__ rD) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < dim) rD[r] = 1. / D[r];
+}
+
 struct LuSolve {
   int dim, gs, shift, rows;  // 2^shift CTAs, rows of the vector in each
   LuRows up, lo, fwd, bwd;
@@ -283,7 +307,10 @@ __device__ __forceinline__ double lu_row(const LuRow& r, const LuRows& s, const 
   if (n > 1) add(r.w.y * v1);
   if (n > 2) add(r.w.z * v2);
   if (n > 3) add(r.w.w * v3);
-  for (int k = 0; k < n - 4; ++k) add(s.w[r.meta.z + k] * v[s.col[r.meta.z + k]]);
+  for (int k = r.meta.z; k < r.meta.z + n - 4; ++k) {
+    const int c = s.col[k];
+    add((s.rD ? s.val[k] * s.rD[c] : s.val[k]) * v[c]);
+  }
   return acc;
 }
 
@@ -428,6 +455,7 @@ struct mst_lu {
   std::vector<void*> allocs;
   // the one-launch solve of scalar systems (cluster = 0: not used)
   int cluster = 0;
+  int *fwd_lev = nullptr, *bwd_lev = nullptr;
   LuRows r_up{}, r_lo{}, r_fwd{}, r_bwd{};
   double* rD = nullptr;
   unsigned* change = nullptr;
@@ -449,18 +477,28 @@ mst_status lu_fail(mst_status s, const std::string& m) { return mst_internal_fai
 // (ascending or descending) and then insertion order
 Csr build_rows(int dim, int n, const int* rows, const int* cols, const double* vals, int B,
                bool lower, bool desc) {
-  std::vector<int> idx;
-  for (int i = 0; i < n; ++i)
-    if (lower ? rows[i] > cols[i] : rows[i] < cols[i]) idx.push_back(i);
-  std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) {
-    if (rows[a] != rows[b]) return rows[a] < rows[b];
-    if (cols[a] != cols[b]) return desc ? cols[a] > cols[b] : cols[a] < cols[b];
-    return a < b;
-  });
   Csr c;
   c.ptr.assign(dim + 1, 0);
-  for (int i : idx) c.ptr[rows[i] + 1]++;
+  auto mine = [&](int i) { return lower ? rows[i] > cols[i] : rows[i] < cols[i]; };
+  for (int i = 0; i < n; ++i)
+    if (mine(i)) c.ptr[rows[i] + 1]++;
   for (int r = 0; r < dim; ++r) c.ptr[r + 1] += c.ptr[r];
+  // entries into their rows in insertion order, then a stable sort within the row
+  std::vector<int> idx(c.ptr[dim]), fill(c.ptr.begin(), c.ptr.end() - 1);
+  for (int i = 0; i < n; ++i)
+    if (mine(i)) idx[fill[rows[i]]++] = i;
+  auto before = [&](int x, int y) { return desc ? cols[x] > cols[y] : cols[x] < cols[y]; };
+  for (int r = 0; r < dim; ++r) {
+    const int a = c.ptr[r], e = c.ptr[r + 1];
+    if (e - a > 16) {
+      std::stable_sort(idx.begin() + a, idx.begin() + e, before);
+      continue;
+    }
+    for (int k = a + 1; k < e; ++k)
+      for (int q = k; q > a && before(idx[q], idx[q - 1]); --q) std::swap(idx[q - 1], idx[q]);
+  }
+  c.col.reserve(idx.size());
+  c.val.reserve(idx.size() * B * B);
   for (int i : idx) {
     c.col.push_back(cols[i]);
     for (int k = 0; k < B * B; ++k) c.val.push_back(vals[(size_t)B * B * i + k]);
@@ -495,46 +533,58 @@ cudaError_t up(mst_lu* s, T** dst, const std::vector<T>& v) {
   cudaError_t e = cudaMalloc((void**)dst, bytes);
   if (e != cudaSuccess) return e;
   s->allocs.push_back(*dst);
-  if (!v.empty()) e = cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  // on the solver's stream: its kernels do not wait for the default one
+  if (!v.empty())
+    e = cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s->stream);
   return e;
 }
 
-// Rows in the given order with their first four entries at fixed places; a
-// sweep's entries times 1 / D[column] (the quotient and product the reference
-// forms at every use), a product's (rD = null) as they are
-cudaError_t up_rows(mst_lu* s, LuRows* out, const Csr& c, const std::vector<int>& rows,
-                    const std::vector<int>& lev, const std::vector<double>* rD) {
-  std::vector<int4> meta(rows.size()), col4(rows.size(), int4{0, 0, 0, 0});
-  std::vector<double4_32a> w4(rows.size(), double4_32a{0., 0., 0., 0.});
-  std::vector<int> col;
-  std::vector<double> w;
-  for (size_t i = 0; i < rows.size(); ++i) {
-    const int k0 = c.ptr[rows[i]], n = c.ptr[rows[i] + 1] - k0;
-    meta[i] = int4{rows[i], n, (int)col.size(), 0};
-    for (int k = 0; k < n; ++k) {
-      const int j = c.col[k0 + k];
-      const double q = rD ? c.val[k0 + k] * (*rD)[j] : c.val[k0 + k];
-      if (k < 4) {
-        (&col4[i].x)[k] = j;
-        (&w4[i].x)[k] = q;
-      } else {
-        col.push_back(j);
-        w.push_back(q);
-      }
-    }
+// the tables of the one-launch solve, in one allocation
+cudaError_t lu_tables(mst_lu* s) {
+  const int dim = s->dim, nb = (dim + 127) / 128;
+  size_t at = 0;
+  auto place = [&](size_t bytes) {
+    const size_t p = at;
+    at += (bytes + 255) / 256 * 256;
+    return p;
+  };
+  struct Rows {
+    LuRows* out;
+    const int *rows, *ptr, *col;
+    const double* val;
+    bool sweep;
+    const int* lev;
+    int n_levels;
+    size_t meta, col4, w4;
+  } t[4] = {{&s->r_up, nullptr, s->ua_ptr, s->ua_col, s->ua_val, false, nullptr, 1},
+            {&s->r_lo, nullptr, s->l_ptr, s->l_col, s->l_val, false, nullptr, 1},
+            {&s->r_fwd, s->fwd_rows, s->l_ptr, s->l_col, s->l_val, true, s->fwd_lev,
+             s->n_fwd_levels},
+            {&s->r_bwd, s->bwd_rows, s->ud_ptr, s->ud_col, s->ud_val, true, s->bwd_lev,
+             s->n_bwd_levels}};
+  for (Rows& q : t) {
+    q.meta = place(sizeof(int4) * (size_t)dim);
+    q.col4 = place(sizeof(int4) * (size_t)dim);
+    q.w4 = place(sizeof(double4_32a) * (size_t)dim);
   }
-  int *d_lev = nullptr, *d_col = nullptr;
-  int4 *d_meta = nullptr, *d_col4 = nullptr;
-  double4_32a* d_w4 = nullptr;
-  double* d_w = nullptr;
-  cudaError_t e = up(s, &d_lev, lev);
-  if (e == cudaSuccess) e = up(s, &d_meta, meta);
-  if (e == cudaSuccess) e = up(s, &d_col4, col4);
-  if (e == cudaSuccess) e = up(s, &d_w4, w4);
-  if (e == cudaSuccess) e = up(s, &d_col, col);
-  if (e == cudaSuccess) e = up(s, &d_w, w);
-  *out = LuRows{d_lev, d_meta, d_col4, d_w4, d_col, d_w, (int)lev.size() - 1};
-  return e;
+  const size_t rD = place(sizeof(double) * (size_t)dim),
+               change = place(sizeof(unsigned) * kLuMaxCta), its = place(sizeof(int));
+  char* d = nullptr;
+  cudaError_t e = cudaMalloc((void**)&d, at);
+  if (e != cudaSuccess) return e;
+  s->allocs.push_back(d);
+  s->rD = (double*)(d + rD);
+  s->change = (unsigned*)(d + change);
+  s->its = (int*)(d + its);
+  k_lu_reciprocal<<<nb, 128, 0, s->stream>>>(dim, s->D, s->rD);
+  for (Rows& q : t) {
+    *q.out = LuRows{q.lev, (int4*)(d + q.meta), (int4*)(d + q.col4), (double4_32a*)(d + q.w4),
+                    q.col, q.val, q.sweep ? s->rD : nullptr, q.n_levels};
+    k_lu_rows<<<nb, 128, 0, s->stream>>>(dim, q.rows, q.ptr, q.col, q.val, q.out->rD,
+                                         (int4*)(d + q.meta), (int4*)(d + q.col4),
+                                         (double4_32a*)(d + q.w4));
+  }
+  return cudaGetLastError();
 }
 
 int lu_cta_rows(int cluster, int dim) {
@@ -696,31 +746,23 @@ mst_status mst_lu_create(int block, int dim, int n, const int* rows, const int* 
   const std::vector<double> zero((size_t)dim * block, 0.0);
   for (double** p : {&s->b, &s->x})
     if (e == cudaSuccess) e = up(s, p, zero);
+  if (e == cudaSuccess) e = up(s, &s->l_ptr, L.ptr);
+  if (e == cudaSuccess) e = up(s, &s->l_col, L.col);
+  if (e == cudaSuccess) e = up(s, &s->l_val, L.val);
+  if (e == cudaSuccess) e = up(s, &s->ua_ptr, Ua.ptr);
+  if (e == cudaSuccess) e = up(s, &s->ua_col, Ua.col);
+  if (e == cudaSuccess) e = up(s, &s->ua_val, Ua.val);
+  if (e == cudaSuccess) e = up(s, &s->ud_ptr, Ud.ptr);
+  if (e == cudaSuccess) e = up(s, &s->ud_col, Ud.col);
+  if (e == cudaSuccess) e = up(s, &s->ud_val, Ud.val);
+  if (e == cudaSuccess) e = up(s, &s->fwd_rows, fr);
+  if (e == cudaSuccess) e = up(s, &s->bwd_rows, br);
   if (block == 1) s->cluster = lu_pick_cluster(dim);
   if (e == cudaSuccess && s->cluster > 0) {
-    std::vector<double> rD(dim);
-    std::vector<int> order(dim);
-    for (int r = 0; r < dim; ++r) rD[r] = 1. / D[r];
-    std::iota(order.begin(), order.end(), 0);
-    e = up_rows(s, &s->r_up, Ua, order, {0, dim}, nullptr);
-    if (e == cudaSuccess) e = up_rows(s, &s->r_lo, L, order, {0, dim}, nullptr);
-    if (e == cudaSuccess) e = up_rows(s, &s->r_fwd, L, fr, s->fwd_ptr, &rD);
-    if (e == cudaSuccess) e = up_rows(s, &s->r_bwd, Ud, br, s->bwd_ptr, &rD);
-    if (e == cudaSuccess) e = up(s, &s->rD, rD);
-    if (e == cudaSuccess) e = up(s, &s->change, std::vector<unsigned>(kLuMaxCta, 0u));
-    if (e == cudaSuccess) e = up(s, &s->its, std::vector<int>(1, 0));
+    e = up(s, &s->fwd_lev, s->fwd_ptr);
+    if (e == cudaSuccess) e = up(s, &s->bwd_lev, s->bwd_ptr);
+    if (e == cudaSuccess) e = lu_tables(s);
   } else {
-    if (e == cudaSuccess) e = up(s, &s->l_ptr, L.ptr);
-    if (e == cudaSuccess) e = up(s, &s->l_col, L.col);
-    if (e == cudaSuccess) e = up(s, &s->l_val, L.val);
-    if (e == cudaSuccess) e = up(s, &s->ua_ptr, Ua.ptr);
-    if (e == cudaSuccess) e = up(s, &s->ua_col, Ua.col);
-    if (e == cudaSuccess) e = up(s, &s->ua_val, Ua.val);
-    if (e == cudaSuccess) e = up(s, &s->ud_ptr, Ud.ptr);
-    if (e == cudaSuccess) e = up(s, &s->ud_col, Ud.col);
-    if (e == cudaSuccess) e = up(s, &s->ud_val, Ud.val);
-    if (e == cudaSuccess) e = up(s, &s->fwd_rows, fr);
-    if (e == cudaSuccess) e = up(s, &s->bwd_rows, br);
     for (double** p : {&s->t1, &s->rhs, &s->rhs1})
       if (e == cudaSuccess) e = up(s, p, zero);
     if (e == cudaSuccess) e = up(s, &s->part, std::vector<double>((dim + 127) / 128 + 1, 0.0));
