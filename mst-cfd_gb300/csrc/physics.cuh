@@ -335,16 +335,30 @@ __device__ __forceinline__ T entropy_fix_fast(T x) {
   const T ax = fabs(x), e = T(0.125);
   return ax > e ? ax : (x * x + e * e) * (T(0.5) / e);
 }
+// Products whose rounded values have to cancel: equal pressures and velocities
+// of the two sides, the terms of mirrored states at a wall.  A fused
+// multiply-add of one of them leaves the other's rounding error (at FP32 a mass
+// flux of 1e-9 through walls).  sep: in FP32 only; in FP64 that error is below
+// 1e-16 and the fused form saves an instruction of the busiest pipe.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float sep(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double sep(double a, double b) { return a * b; }
+// sqrt(R / L) of the Roe average: in FP32 the root itself, which gives 1 where
+// the quotient of equal numbers is off by its rounding
+__device__ __forceinline__ float roe_ratio(float x) { return sqrtf(x); }
+__device__ __forceinline__ double roe_ratio(double x) { return x * inv_sqrt(x); }
+
 template <class T>
 __device__ __forceinline__ void roe_face(const T L[4], const T R[4], int flags, T F[8]) {
   const T eor = T(1e-10), gm1 = Gas<T>::gm1();
   const T irL = T(1) / L[0], irR = T(1) / R[0];
-  const T uL[2] = {L[1] * irL, L[2] * irL}, uR[2] = {R[1] * irR, R[2] * irR};
-  const T pL = (L[3] - T(0.5) * (L[1] * uL[0] + L[2] * uL[1])) * gm1;
-  const T pR = (R[3] - T(0.5) * (R[1] * uR[0] + R[2] * uR[1])) * gm1;
+  const T uL[2] = {mul_rn(L[1], irL), mul_rn(L[2], irL)},
+          uR[2] = {mul_rn(R[1], irR), mul_rn(R[2], irR)};
+  const T pL = mul_rn(L[3] - T(0.5) * (L[1] * uL[0] + L[2] * uL[1]), gm1);
+  const T pR = mul_rn(R[3] - T(0.5) * (R[1] * uR[0] + R[2] * uR[1]), gm1);
   const T hL = (L[3] + pL) * irL, hR = (R[3] + pR) * irR;
-  const T x = fabs(R[0] * irL);
-  const T D = x * inv_sqrt(x);
+  const T D = roe_ratio(fabs(R[0] * irL));
   const T iD = T(1) / (T(1) + D);
   const T u[2] = {(uL[0] + D * uR[0]) * iD, (uL[1] + D * uR[1]) * iD};
   const T H = (hL + D * hR) * iD;
@@ -366,15 +380,15 @@ __device__ __forceinline__ void roe_face(const T L[4], const T R[4], int flags, 
     const T l1 = entropy_fix_fast(ud - a), l2 = entropy_fix_fast(ud),
             l4 = entropy_fix_fast(ud + a);
     const T rd = rta * du[d];
-    const T w1 = l1 * ((dp - rd) * hia2), w4 = l4 * ((dp + rd) * hia2);
-    const T w2 = l2 * al2, w3 = l2 * (rt * du[t]);
+    const T w1 = sep(l1, (dp - rd) * hia2), w4 = sep(l4, (dp + rd) * hia2);
+    const T w2 = sep(l2, al2), w3 = l2 * (rt * du[t]);
     const T ws = (w1 + w2) + w4, wd = (w4 - w1) * a;
     const T sg = ((flags >> d) & 1) ? T(-0.5) : T(0.5);
     const T mL = L[1 + d], mR = R[1 + d];
     F[4 * d] = T(0.5) * (mL + mR) + sg * ws;
-    F[4 * d + 1 + d] = T(0.5) * ((mL * vL[d] + mR * vR[d]) + (pL + pR)) + sg * (ws * ud + wd);
-    F[4 * d + 1 + t] = T(0.5) * (mL * vL[t] + mR * vR[t]) + sg * (ws * ut + w3);
-    F[4 * d + 3] = T(0.5) * (hL * mL + hR * mR) +
+    F[4 * d + 1 + d] = T(0.5) * ((sep(mL, vL[d]) + sep(mR, vR[d])) + (pL + pR)) + sg * (ws * ud + wd);
+    F[4 * d + 1 + t] = T(0.5) * (sep(mL, vL[t]) + sep(mR, vR[t])) + sg * (ws * ut + w3);
+    F[4 * d + 3] = T(0.5) * (sep(hL, mL) + sep(hR, mR)) +
                    sg * ((w1 + w4) * H + (wd * ud + (w2 * ke + w3 * ut)));
   }
 }
