@@ -214,7 +214,7 @@ __global__ void k_invert_blocks(int dim, const double* __restrict__ D, double* _
 // The levels of a sweep are small (800 rows of an 18k-row mesh system) and
 // depend on each other, so a launch per level pays launch and memory latency
 // 230 times a solve.  Here one thread-block cluster runs all iterations and the
-// exit test.  The swept vector lies in the CTAs' shared memory, 512 rows in turn
+// exit test.  The swept vector lies in the CTAs' shared memory, 32 rows in turn
 // to each CTA; a row's dependent values are read from the owner (distributed
 // shared memory: two thirds of the latency of the same vector in L2), and a
 // level ends with the hardware cluster barrier.  A row's columns and weights
@@ -278,9 +278,9 @@ struct LuVec {
   double* base;
   int shift;
   __device__ __forceinline__ double* at(int r) const {
-    const int chunk = r / kLuThreads;
-    return cg::this_cluster().map_shared_rank(base, chunk & ((1 << shift) - 1)) +
-           ((chunk >> shift) * kLuThreads + r % kLuThreads);
+    const int group = r / 32;
+    return cg::this_cluster().map_shared_rank(base, group & ((1 << shift) - 1)) +
+           ((group >> shift) * 32 + r % 32);
   }
   __device__ __forceinline__ double operator[](int r) const { return *(volatile double*)at(r); }
 };
@@ -371,10 +371,11 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lu_solve(const LuSolve S) {
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), n_cta = (int)cl.num_blocks();
   const LuVec y{sm, S.shift}, v{sm + S.rows, S.shift};
-  // this thread's rows of the row-parallel phases lie in its own CTA
-  const int r0 = rank * kLuThreads + threadIdx.x, stride = kLuThreads * n_cta;
-  // its rows of a level: the warps' groups of 32 go to the CTAs in turn
-  const int first = ((int)(threadIdx.x / 32) * n_cta + rank) * 32 + (int)(threadIdx.x % 32);
+  // this thread's rows r0, r0 + stride, .. of the vectors (in its own CTA's shared
+  // memory, at threadIdx.x, + kLuThreads, ..) and of a level: the warps' groups
+  // of 32 go to the CTAs in turn
+  const int stride = kLuThreads * n_cta;
+  const int r0 = ((int)(threadIdx.x / 32) * n_cta + rank) * 32 + (int)(threadIdx.x % 32);
   cl.sync();  // every CTA runs before its shared memory is used
   int it = 0;
   for (it = 0; it < kLuInterval; ++it) {
@@ -400,14 +401,14 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lu_solve(const LuSolve S) {
       }
     }
     cl.sync();
-    lu_sweep(S.fwd, v, first, stride);
+    lu_sweep(S.fwd, v, r0, stride);
     if (!S.gs) {
       for (int r = r0, j = threadIdx.x; r < S.dim; r += stride, j += kLuThreads) {
         const double x1 = S.rD[r] * v.base[j];
         v.base[j] = S.D[r] * x1;
       }
       cl.sync();
-      lu_sweep(S.bwd, v, first, stride);
+      lu_sweep(S.bwd, v, r0, stride);
     }
     // X = D^-1 v
     unsigned ch = 0;

@@ -419,7 +419,12 @@ __device__ void energy_and_residual(const SimpleDev& S, bool last, double (&res)
 
 // nsteps time steps of one case on one thread-block cluster
 __device__ void simple_steps(const SimpleDev& S, int nsteps) {
-  const int gtid = (int)cg::this_cluster().block_rank() * blockDim.x + threadIdx.x;
+  // consecutive groups of 32 rows go to the CTAs in turn: a level of 800 rows, or
+  // the last pass over the cells, then occupies one warp on each of the SMs
+  // instead of all warps of two, and an FP64 warp instruction holds its SM
+  // sub-partition for 64 cycles
+  const int gtid = (int)((threadIdx.x / 32 * cg::this_cluster().num_blocks() +
+                          cg::this_cluster().block_rank()) * 32 + threadIdx.x % 32);
   const int gstride = (int)cg::this_cluster().num_blocks() * blockDim.x;
   const bool writer = (gtid == 0);
   for (int step = 0; step < nsteps; ++step) {
