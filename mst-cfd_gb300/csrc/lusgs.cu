@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "cluster_vec.cuh"
 #include "ctx.hpp"
 #include "smem_limit.hpp"
 
@@ -273,15 +274,7 @@ struct LuSolve {
   int* its;
 };
 
-// a vector over the cluster's shared memory
-struct LuVec {
-  double* base;
-  int shift;
-  __device__ __forceinline__ double* at(int r) const {
-    const int group = r / 32;
-    return cg::this_cluster().map_shared_rank(base, group & ((1 << shift) - 1)) +
-           ((group >> shift) * 32 + r % 32);
-  }
+struct LuVec : mst::ClusterVec<1> {
   __device__ __forceinline__ double operator[](int r) const { return *(volatile double*)at(r); }
 };
 
@@ -296,17 +289,23 @@ __device__ __forceinline__ void lu_fetch(LuRow& r, const LuRows& s, int i, int e
   r.c = s.col4[i];
   r.w = s.w4[i];
 }
-// acc - sum w v (or + : the products), entries in order
-template <bool SUB, class V>
-__device__ __forceinline__ double lu_row(const LuRow& r, const LuRows& s, const V& v, double acc) {
+// acc - sum w v (or + : the products), entries in order; lu_values: the first
+// four entries' v
+template <class V>
+__device__ __forceinline__ double4_32a lu_values(const LuRow& r, const V& v) {
   const int n = r.meta.y;
-  const double v0 = n > 0 ? v[r.c.x] : 0., v1 = n > 1 ? v[r.c.y] : 0., v2 = n > 2 ? v[r.c.z] : 0.,
-               v3 = n > 3 ? v[r.c.w] : 0.;
+  return double4_32a{n > 0 ? v[r.c.x] : 0., n > 1 ? v[r.c.y] : 0., n > 2 ? v[r.c.z] : 0.,
+                     n > 3 ? v[r.c.w] : 0.};
+}
+template <bool SUB, class V>
+__device__ __forceinline__ double lu_row(const LuRow& r, const double4_32a& x, const LuRows& s,
+                                         const V& v, double acc) {
+  const int n = r.meta.y;
   auto add = [&](double p) { acc = SUB ? acc - p : acc + p; };
-  if (n > 0) add(r.w.x * v0);
-  if (n > 1) add(r.w.y * v1);
-  if (n > 2) add(r.w.z * v2);
-  if (n > 3) add(r.w.w * v3);
+  if (n > 0) add(r.w.x * x.x);
+  if (n > 1) add(r.w.y * x.y);
+  if (n > 2) add(r.w.z * x.z);
+  if (n > 3) add(r.w.w * x.w);
   for (int k = r.meta.z; k < r.meta.z + n - 4; ++k) {
     const int c = s.col[k];
     add((s.rD ? s.val[k] * s.rD[c] : s.val[k]) * v[c]);
@@ -329,13 +328,20 @@ __device__ void lu_sweep(const LuRows& s, const LuVec& v, int first, int stride)
   LuRow cur, nxt;
   lu_fetch(cur, s, b + first, e);
   for (int l = 1; l < n; ++l) {
-    lu_fetch(nxt, s, e + first, e1);
-    const int e3 = s.lev[min(l + 4, n)];
+    int e3 = 0;
     for (int i = b + first;;) {
+      // the earlier rows' values first, the next level's row behind them
+      double4_32a x{};
+      double own = 0.;
       if (cur.meta.x >= 0) {
-        double* p = v.at(cur.meta.x);
-        *p = lu_row<true>(cur, s, v, *(volatile double*)p);
+        x = lu_values(cur, v);
+        own = v[cur.meta.x];
       }
+      if (i == b + first) {
+        lu_fetch(nxt, s, e + first, e1);
+        e3 = s.lev[min(l + 4, n)];
+      }
+      if (cur.meta.x >= 0) *v.at(cur.meta.x) = lu_row<true>(cur, x, s, v, own);
       i += stride;
       if (i >= e) break;
       lu_fetch(cur, s, i, e);
@@ -349,28 +355,11 @@ __device__ void lu_sweep(const LuRows& s, const LuVec& v, int first, int stride)
   }
 }
 
-// A row's |X - X'| / X against the bounds of the exit test: bit 0, not below
-// 1e-7; bit 1, above 1e-20 (the test of SparseSolverNUM.cpp:194-205 on the
-// largest quotient, started at 0, NaN never taken).  The quotient lies within a
-// factor of two of the power of two that the exponents give; it is formed where
-// that does not decide.
-__device__ __forceinline__ unsigned lu_change(double xo, double xn) {
-  const double d = fabs(xo - xn);
-  const int ex = (__double2hiint(xo) >> 20) & 0x7ff, ed = __double2hiint(d) >> 20;
-  if (ex > 0 && ex < 0x7ff && ed > 0 && ed < 0x7ff) {
-    if (__double2hiint(xo) < 0) return 0;
-    if (ed - ex >= -22) return 3;                    // > 2^-23 > 1e-7
-    if (ed - ex <= -25 && ed - ex >= -65) return 2;  // < 2^-24 < 1e-7, > 2^-66 > 1e-20
-  }
-  const double q = d / xo;
-  return (q >= 1e-7 ? 1u : 0u) | (q > 1e-10 * 1e-10 ? 2u : 0u);
-}
-
 __global__ void __launch_bounds__(kLuThreads, 1) k_lu_solve(const LuSolve S) {
   extern __shared__ double sm[];
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), n_cta = (int)cl.num_blocks();
-  const LuVec y{sm, S.shift}, v{sm + S.rows, S.shift};
+  const LuVec y{{sm, S.shift}}, v{{sm + S.rows, S.shift}};
   // this thread's rows r0, r0 + stride, .. of the vectors (in its own CTA's shared
   // memory, at threadIdx.x, + kLuThreads, ..) and of a level: the warps' groups
   // of 32 go to the CTAs in turn
@@ -385,7 +374,7 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lu_solve(const LuSolve S) {
     lu_fetch(cur, S.up, r0, S.dim);
     for (int r = r0, j = threadIdx.x; r < S.dim; r += stride, j += kLuThreads) {
       lu_fetch(nxt, S.up, r + stride, S.dim);
-      const double s = lu_row<false>(cur, S.up, x, 0.);
+      const double s = lu_row<false>(cur, lu_values(cur, x), S.up, x, 0.);
       if (S.gs) v.base[j] = S.b[r] - s;
       else y.base[j] = s / S.D[r];
       cur = nxt;
@@ -396,7 +385,7 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lu_solve(const LuSolve S) {
       cl.sync();
       for (int r = r0, j = threadIdx.x; r < S.dim; r += stride, j += kLuThreads) {
         lu_fetch(nxt, S.lo, r + stride, S.dim);
-        v.base[j] = S.b[r] + lu_row<false>(cur, S.lo, y, 0.);
+        v.base[j] = S.b[r] + lu_row<false>(cur, lu_values(cur, y), S.lo, y, 0.);
         cur = nxt;
       }
     }
@@ -414,7 +403,7 @@ __global__ void __launch_bounds__(kLuThreads, 1) k_lu_solve(const LuSolve S) {
     unsigned ch = 0;
     for (int r = r0, j = threadIdx.x; r < S.dim; r += stride, j += kLuThreads) {
       const double xn = S.rD[r] * v.base[j];
-      ch |= lu_change(__ldcg(S.x + r), xn);
+      ch |= mst::gs_change(__ldcg(S.x + r), xn);
       S.x[r] = xn;
     }
     const unsigned big = __syncthreads_or(ch & 1u), any = __syncthreads_or(ch & 2u);
