@@ -1,5 +1,5 @@
 // 3D FP64 parity kernels: compiled with --fmad=false so every product and
-// sum rounds separately, in the order of the checker's restatement.
+// sum rounds separately, in the order of the oracle's restatement.
 #include "devtypes3d.hpp"
 #include "launch3d.hpp"
 #include "mesh.hpp"

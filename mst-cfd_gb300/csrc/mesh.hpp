@@ -170,9 +170,12 @@ void order_faces_by_cell(int nF, int nC, Cell cell, std::vector<int>* iperm,
   iperm->resize(nF);
   std::vector<int> fill(at.begin(), at.end() - 1);
   for (int f = 0; f < nF; ++f) (*iperm)[fill[(*low)[f]]++] = f;
+  // a cell has a few faces: insertion, stable (std::stable_sort allocates a buffer
+  // on every call)
+  int* v = iperm->data();
   for (int c = 0; c < nC; ++c)
-    std::stable_sort(iperm->begin() + at[c], iperm->begin() + at[c + 1],
-                     [&](int x, int y) { return high[x] < high[y]; });
+    for (int k = at[c] + 1; k < at[c + 1]; ++k)
+      for (int q = k; q > at[c] && high[v[q]] < high[v[q - 1]]; --q) std::swap(v[q], v[q - 1]);
 }
 
 }  // namespace mst

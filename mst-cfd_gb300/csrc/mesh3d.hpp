@@ -14,7 +14,7 @@
 //   volume        divergence theorem, V = 1/3 sum (x_f - x_c) . S_out
 //   eta0          |x_f - x_c1| / (|x_f - x_c0| + |x_f - x_c1|) (Face.cpp:62-69)
 // Compiled with -ffp-contract=off: the operation order is the one of the
-// checker's restatement, so both produce the same bits.
+// oracle's restatement, so both produce the same bits.
 #pragma once
 #include <string>
 #include <vector>
