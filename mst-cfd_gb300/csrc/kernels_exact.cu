@@ -1,5 +1,6 @@
 // FP64 parity kernels: compiled with --fmad=false so every product and sum
 // rounds separately, in the reference's order (bit-identical residuals).
+#include "chained.cuh"
 #include "devtypes.hpp"
 #include "mesh.hpp"
 #include "physics.cuh"

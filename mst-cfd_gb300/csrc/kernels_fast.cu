@@ -2,6 +2,7 @@
 // and the FP32 path (FP32 reconstruction and flux; state, residual sums and
 // update as unevaluated FP32 pairs with compensated sums, no FP64
 // instruction except the last stage's norm epilogue).
+#include "chained.cuh"
 #include "devtypes.hpp"
 #include "mesh.hpp"
 #include "physics.cuh"
