@@ -24,9 +24,10 @@ __device__ __forceinline__ void chain() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// on = false: launched the ordinary way
 template <class... P, class... A>
-cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                           A... args) {
+cudaError_t launch_chained(bool on, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -36,7 +37,7 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = on ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
