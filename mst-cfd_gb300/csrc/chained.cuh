@@ -17,11 +17,12 @@
 
 namespace mst {
 
-__device__ __forceinline__ void chain() {
+// next = false: the last kernel on a caller's stream, whose next launch is not ours
+__device__ __forceinline__ void chain(bool next = true) {
   // the previous kernel has ended and its writes are visible
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // the next one may be placed
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (next) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // on = false: launched the ordinary way
