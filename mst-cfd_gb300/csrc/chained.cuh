@@ -2,7 +2,8 @@
 // placed while this one still runs and wait for its end themselves, so that
 // launch and drain are hidden between the short kernels of a time step: 50 FP64
 // RK2 steps of 4,000 cells 3,147 -> 2,490 us, 30 viscous FP32 steps of 97k cells
-// 1,289 -> 1,086, 20 FP32 steps of 2M cells 7,114 -> 6,945.
+// 1,289 -> 1,086, 20 FP32 steps of 2M cells 7,114 -> 6,945; in 3D 10 FP32 steps
+// of 3,072 / 48,000 cells 493 -> 372 / 732 -> 612, 20 of 1.6M 9,322 -> 9,066.
 //
 // Every kernel launched with launch_chained calls chain() in every thread that
 // goes on, and in at least one thread of every block: a block that ended without

@@ -1,5 +1,6 @@
 // 3D FP64 parity kernels: compiled with --fmad=false so every product and
 // sum rounds separately, in the order of the oracle's restatement.
+#include "chained.cuh"
 #include "devtypes3d.hpp"
 #include "launch3d.hpp"
 #include "mesh.hpp"

@@ -1,5 +1,6 @@
 // 3D production kernels: FP64 with fused multiply-add, and the FP32 path
 // (FP32 reconstruction and flux, float-pair state and residual sums).
+#include "chained.cuh"
 #include "devtypes3d.hpp"
 #include "launch3d.hpp"
 #include "mesh.hpp"

@@ -32,3 +32,31 @@ def test_one_call_equals_single_steps(nx, ny, steps, flux, precision):
         s.set_state(q)
         s.step(steps)
         assert np.array_equal(s.state(), one)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["PREC_FP64_EXACT", "PREC_FP64", "PREC_FP32"])
+@pytest.mark.parametrize("n,steps", [(2, 30), (7, 20), (24, 6)])
+def test_one_call_equals_single_steps_3d(n, steps, precision):
+    from mstcfd import capi, meshgen as mg
+    from mstcfd.mesh3d import Mesh3D
+    from mstcfd.solver3d import Solver3D
+    m = mg.tet_box(n)
+    s = Solver3D(Mesh3D.from_dict(m), precision=getattr(capi, precision), order=2, limiter=3,
+                 cfl=0.3)
+    rng = np.random.default_rng(n)
+    k = int(m["n_cells"])
+    r, p = 1 + 0.1 * rng.random(k), 1 + 0.1 * rng.random(k)
+    v = 0.1 * rng.standard_normal((k, 3))
+    v[:, 0] += 0.5
+    q = np.concatenate([r[:, None], r[:, None] * v,
+                        (p / 0.4 + 0.5 * r * (v * v).sum(1))[:, None]], 1)
+    s.set_state(q)
+    for _ in range(steps):
+        s.step(1)
+    one = s.state()
+    assert np.all(np.isfinite(one))
+    for _ in range(3):
+        s.set_state(q)
+        s.step(steps)
+        assert np.array_equal(s.state(), one)
