@@ -255,7 +255,10 @@ typedef struct mst_ctx mst_ctx;
 mst_status mst_ctx_create(const mst_mesh *m, const mst_params *p,
                           mst_ctx **out);
 mst_status mst_ctx_destroy(mst_ctx *c);
-/* Replaces the parameters (the mesh stays resident). */
+/* Replaces the parameters (the mesh stays resident).  The first change
+ * between FP32 and an FP64 precision uploads that precision's geometry, and
+ * one to a wider FP64 precision than before allocates its face buffer: such a
+ * call may return MST_ECUDA, with the parameters as they were. */
 mst_status mst_ctx_set_params(mst_ctx *c, const mst_params *p);
 
 /* RhoSolver::setDT (RhoSolver.cpp:33-35). */

@@ -761,6 +761,7 @@ mst_status mst_internal_geometry(mst_ctx* c, bool f32) {
     CU(up(&dm.cf_face, L.cf_face));
     CU(up(&dm.cf_nb, L.cf_nb));
     CU(up(&dm.cf_nb_fix, L.cf_nb_fix));
+    CU(mst::uploads_done());
     c->geo64 = true;
     return MST_OK;
   }
@@ -816,6 +817,7 @@ mst_status mst_internal_geometry(mst_ctx* c, bool f32) {
   CU(up(&dm.e_nb, nb));
   CU(up(&dm.e_slot, slot));
   CU(up(&dm.e_wd, wd));
+  CU(mst::uploads_done());
   c->geo32 = true;
   return MST_OK;
 }

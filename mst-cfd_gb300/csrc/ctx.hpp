@@ -13,6 +13,14 @@
 // Records msg as this thread's mst_last_error() text and returns s.
 mst_status mst_internal_fail(mst_status s, const std::string& msg);
 
+namespace mst {
+// Waits for the tables uploaded with cudaMemcpy and cudaMemset.  From pageable
+// memory such a copy returns once the source has been read, perhaps before its
+// last bytes have arrived, and the solvers' streams do not wait for the default
+// one: call it before a kernel on such a stream may read what was uploaded.
+inline cudaError_t uploads_done() { return cudaStreamSynchronize(nullptr); }
+}  // namespace mst
+
 struct mst_mesh {
   mst::HostMesh host;
   mst::DevLayout lay;
