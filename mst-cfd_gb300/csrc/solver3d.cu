@@ -430,6 +430,11 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
     cleanup();
     return fail3(MST_ECUDA, "memset failed");
   }
+  // the first state and step may follow at once, on this context's stream
+  if (mst::uploads_done() != cudaSuccess) {
+    cleanup();
+    return fail3(MST_ECUDA, "upload of the mesh failed");
+  }
   c->n_cell_faces = tot;
   c->n_borrowed = (int)L.t_bor.size();
   *out = c.release();
