@@ -523,9 +523,8 @@ cudaError_t up(mst_lu* s, T** dst, const std::vector<T>& v) {
   cudaError_t e = cudaMalloc((void**)dst, bytes);
   if (e != cudaSuccess) return e;
   s->allocs.push_back(*dst);
-  // on the solver's stream: its kernels do not wait for the default one
-  if (!v.empty())
-    e = cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s->stream);
+  // (returns once v has been read; mst_lu_create waits for the arrival)
+  if (!v.empty()) e = cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
   return e;
 }
 
@@ -751,22 +750,23 @@ mst_status mst_lu_create(int block, int dim, int n, const int* rows, const int* 
   if (e == cudaSuccess && s->cluster > 0) {
     e = up(s, &s->fwd_lev, s->fwd_ptr);
     if (e == cudaSuccess) e = up(s, &s->bwd_lev, s->bwd_ptr);
-    if (e == cudaSuccess) e = lu_tables(s);
   } else {
     for (double** p : {&s->t1, &s->rhs, &s->rhs1})
       if (e == cudaSuccess) e = up(s, p, zero);
     if (e == cudaSuccess) e = up(s, &s->part, std::vector<double>((dim + 127) / 128 + 1, 0.0));
   }
-  if (e == cudaSuccess && block == 4) {
+  if (e == cudaSuccess && block == 4)
     e = up(s, &s->Di, std::vector<double>((size_t)dim * 16, 0.0));
+  if (e == cudaSuccess) e = mst::uploads_done();
+  if (e == cudaSuccess && s->cluster > 0) e = lu_tables(s);
+  if (e == cudaSuccess && block == 4) {
     // D^-1 once: the reference re-inverts D[i] at every use, always to the
     // same result
-    if (e == cudaSuccess) {
-      k_invert_blocks<4><<<(dim + 127) / 128, 128, 0, s->stream>>>(dim, s->D, s->Di);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    k_invert_blocks<4><<<(dim + 127) / 128, 128, 0, s->stream>>>(dim, s->D, s->Di);
+    e = cudaGetLastError();
   }
+  // the set-up's failure is this call's
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) {
     mst_lu_destroy(s);
     return lu_fail(MST_ECUDA, std::string("mst_lu_create: ") + cudaGetErrorString(e));
