@@ -161,6 +161,14 @@ mst_status balloc(mst_batch* b, T** p, size_t bytes) {
   return MST_OK;
 }
 
+// n values into a device array that the next launches read
+template <class T>
+mst_status bset(T* dst, const T* src, size_t n) {
+  B_CU(cudaMemcpy(dst, src, n * sizeof(T), cudaMemcpyHostToDevice));
+  B_CU(mst::uploads_done());
+  return MST_OK;
+}
+
 template <class T>
 mst_status bupload(mst_batch* b, T** p, const std::vector<T>& v) {
   mst_status s = balloc(b, p, v.size() * sizeof(T));
@@ -429,8 +437,8 @@ mst_status restart_cases(mst_batch* b, const std::vector<int>& ids, int iters) {
   for (int k : ids) flag[k] = 1;
   int it = 0;
   B_CU(cudaMemcpy(&it, b->iter, sizeof(int), cudaMemcpyDeviceToHost));
-  B_CU(cudaMemcpy(b->restart_flag, flag.data(), sizeof(int) * b->n_cases,
-                  cudaMemcpyHostToDevice));
+  mst_status st = bset(b->restart_flag, flag.data(), flag.size());
+  if (st) return st;
   const int nC = c->dm.n_cells;
   k_restart_cells<<<(nC + 255) / 256, 256, 0, c->stream>>>(
       nC, b->c_case, b->restart_flag, b->q_fb, c->q_old, c->q_new, c->qf_old, c->qf_new);
@@ -451,8 +459,7 @@ mst_status restart_cases(mst_batch* b, const std::vector<int>& ids, int iters) {
       b->lo_best[k] = 1e300;
       b->lo_best_it[k] = iters;
     }
-    B_CU(cudaMemcpy(b->case_lo, b->lo_h.data(), sizeof(int) * b->n_cases,
-                    cudaMemcpyHostToDevice));
+    if ((st = bset(b->case_lo, b->lo_h.data(), b->lo_h.size()))) return st;
     b->lo = true;
     update_both(b);
   }
@@ -494,12 +501,9 @@ mst_status build_lists(mst_batch* b, const std::vector<int>& cv) {
     }
     b->act_off[col + 1] = (int)cells.size();
   }
-  if (!tiles.empty())
-    B_CU(cudaMemcpy(b->tile_list, tiles.data(), sizeof(int) * tiles.size(),
-                    cudaMemcpyHostToDevice));
-  if (!cells.empty())
-    B_CU(cudaMemcpy(b->act_cells, cells.data(), sizeof(int4) * cells.size(),
-                    cudaMemcpyHostToDevice));
+  mst_status st = MST_OK;
+  if (!tiles.empty() && (st = bset(b->tile_list, tiles.data(), tiles.size()))) return st;
+  if (!cells.empty() && (st = bset(b->act_cells, cells.data(), cells.size()))) return st;
   c->dm.tile_list = b->tile_list;
   c->dm.n_list = (int)tiles.size();
   b->compact = true;
@@ -707,7 +711,8 @@ mst_status mst_batch_create(const mst_mesh* const* meshes, const mst_case_params
   b->c_case_h = std::move(c_case);
   b->color_cells_h = std::move(cells);
   b->list_cells = nC;
-  if (cudaStreamSynchronize(b->ctx->stream) != cudaSuccess) {
+  if (mst::uploads_done() != cudaSuccess ||
+      cudaStreamSynchronize(b->ctx->stream) != cudaSuccess) {
     cleanup();
     return mst_internal_fail(MST_ECUDA, "batch setup failed");
   }
@@ -766,8 +771,7 @@ mst_status mst_batch_set_state(mst_batch* b, const double* q) {
   if (b->lo) {
     b->lo_h.assign(b->n_cases, 1);
     update_both(b);
-    B_CU(cudaMemcpy(b->case_lo, b->lo_h.data(), sizeof(int) * b->n_cases,
-                    cudaMemcpyHostToDevice));
+    if ((st = bset(b->case_lo, b->lo_h.data(), b->lo_h.size()))) return st;
   }
   if (b->lo || b->sweep32) {
     cudaError_t e = mst::fast::launch_to_f32(b->ctx->q_old, b->ctx->qf_old, b->ctx->dm.n_cells,
@@ -788,7 +792,8 @@ mst_status mst_batch_set_l2_ref(mst_batch* b, const double* l2_ref) {
     for (int i = 0; i < b->n_cases; ++i)
       if (!(l2_ref[i] > 0.0))
         return mst_internal_fail(MST_EINVAL, "reference L2 values must be > 0");
-    B_CU(cudaMemcpy(b->first, l2_ref, sizeof(double) * b->n_cases, cudaMemcpyHostToDevice));
+    mst_status st = bset(b->first, l2_ref, b->n_cases);
+    if (st) return st;
     b->first_fixed = true;
   }
   // the captured graphs hold the norm arguments: rebuild them
@@ -981,9 +986,7 @@ mst_status mst_batch_solve(mst_batch* b, mst_batch_result* res) {
         st = ensure_graph();
         if (st) return st;
       } else if (moved) {
-        // read by the next iterations' launches (same stream)
-        B_CU(cudaMemcpy(b->case_lo, b->lo_h.data(), sizeof(int) * b->n_cases,
-                        cudaMemcpyHostToDevice));
+        if ((st = bset(b->case_lo, b->lo_h.data(), b->lo_h.size()))) return st;
         update_both(b);
         st = ensure_graph();
         if (st) return st;

@@ -55,3 +55,34 @@ def test_sparse_system(dim, block):
         del junk
         s.close()
     assert np.all(np.isfinite(first[0]))
+
+
+@pytest.mark.gpu
+def test_batch():
+    """Flags and lists that a batch sends while it solves -- phases, restarts, the
+    cells left after a retirement -- are those of its next iterations."""
+    from mstcfd import Mesh, batch, capi
+    from mstcfd import meshgen as mg
+    m = mg.wedge(6000, 9.0, seed=3)
+    mesh = Mesh.from_arrays(m["node_xy"], m["face_nodes"], m["face_cells"], m["zones"],
+                            m["n_cells"])
+    n = mesh.n_cells
+    q0 = [mg.freestream(mach, n) for mach in (1.9, 2.2, 2.5, 2.8)]
+    bad = q0[1].copy()
+    bad[n // 2, 0] = np.nan
+    cases = [(mesh, batch.case_params(mg.freestream(mach))) for mach in (1.9, 2.2, 2.5, 2.8)]
+    first = None
+    for _ in range(4):
+        b = batch.Batch(cases, implicit=dict(max_iter=60, graph_iters=2, autotune=0, tol=1e-30,
+                                             fp32_until=1e-1, fp32_window=10, sweep_fp32=1,
+                                             restart_after=30),
+                        flux=1, order=2, limiter=1, precision=capi.PREC_FP64)
+        for _ in range(2):
+            b.set_state([q0[0], bad, q0[2], q0[3]])
+            b.set_fallback(q0)
+            b.solve()
+            out = b.state()
+            first = out if first is None else first
+            for x, y in zip(out, first):
+                assert np.array_equal(x, y, equal_nan=True)
+        b.close()
