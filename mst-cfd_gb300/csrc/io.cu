@@ -208,6 +208,7 @@ mst_status build_node_avg(mst_ctx* c, int quirks, NodeAvg* a) {
                      cudaMemcpyHostToDevice));
     IO_CU(cudaMemcpy(a->ew, ew.data(), sizeof(double2) * ew.size(), cudaMemcpyHostToDevice));
   }
+  IO_CU(mst::uploads_done());
   a->quirks = quirks;
   a->n_nodes = nN;
   return MST_OK;

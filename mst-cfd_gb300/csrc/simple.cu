@@ -944,6 +944,7 @@ mst_status mst_simple_create(const mst_mesh* mesh, const mst_simple_params* prm,
   }
   if (e == cudaSuccess) e = sup(s, &d.part, none, (size_t)16 * kPart);
   if (e == cudaSuccess) e = sup(s, &d.change, std::vector<unsigned>(16, 0u));
+  if (e == cudaSuccess) e = mst::uploads_done();
   if (e != cudaSuccess) {
     mst_simple_destroy(s);
     return sfail(MST_ECUDA, std::string("mst_simple_create: ") + cudaGetErrorString(e));

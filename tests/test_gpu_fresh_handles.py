@@ -86,3 +86,46 @@ def test_batch():
             for x, y in zip(out, first):
                 assert np.array_equal(x, y, equal_nan=True)
         b.close()
+
+
+def _channel():
+    from mstcfd import Mesh, meshgen as mg
+    m = mg.tri_box(40, 30, 2.0, 1.0, jitter=0.2, seed=5, left=mg.INLET, right=mg.OUTLET,
+                   bottom=mg.WALL, top=mg.WALL)
+    return Mesh.from_arrays(m["node_xy"], m["face_nodes"], m["face_cells"], m["zones"],
+                            m["n_cells"])
+
+
+@pytest.mark.gpu
+def test_simple():
+    from mstcfd.psolver import SimpleSolver, reference_initial
+    mesh = _channel()
+    p0, f0 = reference_initial(mesh, 1.0)
+    first = None
+    for _ in range(6):
+        s = SimpleSolver(mesh, p0, f0)
+        for _ in range(2):
+            s.set_state(p0, f0)
+            out = [s.step(1), *s.state()]
+            first = out if first is None else first
+            for x, y in zip(out, first):
+                assert np.array_equal(x, y, equal_nan=True)
+        s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("quirks", [0, 1])
+def test_node_values(quirks):
+    from mstcfd import Solver, capi, meshgen as mg
+    mesh = _channel()
+    q = mg.random_state(mesh.n_cells, seed=2)
+    first = None
+    for _ in range(6):
+        s = Solver(mesh, order=1, reference_quirks=quirks, precision=capi.PREC_FP64)
+        s.set_state(q)
+        for _ in range(2):
+            out = s.node_values()
+            first = out if first is None else first
+            for x, y in zip(out, first):
+                assert np.array_equal(x, y)
+        s.close()
