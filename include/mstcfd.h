@@ -734,7 +734,9 @@ mst_status mst_simple_get_info(const mst_simple *s, mst_simple_info *info);
 mst_status mst_simple_destroy(mst_simple *s);
 
 /* Per-kernel CUDA-event timing on the context's stream.  When enabled,
- * every kernel launch of mst_solve/mst_step is bracketed by events; the
+ * every kernel launch of mst_solve/mst_step is bracketed by events and
+ * starts after the end of the one before (otherwise a launch's blocks are
+ * placed while the previous one drains; the results are the same); the
  * totals accumulate until mst_profile_reset. */
 mst_status mst_profile_enable(mst_ctx *c, int on);
 mst_status mst_profile_reset(mst_ctx *c);

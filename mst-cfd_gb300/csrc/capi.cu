@@ -1323,6 +1323,7 @@ mst_status mst_profile_enable(mst_ctx* c, int on) {
   if (!c) return fail(MST_EINVAL, "NULL context");
   drain_profile(c);
   c->profiling = on != 0;
+  c->dm.in_turn = c->profiling;
   return MST_OK;
 }
 

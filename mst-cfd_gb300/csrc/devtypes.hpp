@@ -53,6 +53,7 @@ struct DevMesh {
   // (cell, position) of its c0 side and of its c1 side, -1 where none
   int4 quirk_at;
   int deg3;  // every cell has three faces and c_ptr[c] = 3c (triangles)
+  bool in_turn;  // explicit steps: every launch after the end of the one before
   // batches (nullptr for a single mesh): the case of every device cell and
   // the iteration at which each case converged (-1 while it runs).  The
   // residual kernels skip the cells of converged cases: after the

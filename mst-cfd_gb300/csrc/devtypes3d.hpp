@@ -15,6 +15,7 @@ constexpr int kNoFace3 = 0x7fffffff;
 // packed (x, y, z) per face or cell-face (FP64 paths), FP32 tables (FP32 path)
 struct DevMesh3 {
   int n_cells, n_faces;
+  bool in_turn;  // every launch after the end of the one before
   const int2* f_c0c1;
   const int* f_info;
   const double *f_dir, *f_r0, *f_r1, *f_eta;

@@ -579,6 +579,7 @@ mst_status mst_ctx3d_profile(mst_ctx3d* c, int on) {
   if (!c) return fail3(MST_EINVAL, "NULL context");
   drain3(c);
   c->profiling = on != 0;
+  c->dm.in_turn = c->profiling;
   c->kname.clear();
   c->klaunch.clear();
   c->kms.clear();
