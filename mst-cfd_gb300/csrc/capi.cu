@@ -423,9 +423,9 @@ mst_status compute_dt(mst_ctx* c, const double4_32a* q, double t_end,
   } else {
     ProfScope ps(c, "k_spectral_dt");
     cudaError_t e = (c->p.precision == MST_PREC_FP64_EXACT)
-                        ? mst::exact::launch_spectral_dt(prec_of(c->p), c->dm, q, c->p.cfl,
+                        ? mst::exact::launch_spectral_dt(prec_of(c->p), c->dm, q, qf, c->p.cfl,
                                                          c->dt_cell, c->dt_part, own, c->stream)
-                        : mst::fast::launch_spectral_dt(prec_of(c->p), c->dm, q, c->p.cfl,
+                        : mst::fast::launch_spectral_dt(prec_of(c->p), c->dm, q, qf, c->p.cfl,
                                                         c->dt_cell, c->dt_part, own, c->stream);
     c->last_launches++;
     if (e != cudaSuccess) return fail(MST_ECUDA, std::string("spectral_dt: ") + cudaGetErrorString(e));

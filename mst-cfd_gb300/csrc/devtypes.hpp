@@ -338,8 +338,9 @@ enum { kFluxAusm = 0, kFluxRoe = 1 };
                                const DevMesh& m, const StepArgs& a,           \
                                double* F, cudaStream_t s);                    \
   cudaError_t launch_spectral_dt(int prec, const DevMesh& m,                 \
-                                 const double4_32a* q, double cfl,            \
-                                 double* dt_cell, double* partials,           \
+                                 const double4_32a* q, const float4* qf,      \
+                                 double cfl, double* dt_cell,                 \
+                                 double* partials,                            \
                                  const FinishDt& fin, cudaStream_t s);        \
   cudaError_t lusgs_forward_t(const DevMesh& m, const LusgsArgs& a,          \
                               int threads, bool turn, cudaStream_t s);        \

@@ -34,11 +34,11 @@ cudaError_t launch_face_flux(int, int flux, int order, const DevMesh& m,
                              const StepArgs& a, double* F, cudaStream_t s) {
   return face_dispatch<double>(flux, order, m, a, F, s);
 }
-cudaError_t launch_spectral_dt(int, const DevMesh& m, const double4_32a* q,
+cudaError_t launch_spectral_dt(int, const DevMesh& m, const double4_32a* q, const float4*,
                                double cfl, double* dt_cell, double* partials,
                                const FinishDt& fin, cudaStream_t s) {
   const int nb = (m.n_cells + 255) / 256;
-  k_spectral_dt<double><<<nb, 256, 0, s>>>(m, q, cfl, dt_cell, partials, fin);
+  k_spectral_dt<double><<<nb, 256, 0, s>>>(m, q, nullptr, cfl, dt_cell, partials, fin);
   return cudaGetLastError();
 }
 }  // namespace exact

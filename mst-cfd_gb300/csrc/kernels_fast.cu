@@ -43,13 +43,13 @@ cudaError_t launch_face_flux(int prec, int flux, int order, const DevMesh& m,
   return face_dispatch<double>(flux, order, m, a, F, s);
 }
 cudaError_t launch_spectral_dt(int prec, const DevMesh& m, const double4_32a* q,
-                               double cfl, double* dt_cell, double* partials,
+                               const float4* qf, double cfl, double* dt_cell, double* partials,
                                const FinishDt& fin, cudaStream_t s) {
   const int nb = (m.n_cells + 255) / 256;
   if (prec == kPrecF32)
-    k_spectral_dt<float><<<nb, 256, 0, s>>>(m, q, cfl, dt_cell, partials, fin);
+    k_spectral_dt<float, true><<<nb, 256, 0, s>>>(m, q, qf, cfl, dt_cell, partials, fin);
   else
-    k_spectral_dt<double><<<nb, 256, 0, s>>>(m, q, cfl, dt_cell, partials, fin);
+    k_spectral_dt<double><<<nb, 256, 0, s>>>(m, q, nullptr, cfl, dt_cell, partials, fin);
   return cudaGetLastError();
 }
 }  // namespace fast
