@@ -299,7 +299,8 @@ __device__ __forceinline__ F8 div_deg(F8 v, float d, float r) {
   float m = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v.x[i]));
-  if (m == __int_as_float(0x7f800000) || d > 256.f) {
+  // (d = 0: a neighbour whose own list is empty)
+  if (m == __int_as_float(0x7f800000) || !(d >= 1.f && d <= 256.f)) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) v.x[i] /= d;
   } else {
