@@ -216,44 +216,27 @@ int build_layout3d(const SolverMesh3D& m, DevLayout3D* L, std::string* err) {
   const int nT = (nC + kTileCells - 1) / kTileCells;
   L->n_tiles = nT;
   // faces by the lower, then the higher device cell (a warp's faces gather
-  // from neighbouring cells); a tile owns those whose lower cell is its own
-  std::vector<int> owner, face_iperm;
+  // from neighbouring cells)
+  std::vector<int> low, face_iperm;
   order_faces_by_cell(nF, nC, [&](int f, int side) {
     const int c = m.face_cells[2 * (size_t)f + side];
     return c >= 0 ? L->cell_perm[c] : -1;
-  }, &face_iperm, &owner);
+  }, &face_iperm, &low);
   L->face_perm.assign(nF, 0);
   for (int i = 0; i < nF; ++i) L->face_perm[face_iperm[i]] = i;
-  L->t_own_ptr.assign(nT + 1, 0);
-  for (int f = 0; f < nF; ++f) L->t_own_ptr[owner[f] / kTileCells + 1]++;
-  for (int t = 0; t < nT; ++t) L->t_own_ptr[t + 1] += L->t_own_ptr[t];
-  // borrowed faces: cut faces owned by the other tile, ascending device id
-  L->t_bor_ptr.assign(nT + 1, 0);
+  // faces a tile touches: its own, and the cut faces another tile owns
+  std::vector<int> touched(nT, 0);
+  L->n_borrowed = 0;
   for (int f = 0; f < nF; ++f) {
     const int c1 = m.face_cells[2 * (size_t)f + 1];
-    if (c1 < 0) continue;
     const int ta = L->cell_perm[m.face_cells[2 * (size_t)f]] / kTileCells;
-    const int tb = L->cell_perm[c1] / kTileCells;
-    if (ta != tb) L->t_bor_ptr[std::max(ta, tb) + 1]++;
+    const int tb = c1 >= 0 ? L->cell_perm[c1] / kTileCells : ta;
+    ++touched[ta];
+    if (ta == tb) continue;
+    ++touched[tb];
+    ++L->n_borrowed;
   }
-  for (int t = 0; t < nT; ++t) L->t_bor_ptr[t + 1] += L->t_bor_ptr[t];
-  L->t_bor.assign(L->t_bor_ptr[nT], 0);
-  {
-    std::vector<int> fill(L->t_bor_ptr.begin(), L->t_bor_ptr.end() - 1);
-    for (int df = 0; df < nF; ++df) {  // device order: each list ascends
-      const int f = face_iperm[df];
-      const int c1 = m.face_cells[2 * (size_t)f + 1];
-      if (c1 < 0) continue;
-      const int ta = L->cell_perm[m.face_cells[2 * (size_t)f]] / kTileCells;
-      const int tb = L->cell_perm[c1] / kTileCells;
-      if (ta != tb) L->t_bor[fill[std::max(ta, tb)]++] = df;
-    }
-  }
-  L->max_tile_faces = 0;
-  for (int t = 0; t < nT; ++t)
-    L->max_tile_faces =
-        std::max(L->max_tile_faces, (L->t_own_ptr[t + 1] - L->t_own_ptr[t]) +
-                                        (L->t_bor_ptr[t + 1] - L->t_bor_ptr[t]));
+  L->max_tile_faces = nT ? *std::max_element(touched.begin(), touched.end()) : 0;
   L->f_c0c1.assign(2 * (size_t)nF, -1);
   L->f_info.assign(nF, 0);
   L->f_dir.assign(3 * (size_t)nF, 0.0);
@@ -283,41 +266,21 @@ int build_layout3d(const SolverMesh3D& m, DevLayout3D* L, std::string* err) {
     L->c_ptr[dc + 1] = L->c_ptr[dc] + (m.cell_ptr[c + 1] - m.cell_ptr[c]);
   }
   const int tot = L->c_ptr[nC];
-  L->cf_slot.assign(tot, 0);
   L->cf_face.assign(tot, 0);
   L->cf_nb.assign(tot, -1);
   L->cf_w.assign(2 * (size_t)tot, 0.0);
   L->cf_dir.assign(3 * (size_t)tot, 0.0);
-  for (int t = 0; t < nT; ++t) {
-    const int ob = L->t_own_ptr[t], oe = L->t_own_ptr[t + 1], n_own = oe - ob;
-    const int* bb = L->t_bor.data() + L->t_bor_ptr[t];
-    const int* be = L->t_bor.data() + L->t_bor_ptr[t + 1];
-    const int cb = t * kTileCells, ce = std::min(nC, cb + kTileCells);
-    for (int dc = cb; dc < ce; ++dc) {
-      const int c = L->cell_iperm[dc];
-      for (int j = 0; j < m.cell_ptr[c + 1] - m.cell_ptr[c]; ++j) {
-        const int k = m.cell_ptr[c] + j, dk = L->c_ptr[dc] + j;
-        const int f = m.cell_faces[k], df = L->face_perm[f];
-        int slot;
-        if (df >= ob && df < oe) {
-          slot = df - ob;
-        } else {
-          const int* p = std::lower_bound(bb, be, df);
-          if (p == be || *p != df) {
-            *err = "internal: face missing from its tile";
-            return kEInval;
-          }
-          slot = n_own + (int)(p - bb);
-        }
-        const bool own = m.face_cells[2 * (size_t)f] == c;
-        L->cf_slot[dk] = (slot << 1) | (own ? 0 : 1);
-        L->cf_face[dk] = own ? df : ~df;
-        const int nb = m.cell_nb[k];
-        L->cf_nb[dk] = nb >= 0 ? L->cell_perm[nb] : -1;
-        L->cf_w[2 * (size_t)dk] = m.cell_w[2 * (size_t)k];
-        L->cf_w[2 * (size_t)dk + 1] = m.cell_w[2 * (size_t)k + 1];
-        for (int d = 0; d < 3; ++d) L->cf_dir[3 * (size_t)dk + d] = m.cell_dir[3 * (size_t)k + d];
-      }
+  for (int dc = 0; dc < nC; ++dc) {
+    const int c = L->cell_iperm[dc];
+    for (int j = 0; j < m.cell_ptr[c + 1] - m.cell_ptr[c]; ++j) {
+      const int k = m.cell_ptr[c] + j, dk = L->c_ptr[dc] + j;
+      const int f = m.cell_faces[k], df = L->face_perm[f];
+      L->cf_face[dk] = m.face_cells[2 * (size_t)f] == c ? df : ~df;
+      const int nb = m.cell_nb[k];
+      L->cf_nb[dk] = nb >= 0 ? L->cell_perm[nb] : -1;
+      L->cf_w[2 * (size_t)dk] = m.cell_w[2 * (size_t)k];
+      L->cf_w[2 * (size_t)dk + 1] = m.cell_w[2 * (size_t)k + 1];
+      for (int d = 0; d < 3; ++d) L->cf_dir[3 * (size_t)dk + d] = m.cell_dir[3 * (size_t)k + d];
     }
   }
   return kOk;

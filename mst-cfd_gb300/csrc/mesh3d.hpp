@@ -43,17 +43,19 @@ int build_solver3d(const HostMesh3D& h, const std::vector<double>& c1_shift,
 constexpr int kInfo3Flag = 3;
 
 struct DevLayout3D {
-  int n_cells = 0, n_faces = 0, n_tiles = 0, max_tile_faces = 0;
+  int n_cells = 0, n_faces = 0;
+  // runs of kTileCells cells: their number, the most faces one touches, the cut
+  // faces (layout statistics)
+  int n_tiles = 0, max_tile_faces = 0, n_borrowed = 0;
   std::vector<int> cell_perm, cell_iperm;   // file <-> device cells
   std::vector<int> face_perm;               // file face -> device face
   std::vector<int> f_c0c1, f_info;          // [nF][2], [nF]
   std::vector<double> f_dir, f_r0, f_r1;    // [nF][3]
   std::vector<double> f_eta;                // [nF]
   std::vector<double> c_vol;                // [nC]
-  std::vector<int> c_ptr, cf_slot, cf_nb;   // cf_slot = tile slot << 1 | (cell is c1)
+  std::vector<int> c_ptr, cf_nb;
   std::vector<int> cf_face;                 // device face, ~face where the cell is c1
   std::vector<double> cf_w, cf_dir;         // [tot][2], [tot][3]
-  std::vector<int> t_own_ptr, t_bor_ptr, t_bor;
 };
 
 // Morton renumbering of the cell centres, tiles of kTileCells cells, faces

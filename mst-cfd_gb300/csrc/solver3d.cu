@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -86,13 +87,12 @@ mst_status alloc3(mst_ctx3d* c, T** p, size_t count) {
   return MST_OK;
 }
 
-template <class T, class S>
-mst_status upload3(mst_ctx3d* c, const T** dst, const std::vector<S>& src) {
+template <class T>
+mst_status upload3(mst_ctx3d* c, const T** dst, const std::vector<T>& src) {
   T* d = nullptr;
   mst_status st = alloc3(c, &d, src.size());
   if (st) return st;
-  std::vector<T> tmp(src.begin(), src.end());
-  if (!tmp.empty()) C3(cudaMemcpy(d, tmp.data(), tmp.size() * sizeof(T), cudaMemcpyHostToDevice));
+  if (!src.empty()) C3(cudaMemcpy(d, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
   *dst = d;
   return MST_OK;
 }
@@ -370,7 +370,7 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
     std::vector<int> nb(deg * n), face(deg * n, mst::kNoFace3);
     std::vector<float4> dw(deg * n, make_float4(0.f, 0.f, 0.f, 0.f));
     std::vector<float> w1(deg * n, 0.f);
-    for (size_t at = 0; at < nb.size(); ++at) nb[at] = (int)(at % n);
+    for (int k = 0; k < deg; ++k) std::iota(nb.begin() + k * n, nb.begin() + (k + 1) * n, 0);
     for (int i = 0; i < nC; ++i)
       for (int k = L.c_ptr[i]; k < L.c_ptr[i + 1]; ++k) {
         const size_t at = (size_t)(k - L.c_ptr[i]) * n + i;
@@ -436,7 +436,7 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
     return fail3(MST_ECUDA, "upload of the mesh failed");
   }
   c->n_cell_faces = tot;
-  c->n_borrowed = (int)L.t_bor.size();
+  c->n_borrowed = L.n_borrowed;
   *out = c.release();
   return MST_OK;
 }
