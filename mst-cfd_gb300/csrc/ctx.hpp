@@ -61,7 +61,8 @@ struct mst_ctx {
   float4 *qf_old = nullptr, *qf_new = nullptr, *qf_stage = nullptr;
   float4 *ql_old = nullptr, *ql_new = nullptr, *ql_stage = nullptr;
   void* grad = nullptr;
-  double* flux = nullptr;      // [nF][8] debug output
+  double* flux = nullptr;      // [nF][8] face fluxes in file order (mst_get_face_flux)
+  const int* face_file = nullptr;  // file face of every device face, with flux
   // FP64 paths: the face-flux buffer, 4 (production) or 8 (exact) doubles
   // per face; allocated once a context runs one of them
   double* fx = nullptr;

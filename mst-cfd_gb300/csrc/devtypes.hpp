@@ -336,7 +336,7 @@ enum { kFluxAusm = 0, kFluxRoe = 1 };
                                  int threads, cudaStream_t s);                \
   cudaError_t launch_face_flux(int prec, int flux, int order,                \
                                const DevMesh& m, const StepArgs& a,           \
-                               double* F, cudaStream_t s);                    \
+                               const int* file, double* F, cudaStream_t s);   \
   cudaError_t launch_spectral_dt(int prec, const DevMesh& m,                 \
                                  const double4_32a* q, const float4* qf,      \
                                  double cfl, double* dt_cell,                 \

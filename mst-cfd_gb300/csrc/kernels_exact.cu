@@ -31,8 +31,8 @@ cudaError_t launch_flux_update(int, int flux, int order, const DevMesh& m,
   return flux_dispatch<double>(flux, order, m, a, s);
 }
 cudaError_t launch_face_flux(int, int flux, int order, const DevMesh& m,
-                             const StepArgs& a, double* F, cudaStream_t s) {
-  return face_dispatch<double>(flux, order, m, a, F, s);
+                             const StepArgs& a, const int* file, double* F, cudaStream_t s) {
+  return face_dispatch<double>(flux, order, m, a, file, F, s);
 }
 cudaError_t launch_spectral_dt(int, const DevMesh& m, const double4_32a* q, const float4*,
                                double cfl, double* dt_cell, double* partials,

@@ -38,9 +38,9 @@ cudaError_t launch_flux_update(int prec, int flux, int order, const DevMesh& m,
   return flux_dispatch<double>(flux, order, m, a, s);
 }
 cudaError_t launch_face_flux(int prec, int flux, int order, const DevMesh& m,
-                             const StepArgs& a, double* F, cudaStream_t s) {
-  if (prec == kPrecF32) return face_dispatch<float>(flux, order, m, a, F, s);
-  return face_dispatch<double>(flux, order, m, a, F, s);
+                             const StepArgs& a, const int* file, double* F, cudaStream_t s) {
+  if (prec == kPrecF32) return face_dispatch<float>(flux, order, m, a, file, F, s);
+  return face_dispatch<double>(flux, order, m, a, file, F, s);
 }
 cudaError_t launch_spectral_dt(int prec, const DevMesh& m, const double4_32a* q,
                                const float4* qf, double cfl, double* dt_cell, double* partials,
