@@ -35,6 +35,7 @@ struct mst_ctx3d {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   mst::DevMesh3 dm{};
   const int *cell_perm = nullptr, *cell_iperm = nullptr;  // device: file -> device cell, back
+  std::vector<int> host_perm;  // the first of them, where the host reorders states
   int n_cell_faces = 0, n_borrowed = 0, n_tiles = 0, max_tile_faces = 0;
   std::vector<void*> allocs;
   size_t bytes = 0;
@@ -220,6 +221,14 @@ mst_status residual_dev(mst_ctx3d* c) {
   C3(flux3(c, a, 3));
   return MST_OK;
 }
+
+// States cross the boundary as one linear copy each way, reordered on the
+// device (1.6M cells: 11.1 and 12.5 ms with the host reordering).  On FP64 paths
+// a state of few cells is reordered by the host, which saves the launch: 48 / 750
+// / 1,000 / 4,096 cells 8.5 / 12.2 / 13.2 / 20.7 us against 12.3 / 14.5 / 14.9 /
+// 20.9 inwards, 11.7 / 16.3 / 17.0 / 25.2 against 15.5 / 15.6 / 14.7 / 16.2
+// outwards.  (FP32 converts on the device anyway.)
+constexpr int kHostSet = 2048, kHostGet = 512;  // most cells
 
 // device-order rows of `width` values to the host in file order: reordered
 // on the device, one linear copy
@@ -437,6 +446,7 @@ mst_status mst_ctx3d_create(const mst_mesh3d* mesh, const mst_params3d* p, mst_c
   }
   c->n_cell_faces = tot;
   c->n_borrowed = L.n_borrowed;
+  if (nC <= kHostSet) c->host_perm = L.cell_perm;
   *out = c.release();
   return MST_OK;
 }
@@ -469,11 +479,18 @@ mst_status mst_ctx3d_info_get(mst_ctx3d* c, mst_ctx3d_info* info) {
   return MST_OK;
 }
 
-// States cross the boundary as one linear copy each way, reordered on the
-// device (1.6M cells: 11.1 and 12.5 ms with the host reordering).
 mst_status mst_ctx3d_set_state(mst_ctx3d* c, const double* q) {
   if (!c || !q) return fail3(MST_EINVAL, "NULL argument");
   const int nC = c->dm.n_cells, i = c->cur;
+  if (!f32(c) && nC <= kHostSet) {
+    std::vector<double> h(5 * (size_t)nC);
+    for (int f = 0; f < nC; ++f)
+      std::memcpy(h.data() + 5 * (size_t)c->host_perm[f], q + 5 * (size_t)f, 5 * sizeof(double));
+    C3(cudaMemcpyAsync(c->q[i], h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice,
+                       c->stream));
+    C3(cudaStreamSynchronize(c->stream));
+    return MST_OK;
+  }
   C3(cudaMemcpyAsync(c->qtmp, q, sizeof(double) * 5 * (size_t)nC, cudaMemcpyHostToDevice,
                      c->stream));
   if (f32(c))
@@ -488,6 +505,15 @@ mst_status mst_ctx3d_set_state(mst_ctx3d* c, const double* q) {
 mst_status mst_ctx3d_get_state(mst_ctx3d* c, double* q) {
   if (!c || !q) return fail3(MST_EINVAL, "NULL argument");
   const int nC = c->dm.n_cells, i = c->cur;
+  if (!f32(c) && nC <= kHostGet) {
+    std::vector<double> h(5 * (size_t)nC);
+    C3(cudaMemcpyAsync(h.data(), c->q[i], h.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                       c->stream));
+    C3(cudaStreamSynchronize(c->stream));
+    for (int f = 0; f < nC; ++f)
+      std::memcpy(q + 5 * (size_t)f, h.data() + 5 * (size_t)c->host_perm[f], 5 * sizeof(double));
+    return MST_OK;
+  }
   if (f32(c))
     C3(mst::fast3::pairs(false, c->qtmp, c->cell_perm, nC, c->h4[i], c->h1[i], c->l4[i], c->l1[i],
                          c->stream));
