@@ -4,6 +4,8 @@
 // RK2 steps of 4,000 cells 3,147 -> 2,490 us, 30 viscous FP32 steps of 97k cells
 // 1,289 -> 1,086, 20 FP32 steps of 2M cells 7,114 -> 6,945; in 3D 10 FP32 steps
 // of 3,072 / 48,000 cells 493 -> 372 / 732 -> 612, 20 of 1.6M 9,322 -> 9,066.
+// Blocks placed early go where the previous kernel has left room, not evenly:
+// the launchers leave out the kernels that lose by that.
 //
 // Every kernel launched with launch_chained calls chain() in every thread that
 // goes on, and in at least one thread of every block: a block that ended without
