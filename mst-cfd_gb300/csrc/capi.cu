@@ -114,7 +114,11 @@ __global__ void k_fixed_dt(double dt, const mst::FinishDt f) { mst::set_step(dt,
 // additions on one SM -- now 9.)
 // out: linf[4], l2[4] (sqrt(mean)), mass, dt, time
 constexpr int kNormBlocks = 64;    // most blocks
-constexpr int kNormTiles = 128;    // tiles per block before there are more blocks
+constexpr int kNormTiles = 128;    // tiles per block where there are several
+// Most tiles of one block: the ticket of several costs 2 us (FP32 first-order
+// solve, one block / several: 220 tiles 19.4 / 21.7, 352 20.2 / 22.3, 507 24.1 /
+// 23.6, 757 26.9 / 25.1, 1,024 29.9 / 27.6 us)
+constexpr int kNormOne = 400;
 __device__ __forceinline__ double norm_op(int j, double x, double v) {
   return (j < 4) ? ((x < v) ? v : x) : x + v;
 }
@@ -444,8 +448,9 @@ mst_status compute_dt(mst_ctx* c, const double4_32a* q, double t_end,
 
 mst_status finalize_norms(mst_ctx* c) {
   ProfScope ps(c, "k_finalize_norms");
-  const int nb = std::min(kNormBlocks, (c->dm.n_tiles + kNormTiles - 1) / kNormTiles);
-  k_finalize_norms<<<std::max(nb, 1), dim3(64, kNormSlots), 0, c->stream>>>(
+  const int nt = c->dm.n_tiles;
+  const int nb = nt <= kNormOne ? 1 : std::min(kNormBlocks, (nt + kNormTiles - 1) / kNormTiles);
+  k_finalize_norms<<<nb, dim3(64, kNormSlots), 0, c->stream>>>(
       c->partials, c->dm.n_tiles, c->dm.n_cells, c->scal, c->norm_part, c->dt_ticket + 1, c->norms);
   c->last_launches++;
   CU(cudaGetLastError());
