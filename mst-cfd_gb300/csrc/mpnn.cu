@@ -1019,9 +1019,9 @@ mst_status mst_mpnn_set_graph(mst_mpnn* m, int n, const float* features, const i
   if (!m || n <= 0 || !features || !nbr_ptr || !nbr)
     return mst_internal_fail(MST_EINVAL, "bad graph arguments");
   const int n_nbr = nbr_ptr[n];
-  int bad = 0;  // (no early exit: the loops vectorise)
+  int bad = nbr_ptr[0] < 0;  // (no early exit: the loops vectorise)
   for (int i = 0; i < n; ++i) bad |= nbr_ptr[i + 1] < nbr_ptr[i];
-  if (bad) return mst_internal_fail(MST_EINVAL, "nbr_ptr not ascending");
+  if (bad) return mst_internal_fail(MST_EINVAL, "nbr_ptr not ascending from 0 on");
   for (int i = 0; i < n_nbr; ++i) bad |= (unsigned)nbr[i] >= (unsigned)n;
   if (bad) return mst_internal_fail(MST_EINVAL, "neighbour id out of range");
   cudaError_t e = ensure_cap(m, n, std::max(n_nbr, 1));

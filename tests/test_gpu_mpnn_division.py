@@ -139,3 +139,17 @@ def test_infinite_value_reaches_the_neighbours_only(d):
     assert np.array_equal(y[1:4], [[np.inf, nan, nan, nan]] * 3, equal_nan=True)
     assert np.array_equal(y[4:], [[1.0, 2.0, 3.0, 4.0]] * (N - 4))
     net.close()
+
+
+@pytest.mark.gpu
+def test_lists_before_their_start_are_refused():
+    """A list that begins before the array is an error of the call, not a read."""
+    from mstcfd import capi
+    from mstcfd.mpnn import Network
+    net = Network(seed=1)
+    feats = np.zeros((3, mr.IN), np.float32)
+    with pytest.raises(capi.MstError):
+        net.set_graph(feats, [-4, 0, 1, 2], [1, 0])
+    net.set_graph(feats, [0, 1, 2, 2], [1, 0])
+    assert np.all(np.isfinite(net.forward()))
+    net.close()
