@@ -38,16 +38,6 @@ mst_status fail(mst_status s, const std::string& msg) {
       return fail(MST_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-template <class T>
-cudaError_t upload(T** dst, const std::vector<T>& src) {
-  *dst = nullptr;
-  size_t n = std::max<size_t>(src.size(), 1) * sizeof(T);
-  cudaError_t e = cudaMalloc((void**)dst, n);
-  if (e != cudaSuccess) return e;
-  if (!src.empty()) e = cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice);
-  return e;
-}
-
 // ---- small orchestration kernels (not on the arithmetic-parity path) ----
 // device state -> file order and back
 __global__ void k_gather_rows(const double4_32a* __restrict__ src,
