@@ -105,8 +105,13 @@ __device__ __forceinline__ bool range_cases_done(const DevMesh& m, int c0, int c
   return true;
 }
 
-// Most blocks of a launch that sets the step itself (finish_dt).
-constexpr int kFinishBlocks = 1024;
+// Most blocks of a launch that sets the step itself (finish_dt).  RK2 steps with
+// that / with a launch of its own (us): FP32 64 blocks 22.7 / 27.2, 512 37.6 / 40.8,
+// 1,024 65.0 / 66.9, 2,048 114.8 / 117.0, 3,000 161.9 / 162.2, 4,096 206.2 / 205.6,
+// 7,813 367 / 360; FP64 64 50.2 / 54.9, 1,024 217.5 / 219.5, 2,048 370.8 / 373.0,
+// 3,000 526 / 526, 7,813 1,313 / 1,305; 3D FP32 768 64.2 / 67.3, 1,500 117.8 / 119.5,
+// 2,592 198.2 / 197.1.
+constexpr int kFinishBlocks = 2048;
 
 // Cells per block of the FP64 gradient kernels.
 constexpr int kGrad64Cells = 64;
@@ -138,10 +143,10 @@ __device__ __forceinline__ void set_step(double x, const FinishDt& f) {
 
 // The minima that this launch's blocks leave in part, reduced by the last
 // block to arrive (every block calls it after its thread 0 stored its own
-// minimum).  Saves the launch of a one-block reduction (6 us) where the
-// launch is about one wave of blocks; beyond kFinishBlocks the atomics on one
-// address and the blocks that wait for them cost more than that launch
-// (7,813 blocks: gradient 48 -> 76 us, the launch 7).
+// minimum).  Saves the launch of a one-block reduction; beyond kFinishBlocks the
+// atomics on one address and the blocks that wait for them cost more than that
+// launch (7,813 blocks: gradient 57.9 -> 66.5 us, each launch waiting for the one
+// before; the reduction 12.8).
 __device__ __forceinline__ void finish_dt(const double* part, const FinishDt& f) {
   if (!f.ticket) return;
   __shared__ bool last_block;
